@@ -218,6 +218,16 @@ int varq_attn_fwd(const varq_tensor_t* q, const varq_tensor_t* k_codes, const va
                   int32_t k_store_bits, int32_t v_store_bits, float softmax_scale,
                   const varq_tensor_t* out, void* workspace, size_t workspace_bytes, void* stream);
 
+/* varq_attn_fwd on queries normalised on the way in: q / max(||q||_2, q_eps) * q_mul[h] in fp32 (q_mul may be NULL = 1), so a
+ * normalised copy of the queries is never stored.  VARQ_ERR_UNSUPPORTED, without a launch, where no kernel does that
+ * (head_dim other than 64 or 128, caches that are not head-major).
+ * Replaces VAR/models/basic_var.py:137-139 in front of the attention call. */
+int varq_attn_fwd_qnorm(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
+                        const varq_qparams_t* kp, const varq_qparams_t* vp,
+                        int32_t B, int32_t H, int32_t Lq, int32_t Lk, int32_t D,
+                        int32_t k_store_bits, int32_t v_store_bits, float softmax_scale, const float* q_mul, float q_eps,
+                        const varq_tensor_t* out, void* workspace, size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

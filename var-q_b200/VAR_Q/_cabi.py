@@ -22,7 +22,7 @@ SYMBOLS = (
     "varq_quant_workspace_bytes", "varq_quant_pack", "varq_quant_pack_static",
     "varq_quant_static_scratch_bytes", "varq_unpack_dequant",
     "varq_attn_workspace_bytes", "varq_attn_fwd", "varq_attn_force_path",
-    "varq_qk_norm_stats", "varq_quant_pack_prestats",
+    "varq_qk_norm_stats", "varq_quant_pack_prestats", "varq_attn_fwd_qnorm",
 )
 
 
@@ -79,6 +79,8 @@ def _declare(lib):
     lib.varq_attn_force_path.argtypes = [i32]
     lib.varq_attn_fwd.restype = i32
     lib.varq_attn_fwd.argtypes = [T, T, T, Q, Q, i32, i32, i32, i32, i32, i32, i32, f32, T, vp, sz, vp]
+    lib.varq_attn_fwd_qnorm.restype = i32
+    lib.varq_attn_fwd_qnorm.argtypes = [T, T, T, Q, Q, i32, i32, i32, i32, i32, i32, i32, f32, vp, f32, T, vp, sz, vp]
     return lib
 
 

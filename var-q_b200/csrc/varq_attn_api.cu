@@ -17,15 +17,15 @@ extern "C" size_t varq_attn_workspace_bytes(int32_t B, int32_t H, int32_t Lq, in
     (void)k_store_bits; (void)v_store_bits;
     if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0 || D <= 0) return 0;
     const size_t s1 = attn_small_workspace_bytes(B, H, Lq, Lk, D), s2 = attn_stream_workspace_bytes(B, H, Lq, Lk, D);
-    const size_t s3 = attn_tc_workspace_bytes(B, H, Lk, D);
+    const size_t s3 = attn_tc_workspace_bytes(B, H, Lq, Lk, D);
     const size_t s12 = s1 > s2 ? s1 : s2;
     return s12 > s3 ? s12 : s3;
 }
 
-extern "C" int varq_attn_fwd(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
-                             const varq_qparams_t* kp, const varq_qparams_t* vp, int32_t B, int32_t H, int32_t Lq,
-                             int32_t Lk, int32_t D, int32_t kb, int32_t vb, float softmax_scale,
-                             const varq_tensor_t* out, void* workspace, size_t workspace_bytes, void* stream) {
+static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
+                     const varq_qparams_t* kp, const varq_qparams_t* vp, int32_t B, int32_t H, int32_t Lq,
+                     int32_t Lk, int32_t D, int32_t kb, int32_t vb, float softmax_scale,
+                     const varq_tensor_t* out, void* workspace, size_t workspace_bytes, void* stream, bool q_norm, const float* q_mul, float q_eps) {
     if (!q || !k_codes || !v_codes || !kp || !vp || !out) return fail(VARQ_ERR_ARG, "varq_attn_fwd: null descriptor");
     if ((kb != 2 && kb != 4 && kb != 8) || (vb != 2 && vb != 4 && vb != 8))
         return fail(VARQ_ERR_ARG, "varq_attn_fwd: store bits must be 2, 4 or 8 (got %d, %d)", kb, vb);
@@ -57,6 +57,11 @@ extern "C" int varq_attn_fwd(const varq_tensor_t* q, const varq_tensor_t* k_code
     a.v16 = words_aligned16(v_codes, wv);
     a.scale_log2 = softmax_scale * 1.4426950408889634f;
     a.splits = 1; a.tiles_per_split = 0; a.n_qtiles = 1; a.ws = reinterpret_cast<float*>(workspace);
+    a.q_norm = q_norm ? 1 : 0; a.q_mul = q_mul; a.q_eps = q_eps;
+    if (q_norm) {       // the tensor-core kernel normalises queries as it loads them
+        if (!attn_tc_eligible(a, kb, vb)) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd_qnorm: no kernel normalises the queries of this shape or layout");
+        return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
+    }
     // The CUDA-core streaming kernel is memory-bound only while its arithmetic (queries x keys x head_dim on the FMA pipe)
     // stays below the time to stream the packed cache: up to 4 queries at any cache length, and the 1-16-query first scales
     // of a schedule, whose caches are a few hundred tokens at most.  Everything else goes to the tensor cores, where a
@@ -73,6 +78,20 @@ extern "C" int varq_attn_fwd(const varq_tensor_t* q, const varq_tensor_t* k_code
     const bool want_stream = force ? (force == VARQ_ATTN_PATH_STREAM) : small_q;
     if (want_stream && attn_stream_eligible(a, kb, vb)) return attn_stream_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     return attn_small_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+extern "C" int varq_attn_fwd(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
+                             const varq_qparams_t* kp, const varq_qparams_t* vp, int32_t B, int32_t H, int32_t Lq,
+                             int32_t Lk, int32_t D, int32_t kb, int32_t vb, float softmax_scale,
+                             const varq_tensor_t* out, void* workspace, size_t workspace_bytes, void* stream) {
+    return attn_impl(q, k_codes, v_codes, kp, vp, B, H, Lq, Lk, D, kb, vb, softmax_scale, out, workspace, workspace_bytes, stream, false, nullptr, 0.f);
+}
+
+extern "C" int varq_attn_fwd_qnorm(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
+                                   const varq_qparams_t* kp, const varq_qparams_t* vp, int32_t B, int32_t H, int32_t Lq,
+                                   int32_t Lk, int32_t D, int32_t kb, int32_t vb, float softmax_scale, const float* q_mul, float q_eps,
+                                   const varq_tensor_t* out, void* workspace, size_t workspace_bytes, void* stream) {
+    return attn_impl(q, k_codes, v_codes, kp, vp, B, H, Lq, Lk, D, kb, vb, softmax_scale, out, workspace, workspace_bytes, stream, true, q_mul, q_eps);
 }
 
 extern "C" int varq_attn_force_path(int32_t path) {

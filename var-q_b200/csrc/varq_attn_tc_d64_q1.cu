@@ -1,0 +1,6 @@
+// Tensor-core attention: head_dim 64, 16-bit queries, 1 query tile per CTA.
+#include "varq_attn_tc.cuh"
+
+namespace varq {
+const TcFile tc_d64_q1 = {tc_launch_modes<64, 1, 1>, tc_file_status};
+}
