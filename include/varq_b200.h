@@ -143,6 +143,33 @@ int varq_quant_pack_prestats(const varq_tensor_t* x, int32_t B, int32_t L, int32
                              const varq_tensor_t* codes, const varq_qparams_t* p,
                              void* stats, size_t stats_bytes, void* stream);
 
+/* One tensor of an appended step: what varq_quant_pack takes, plus the cache's bookkeeping for modes that keep one
+ * parameter row per appended step.  row_of_token (or NULL): the entries of this step's L tokens, set to row0.
+ * row_begin (with row_of_token): two entries, set to token0 and token0 + L. */
+typedef struct {
+    varq_tensor_t x;
+    int32_t bits, store_bits;
+    float eps;
+    int32_t token0, row0, _pad;
+    varq_tensor_t codes;
+    varq_qparams_t p;
+    int32_t* row_of_token;
+    int32_t* row_begin;
+} varq_append_job_t;
+
+/* Quantize + pack the K and V of an appended step (one or two jobs of the same B, L, H, D) -- in a single launch for
+ * per-token-per-head, short per-dim and small per-token steps of 16-byte aligned inputs, otherwise through varq_quant_pack.
+ * first_norm_eps >= 0: the rows of the first job (K) are replaced by x / max(||x||_2, first_norm_eps) on the way in
+ * (VAR/models/basic_var.py:137-141); VARQ_ERR_UNSUPPORTED where no kernel does that.  Workspace:
+ * varq_append_workspace_bytes(); a call that needs more (per-token-per-head groups in a layout without the single-pass
+ * kernel) fails with VARQ_ERR_WORKSPACE and wants varq_quant_workspace_bytes().  Same codes and parameters as
+ * varq_quant_pack.
+ * Replaces VAR_Q.quant + VAR_Q.cache for both tensors (VAR_Q/quant.py:140-205). */
+size_t varq_append_workspace_bytes(const varq_append_job_t* jobs, int32_t n_jobs, int32_t B, int32_t L, int32_t H, int32_t D,
+                                   float first_norm_eps);
+int varq_append(const varq_append_job_t* jobs, int32_t n_jobs, int32_t B, int32_t L, int32_t H, int32_t D,
+                float first_norm_eps, void* workspace, size_t workspace_bytes, void* stream);
+
 /* varq_quant_pack for callers that may not allocate device memory and have no scratch
  * buffer to lend.  No counterpart in the reference.
  *

@@ -22,7 +22,7 @@ SYMBOLS = (
     "varq_quant_workspace_bytes", "varq_quant_pack", "varq_quant_pack_static",
     "varq_quant_static_scratch_bytes", "varq_unpack_dequant",
     "varq_attn_workspace_bytes", "varq_attn_fwd", "varq_attn_force_path",
-    "varq_qk_norm_stats", "varq_quant_pack_prestats", "varq_attn_fwd_qnorm",
+    "varq_qk_norm_stats", "varq_quant_pack_prestats", "varq_attn_fwd_qnorm", "varq_append", "varq_append_workspace_bytes",
 )
 
 
@@ -38,6 +38,12 @@ class QParams(ctypes.Structure):
                 ("share_b", ctypes.c_int32), ("share_l", ctypes.c_int32), ("share_h", ctypes.c_int32),
                 ("group", ctypes.c_int32),
                 ("row_begin", ctypes.c_void_p), ("n_rows", ctypes.c_int32), ("_pad", ctypes.c_int32)]
+
+
+class AppendJob(ctypes.Structure):
+    _fields_ = [("x", Tensor), ("bits", ctypes.c_int32), ("store_bits", ctypes.c_int32), ("eps", ctypes.c_float),
+                ("token0", ctypes.c_int32), ("row0", ctypes.c_int32), ("_pad", ctypes.c_int32), ("codes", Tensor), ("p", QParams),
+                ("row_of_token", ctypes.c_void_p), ("row_begin", ctypes.c_void_p)]
 
 
 _lib = None
@@ -79,6 +85,10 @@ def _declare(lib):
     lib.varq_attn_force_path.argtypes = [i32]
     lib.varq_attn_fwd.restype = i32
     lib.varq_attn_fwd.argtypes = [T, T, T, Q, Q, i32, i32, i32, i32, i32, i32, i32, f32, T, vp, sz, vp]
+    lib.varq_append_workspace_bytes.restype = sz
+    lib.varq_append_workspace_bytes.argtypes = [ctypes.POINTER(AppendJob), i32, i32, i32, i32, i32, f32]
+    lib.varq_append.restype = i32
+    lib.varq_append.argtypes = [ctypes.POINTER(AppendJob), i32, i32, i32, i32, i32, f32, vp, sz, vp]
     lib.varq_attn_fwd_qnorm.restype = i32
     lib.varq_attn_fwd_qnorm.argtypes = [T, T, T, Q, Q, i32, i32, i32, i32, i32, i32, i32, f32, vp, f32, T, vp, sz, vp]
     return lib

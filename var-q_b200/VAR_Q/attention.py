@@ -10,7 +10,7 @@ from typing import Optional
 import torch
 
 from . import _cabi
-from .quant import VAR_Q
+from .quant import VAR_Q, _host
 
 
 def attend_cached(q: torch.Tensor, k_quant: VAR_Q, v_quant: VAR_Q, softmax_scale: float,
@@ -20,6 +20,10 @@ def attend_cached(q: torch.Tensor, k_quant: VAR_Q, v_quant: VAR_Q, softmax_scale
     ``q`` is in the quantizers' ``qkv_format``.  Returns ``[B, Lq, H, c]`` (contiguous), which
     both hook sites immediately view as ``[B, Lq, H*c]``.
     """
+    if _host is not None:
+        out = _host.attend(q, k_quant, v_quant, softmax_scale, out_dtype)
+        if out is not None:
+            return out
     _cabi.require_cuda(q, "q")
     if k_quant.n_tokens == 0 or k_quant.n_tokens != v_quant.n_tokens:
         raise ValueError("[VAR-Q]: K and V caches must hold the same, non-zero number of tokens")
@@ -53,6 +57,10 @@ def attend_cached(q: torch.Tensor, k_quant: VAR_Q, v_quant: VAR_Q, softmax_scale
 def attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_quant: VAR_Q, v_quant: VAR_Q,
            softmax_scale: float, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """Quantize and append this step's K and V, then attend over everything cached."""
+    if _host is not None:
+        out = _host.step(q, k, v, k_quant, v_quant, softmax_scale, out_dtype)
+        if out is not None:
+            return out
     k_quant.append(k)
     v_quant.append(v)
     return attend_cached(q, k_quant, v_quant, softmax_scale, out_dtype)

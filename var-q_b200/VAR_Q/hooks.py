@@ -22,7 +22,7 @@ import torch
 
 from . import _cabi
 from .attention import attend, attend_cached
-from .quant import VAR_Q
+from .quant import VAR_Q, _host
 
 
 class LayerKV:
@@ -138,7 +138,13 @@ def normalise_qk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_quant: VAR
 
 
 def _step_normalised(self, q, k, v, scale_mul, softmax_scale, out_dtype=None):
-    """``LayerKV.step`` with the L2-normalisation of q and k (and the statistics pass of column groupings) fused in front."""
+    """``LayerKV.step`` with the L2-normalisation of q and k fused in: k is normalised inside the quantize launch and q as the
+    attention kernel loads it, so neither is stored.  Groupings and layouts without such kernels take the separate producer
+    kernel (``normalise_qk``) in front of the ordinary step."""
+    if _host is not None:
+        out = _host.step_normalised(q, k, v, scale_mul, self.k_quant, self.v_quant, softmax_scale, out_dtype, 1e-12)
+        if out is not None:
+            return out
     qn, kn, ks, vs = normalise_qk(q, k, v, self.k_quant, self.v_quant, scale_mul)
     self.k_quant.append(kn, ks)
     self.v_quant.append(v, vs)

@@ -30,6 +30,11 @@ import torch
 
 from . import _cabi
 
+try:
+    from . import _host                 # native state and call path (csrc_host/)
+except ImportError:                     # not built yet: construction and configuration work, device calls say what is missing
+    _host = None
+
 _METHODS = ('G_TENSOR', 'G_SCALE_HEAD_DIM', 'G_HEAD_DIM', 'G_SCALE', 'G_TOKEN', 'G_TOKEN_HEAD')
 _REQUANT = ('G_HEAD_DIM', 'G_TENSOR')
 # method -> (share_l, share_h, per_dim)
@@ -44,7 +49,21 @@ def _round_up(n: int, m: int) -> int:
     return (n + m - 1) // m * m
 
 
-class VAR_Q:
+_STATE = ('quant_bits', 'quant_method', 'pack_to_int32', 'symmetric', 'reduce_batch', 'group_size', '_max_tokens', 'debug', '_fmt',
+          'eps', '_shape', '_pending', '_last', '_pack_meta', '_words', '_nB', '_nH', '_nG', '_lcap', '_rcap', '_n_tokens', '_n_rows',
+          '_codes', '_codes_next', '_scale_tbl', '_zp_tbl', '_scale_next', '_zp_next', '_row_of_token', '_row_begin')
+
+
+class _Unbuilt:
+    """Stands in for the native state while the host extension is not built."""
+
+    def __init__(self):
+        for name in _STATE:
+            setattr(self, name, None)
+        self._n_tokens = self._n_rows = self._lcap = self._rcap = 0
+
+
+class VAR_Q(_host.Cache if _host is not None else _Unbuilt):
     def __init__(
         self,
         quant_bits: int = 8,
@@ -67,6 +86,7 @@ class VAR_Q:
             raise ValueError("[VAR-Q]: group_size is defined for quant_method='G_TOKEN_HEAD' only")
         if not reduce_batch and quant_method not in ('G_TOKEN', 'G_TOKEN_HEAD'):
             raise ValueError("[VAR-Q]: reduce_batch=False is defined for G_TOKEN and G_TOKEN_HEAD only")
+        super().__init__()
         self.quant_bits = int(quant_bits)
         self.quant_method = quant_method
         self.cur_blk_idx = blk_idx
@@ -79,18 +99,24 @@ class VAR_Q:
         self.bound_min = -(2 ** (quant_bits - 1))
         self.bound_max = (2 ** (quant_bits - 1)) - 1
         self.qkv_format = qkv_format          # property: derives dim_cat / dim_map
-        self._pack_meta: Optional[Dict[str, int]] = None
         self._max_tokens = max_tokens
-        # device state, allocated at the first quant()
-        self._codes = self._codes_next = None   # int32 [B, H, Lcap, W]
-        self._scale_tbl = self._zp_tbl = None   # fp32 [nB, nH, Rcap, nG]
-        self._scale_next = self._zp_next = None
-        self._row_of_token = None               # int32 [Lcap] (per-step tables only)
-        self._row_begin = None                  # int32 [Rcap + 1]: first token of every row (per-step tables only)
-        self._shape = None                      # (B, H, D)
-        self._n_tokens = self._n_rows = 0       # committed by cache()
-        self._pending = None                    # (tokens, rows, replaces_cache)
-        self._last = None                       # (tokens, rows) of the step committed last
+        # The state (native, empty until the first quant()):
+        #   _codes, _codes_next            int32 [B, H, Lcap, W]
+        #   _scale_tbl, _zp_tbl (, _next)  fp32 [nB, nH, Rcap, nG]
+        #   _row_of_token                  int32 [Lcap] (per-step tables only)
+        #   _row_begin                     int32 [Rcap + 1]: first token of every row (per-step tables only)
+        #   _shape                         (B, H, D)
+        #   _n_tokens, _n_rows             committed by cache()
+        #   _pending                       (tokens, rows, replaces_cache)
+        #   _last                          (tokens, rows) of the step committed last
+        #   _pack_meta                     the reference's packing record
+
+    def __getstate__(self):
+        return {**self.__dict__, **{name: getattr(self, name) for name in _STATE}}
+
+    def __setstate__(self, state):
+        for name, value in state.items():
+            setattr(self, name, value)
 
     # ------------------------------------------------------------------ layout
     @property
@@ -247,6 +273,8 @@ class VAR_Q:
     def quant(self, item: torch.Tensor, stats: Optional[torch.Tensor] = None):
         """Quantize one appended step (VAR_Q/quant.py:140-177).  `stats`: statistics table of this very tensor as left by
         ``varq_qk_norm_stats`` (see ``column_grouping``); the kernel then skips its own statistics pass."""
+        if stats is None and _host is not None and _host.append(self, item, False):
+            return
         _cabi.require_cuda(item, "item")
         if item.dim() != 4:
             raise ValueError(f"[VAR-Q]: item must be 4-D ({self._fmt}), got {tuple(item.shape)}")
@@ -317,6 +345,9 @@ class VAR_Q:
 
     def dequant_current(self) -> torch.Tensor:
         """fp32 dequantisation of the step quantized last (VAR_Q/quant.py:208-214)."""
+        out = _host.dequant(self, 1) if _host is not None else None
+        if out is not None:
+            return out
         if self._pending is None and self._n_tokens:
             # after cache(): the reference's `quantized_item` still names the last step
             n, rows = self._last
@@ -327,12 +358,18 @@ class VAR_Q:
 
     def dequant_all(self) -> torch.Tensor:
         """fp32 dequantisation of the whole cache (VAR_Q/quant.py:216-224)."""
+        out = _host.dequant(self, 0) if _host is not None else None
+        if out is not None:
+            return out
         if self._n_tokens == 0:
             return self.dequant_current()
         return self._dequant(self._codes, self._scale_tbl, self._zp_tbl, 0, self._n_tokens, 0, self._row_of_token)
 
     def use_var_q(self, item: torch.Tensor) -> torch.Tensor:
         """quant -> cache -> dequant_all (VAR_Q/quant.py:227-230)."""
+        out = _host.use_var_q(self, item) if _host is not None else None
+        if out is not None:
+            return out
         self.quant(item)
         self.cache()
         if self.debug:
@@ -342,6 +379,8 @@ class VAR_Q:
     # ------------------------------------------------------------------ fused path
     def append(self, item: torch.Tensor, stats: Optional[torch.Tensor] = None):
         """quant + cache without materialising the dequantised cache."""
+        if stats is None and _host is not None and not self.debug and _host.append(self, item, True):
+            return
         self.quant(item, stats)
         self.cache()
         if self.debug:

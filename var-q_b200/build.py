@@ -1,4 +1,4 @@
-"""Build libvarq_b200.so in-tree with nvcc for sm_100a.
+"""Build libvarq_b200.so (nvcc, sm_100a) and the host extension _host.so (g++, CPython over ATen) in-tree.
 
     python var-q_b200/build.py [--force] [--verbose]
 
@@ -17,6 +17,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "VAR_Q", "libvarq_b200.so")
+HOST_SRC = os.path.join(HERE, "csrc_host", "varq_host.cpp")
+HOST_PATH = os.path.join(HERE, "VAR_Q", "_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -43,9 +45,34 @@ def is_stale():
     return any(os.path.getmtime(p) > built for p in deps)
 
 
+def build_host(force=False, verbose=False):
+    """Compile the host extension against the installed torch; it links to libvarq_b200.so next to it."""
+    header = os.path.join(INCLUDE, "varq_b200.h")
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) > max(os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
+        return HOST_PATH
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda_home = os.path.dirname(os.path.dirname(find_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", INCLUDE, "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda_home, "include")]
+    for p in cpp_extension.include_paths():
+        cmd += ["-isystem", p]
+    cmd += [HOST_SRC, "-o", HOST_PATH, "-L", os.path.dirname(LIB_PATH), "-l:libvarq_b200.so", "-Wl,-rpath,$ORIGIN", "-L", torch_lib,
+            "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed building _host.so")
+    return HOST_PATH
+
+
 def build_library(force=False, verbose=False):
-    """Compile every .cu of csrc/ into one shared library; returns its path."""
+    """Compile every .cu of csrc/ into one shared library, and the host extension; returns the library's path."""
     if not force and not is_stale():
+        build_host()
         return LIB_PATH
     cmd = [find_nvcc()] + NVCC_FLAGS + ["-I", INCLUDE, "-I", CSRC]
     if verbose:
@@ -56,6 +83,7 @@ def build_library(force=False, verbose=False):
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed building libvarq_b200.so")
+    build_host(force=force, verbose=verbose)
     return LIB_PATH
 
 

@@ -1,4 +1,4 @@
-// Fused quantize + pack of fresh K/V.
+// Fused quantize + pack of fresh K/V: the groupings and layouts that the append kernels (varq_append.cu) do not take, and the entry points.
 //
 // Two device paths, both with one thread per packed int32 word (4 / 8 / 16 inputs):
 //   * rows path   - groups that keep (token, head) [per-token-per-head, optionally split
@@ -8,7 +8,7 @@
 //                   kernel folds min/max into a small table with integer atomics on an
 //                   order-preserving encoding, a second kernel quantizes.
 // Arithmetic is fp32 with true division and round-half-even, the clamp after the round.
-#include "varq_common.cuh"
+#include "varq_quant.cuh"
 
 namespace varq {
 
@@ -29,34 +29,6 @@ struct QuantArgs {
     int l_fixed;                        // tables path: the row stride is a multiple of L, so a thread keeps its token index
 };
 
-struct Range { uint32_t hi, lo; };      // hi = max f2ord(x or |x|), lo = max ~f2ord(x)
-
-__device__ __forceinline__ void range_init(Range& r) { r.hi = 0u; r.lo = 0u; }
-__device__ __forceinline__ void range_add(Range& r, float v, bool symmetric) {
-    if (symmetric) {
-        r.hi = max(r.hi, f2ord(fabsf(v)));
-    } else {
-        const uint32_t o = f2ord(v);
-        r.hi = max(r.hi, o);
-        r.lo = max(r.lo, ~o);
-    }
-}
-__device__ __forceinline__ void range_merge(Range& r, const Range& o) { r.hi = max(r.hi, o.hi); r.lo = max(r.lo, o.lo); }
-
-// scale / zero-point of a group from its range
-__device__ __forceinline__ void params_from_range(const Range& r, int bits, bool symmetric, float eps, float& scale,
-                                                  float& zp) {
-    if (symmetric) {
-        const float amax = ord2f(r.hi);
-        scale = fmaxf(__fdiv_rn(amax, (float)((1 << (bits - 1)) - 1)), eps);
-        zp = 0.0f;
-    } else {
-        const float mx = ord2f(r.hi), mn = ord2f(~r.lo);
-        scale = fmaxf(__fdiv_rn(__fsub_rn(mx, mn), (float)((1 << bits) - 1)), eps);
-        zp = __fadd_rn(rintf(__fsub_rn(-(float)(1 << (bits - 1)), __fdiv_rn(mn, scale))), 0.0f);
-    }
-}
-
 // Per-group constants of the division-free quantizer.  RN(x / scale) lies strictly between
 // x * rcp_lo and x * rcp_hi (rcp_lo/hi = RN(1/scale) * (1 -/+ 2^-21)), and rint is monotonic, so
 // when both ends round to the same integer that integer is the reference's code; otherwise (about
@@ -65,7 +37,6 @@ __device__ __forceinline__ void params_from_range(const Range& r, int bits, bool
 struct GroupQ {
     float scale, zp, rcp_lo, rcp_hi;
 };
-constexpr float Q_MAGIC = 12582912.0f;
 __device__ __forceinline__ GroupQ make_group_q(float scale, float zp) {
     GroupQ g;
     const float rcp = __frcp_rn(scale);
@@ -252,89 +223,6 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(QuantArgs a, RowPlan pl
     }
 }
 
-
-// =====================================================================================
-// lean rows path: groups shared over the batch, every thread holds a full set of vectors
-// =====================================================================================
-struct LeanPlan {
-    int tpr, bp, ngr, lpg, h_fast;
-    int xs_row_in, xs_row_out;     // element strides of the inner / outer coordinate of a group row
-    int cs_row_in, cs_row_out, ps_row_in, ps_row_out;
-    int n_in;                      // size of the inner coordinate (H if h_fast else L)
-    int xs_bstep, cs_bstep;        // bp * batch stride (elements / words)
-};
-
-template <typename T, int STORE_BITS, bool SYM>
-__global__ void __launch_bounds__(256) quant_rows_lean_kernel(QuantArgs a, LeanPlan pl) {
-    constexpr int VPW = 32 / STORE_BITS;
-    constexpr int NV = 32 / VPW;
-    __shared__ uint32_t s_stats[256];          // [ngr * groups per row][2]
-    const int tid = threadIdx.x;
-    const int w = tid % pl.tpr;
-    const int rest = tid / pl.tpr;
-    const int g_local = rest % pl.ngr;
-    const int bl = rest / pl.ngr;
-    const int d0 = w * VPW;
-    const int gpr = a.D / a.group;
-    const unsigned gr = blockIdx.x * (unsigned)pl.ngr + g_local;
-    const int r_in = (int)(gr % (unsigned)pl.n_in), r_out = (int)(gr / (unsigned)pl.n_in);
-    const int x0 = bl * (int)a.xs_b + r_in * pl.xs_row_in + r_out * pl.xs_row_out + d0;
-    const int c0 = bl * (int)a.cs_b + r_in * pl.cs_row_in + r_out * pl.cs_row_out + w;
-
-    if (pl.bp > 1) {
-        if (tid < pl.ngr * gpr * 2) s_stats[tid] = 0u;
-        __syncthreads();
-    }
-    float v[NV][VPW];
-    const T* xp = reinterpret_cast<const T*>(a.x) + x0;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) load_vals<T, VPW, true>(xp + k * pl.xs_bstep, v[k], VPW);
-
-    // statistics in float registers; the order-preserving integer form is only needed for the shared atomics
-    float hi = SYM ? 0.f : v[0][0], lo = v[0][0];
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-#pragma unroll
-        for (int j = 0; j < VPW; ++j) {
-            if (SYM) hi = fmaxf(hi, fabsf(v[k][j]));
-            else { hi = fmaxf(hi, v[k][j]); lo = fminf(lo, v[k][j]); }
-        }
-    for (int m = 1; m < pl.lpg; m <<= 1) {
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, m));
-        if (!SYM) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, m));
-    }
-    Range rg;
-    rg.hi = f2ord(hi);
-    rg.lo = SYM ? 0u : ~f2ord(lo);
-    if (pl.bp > 1) {
-        const int slot = (g_local * gpr + d0 / a.group) * 2;
-        if ((w % pl.lpg) == 0) {
-            atomicMax(&s_stats[slot], rg.hi);
-            if (!SYM) atomicMax(&s_stats[slot + 1], rg.lo);
-        }
-        __syncthreads();
-        rg.hi = s_stats[slot];
-        rg.lo = s_stats[slot + 1];
-    }
-    float scale, zp;
-    params_from_range(rg, a.bits, SYM, a.eps, scale, zp);
-    const GroupQ gq = make_group_q(scale, zp);
-    const CodeRange cr = make_code_range(a.bits);
-    int32_t* cp = a.codes + c0;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int j = 0; j < VPW; ++j)
-            word |= (quant_code<SYM>(v[k][j], gq, cr) & ((1u << STORE_BITS) - 1u)) << (j * STORE_BITS);
-        cp[k * pl.cs_bstep] = (int32_t)word;
-    }
-    if (bl == 0 && (d0 % a.group) == 0) {
-        const long long pi = (long long)r_in * pl.ps_row_in + (long long)r_out * pl.ps_row_out + (long long)(d0 / a.group) * a.ps_g;
-        a.scale[pi] = scale;
-        if (!SYM) a.zp[pi] = zp;
-    }
-}
 
 // =====================================================================================
 // tables path: blockDim = (TX column slots, TY rows); a column slot is one word of one head
@@ -667,33 +555,6 @@ static bool plan_rows(const QuantArgs& a, int vpw, bool vec, RowPlan& pl, int& t
     return threads % 32 == 0 && threads <= 256;
 }
 
-// The lean kernel applies when the batch is shared, fills every register slot (B = bp * NV) and
-// all offsets fit 32 bits.
-static bool plan_lean(const QuantArgs& a, int vpw, bool vec, const RowPlan& rp, LeanPlan& lp, long long x_extent) {
-    if (!vec || !a.share_b || a.share_l || a.share_h) return false;
-    const int nv = 32 / vpw;
-    if (rp.bp * nv != a.B || rp.nv != nv) return false;
-    if (rp.n_gr % rp.ngr != 0) return false;
-    if (rp.ngr * (a.D / a.group) * 2 > 256) return false;
-    const long long c_extent = (long long)a.B * a.cs_b;
-    if (x_extent >= 0x7fffffffLL || c_extent >= 0x7fffffffLL || x_extent < 0) return false;
-    lp.tpr = rp.tpr; lp.bp = rp.bp; lp.ngr = rp.ngr; lp.lpg = rp.lpg; lp.h_fast = rp.h_fast;
-    if (rp.h_fast) {
-        lp.n_in = a.H;
-        lp.xs_row_in = (int)a.xs_h; lp.xs_row_out = (int)a.xs_l;
-        lp.cs_row_in = (int)a.cs_h; lp.cs_row_out = (int)a.cs_l;
-        lp.ps_row_in = (int)a.ps_h; lp.ps_row_out = (int)a.ps_r;
-    } else {
-        lp.n_in = a.L;
-        lp.xs_row_in = (int)a.xs_l; lp.xs_row_out = (int)a.xs_h;
-        lp.cs_row_in = (int)a.cs_l; lp.cs_row_out = (int)a.cs_h;
-        lp.ps_row_in = (int)a.ps_r; lp.ps_row_out = (int)a.ps_h;
-    }
-    lp.xs_bstep = rp.bp * (int)a.xs_b;
-    lp.cs_bstep = rp.bp * (int)a.cs_b;
-    return true;
-}
-
 // `have_stats`: the statistics table in `ws` is already filled (by varq_qk_norm_stats); only finalize + apply run.
 template <typename T, int SB>
 static int launch_quant(const QuantArgs& a0, bool vec, void* ws, size_t ws_bytes, cudaStream_t st, bool have_stats = false) {
@@ -706,15 +567,6 @@ static int launch_quant(const QuantArgs& a0, bool vec, void* ws, size_t ws_bytes
         const long long per_cta = a.share_b ? pl.ngr : (long long)pl.ngr * pl.nv;
         const long long blocks = (pl.n_gr + per_cta - 1) / per_cta;
         if (blocks > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_quant_pack: tensor too large");
-        LeanPlan lp;
-        const long long x_extent = (long long)(a.B - 1) * a.xs_b + (long long)(a.L - 1) * a.xs_l + (long long)(a.H - 1) * a.xs_h + a.D;
-        if (plan_lean(a, VPW, vec, pl, lp, x_extent)) {
-            if (a.symmetric) quant_rows_lean_kernel<T, SB, true><<<(unsigned)blocks, threads, 0, st>>>(a, lp);
-            else             quant_rows_lean_kernel<T, SB, false><<<(unsigned)blocks, threads, 0, st>>>(a, lp);
-            VARQ_CUDA_TRY(cudaGetLastError());
-            count_launches(1);
-            return VARQ_OK;
-        }
         quant_rows_kernel<T, SB><<<(unsigned)blocks, threads, smem, st>>>(a, pl);
         VARQ_CUDA_TRY(cudaGetLastError());
         count_launches(1);
@@ -825,6 +677,12 @@ static int quant_pack_impl(const char* fn, const varq_tensor_t* x, int32_t B, in
     if ((long long)B * L * H == 0) return VARQ_OK;
     if (!x->ptr || !codes->ptr || !p->scale) return fail(VARQ_ERR_ARG, "%s: null pointer", fn);
 
+    if (!have_stats) {       // per-token-per-head groups over the batch, and per-dim groups, of aligned inputs
+        varq_append_job_t job = {};
+        job.x = *x; job.bits = bits; job.store_bits = store_bits; job.eps = eps; job.codes = *codes; job.p = *p;
+        const int rc = append_fast(&job, 1, B, L, H, D, -1.f, workspace, workspace_bytes, (cudaStream_t)stream);
+        if (rc != VARQ_ERR_UNSUPPORTED) return rc;
+    }
     const int vpw = 32 / store_bits;
     QuantArgs a;
     a.x = x->ptr; a.xs_b = x->stride_b; a.xs_l = x->stride_l; a.xs_h = x->stride_h;
@@ -854,6 +712,59 @@ extern "C" int varq_quant_pack_prestats(const varq_tensor_t* x, int32_t B, int32
                                         int32_t store_bits, float eps, const varq_tensor_t* codes, const varq_qparams_t* p,
                                         void* stats, size_t stats_bytes, void* stream) {
     return quant_pack_impl("varq_quant_pack_prestats", x, B, L, H, D, bits, store_bits, eps, codes, p, stats, stats_bytes, stream, true);
+}
+
+// =====================================================================================
+// Append: K and V of a step, with the bookkeeping tables of per-step parameters
+// =====================================================================================
+namespace varq {
+__global__ void __launch_bounds__(256) step_rows_kernel(int32_t* row_of_token, int32_t* row_begin, int token0, int row0, int L) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < L) row_of_token[i] = row0;
+    if (i == 0) { row_begin[0] = token0; row_begin[1] = token0 + L; }
+}
+}  // namespace varq
+
+extern "C" size_t varq_append_workspace_bytes(const varq_append_job_t* jobs, int32_t n_jobs, int32_t B, int32_t L, int32_t H, int32_t D, float first_norm_eps) {
+    if (!jobs || n_jobs < 1 || n_jobs > 2 || B <= 0 || L <= 0 || H <= 0 || D <= 0) return 0;
+    size_t bytes = append_workspace_bytes(jobs, n_jobs, B, L, H, D, first_norm_eps);
+    for (int i = 0; i < n_jobs; ++i) {
+        // (per-token-per-head groups take a table only in unusual layouts, as large as their parameters: not worth asking for up front)
+        const size_t t = jobs[i].p.share_b && !jobs[i].p.share_l && !jobs[i].p.share_h ? 0
+                       : varq_quant_workspace_bytes(B, L, H, D, jobs[i].x.dtype, jobs[i].store_bits, &jobs[i].p);
+        if (t > bytes) bytes = t;
+    }
+    return bytes;
+}
+
+extern "C" int varq_append(const varq_append_job_t* jobs, int32_t n_jobs, int32_t B, int32_t L, int32_t H, int32_t D, float first_norm_eps,
+                           void* workspace, size_t workspace_bytes, void* stream) {
+    if (!jobs || n_jobs < 1 || n_jobs > 2) return fail(VARQ_ERR_ARG, "varq_append: one or two jobs");
+    if (B < 0 || L < 0 || H < 0 || D <= 0) return fail(VARQ_ERR_ARG, "varq_append: bad shape (%d,%d,%d,%d)", B, L, H, D);
+    for (int i = 0; i < n_jobs; ++i) {
+        const varq_append_job_t& j = jobs[i];
+        if (j.bits < 2 || j.bits > 8 || (j.store_bits != 2 && j.store_bits != 4 && j.store_bits != 8) || j.store_bits < j.bits)
+            return fail(VARQ_ERR_ARG, "varq_append: bits must be in [2, 8] and fit store_bits 2, 4 or 8 (got %d, %d)", j.bits, j.store_bits);
+        if (!dtype_ok(j.x.dtype)) return fail(VARQ_ERR_ARG, "varq_append: bad input dtype %d", j.x.dtype);
+        if (int rc = check_grouping("varq_append", &j.p, D)) return rc;
+        if ((j.row_of_token == nullptr) != (j.row_begin == nullptr)) return fail(VARQ_ERR_ARG, "varq_append: row_of_token and row_begin go together");
+        if ((long long)B * L * H != 0 && (!j.x.ptr || !j.codes.ptr || !j.p.scale)) return fail(VARQ_ERR_ARG, "varq_append: null pointer");
+    }
+    if ((long long)B * L * H == 0) return VARQ_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int rc = append_fast(jobs, n_jobs, B, L, H, D, first_norm_eps, workspace, workspace_bytes, st);
+    if (rc != VARQ_ERR_UNSUPPORTED) return rc;
+    if (first_norm_eps >= 0.f) return fail(VARQ_ERR_UNSUPPORTED, "varq_append: no kernel normalises rows of this layout or grouping");
+    for (int i = 0; i < n_jobs; ++i) {
+        const varq_append_job_t& j = jobs[i];
+        if (int r = quant_pack_impl("varq_append", &j.x, B, L, H, D, j.bits, j.store_bits, j.eps, &j.codes, &j.p, workspace, workspace_bytes, stream, false)) return r;
+        if (j.row_of_token) {
+            step_rows_kernel<<<(L + 255) / 256, 256, 0, st>>>(j.row_of_token, j.row_begin, j.token0, j.row0, L);
+            VARQ_CUDA_TRY(cudaGetLastError());
+            count_launches(1);
+        }
+    }
+    return VARQ_OK;
 }
 
 // =====================================================================================
