@@ -44,6 +44,7 @@ struct AppendJob {
     int group;
     // rows kernel
     int bp, nv, ngr, h_fast;
+    unsigned div_m, div_s;            // division by the inner extent as multiply-high + add + shift
     unsigned blocks;
     // planes
     long long xs_out, xs_in, cs_out, cs_in, ps_out;
@@ -77,6 +78,11 @@ template <typename T, bool SYM> struct RangeAcc {               // fp32 values
 #pragma unroll
         for (int j = 0; j < 8; ++j) { h[j] = hi[j]; l[j] = lo[j]; }
     }
+    __device__ __forceinline__ void fold(float& h, float& l) const {
+        h = hi[0]; l = lo[0];
+#pragma unroll
+        for (int j = 1; j < 8; ++j) { h = fmaxf(h, hi[j]); l = fminf(l, lo[j]); }
+    }
 };
 template <typename T2, typename T, bool SYM> struct RangeAcc16 {
     T2 hi[4], lo[4];
@@ -95,6 +101,10 @@ template <typename T2, typename T, bool SYM> struct RangeAcc16 {
         memcpy(&b.r, lo, 16);
         a.get(h);
         b.get(l);
+    }
+    __device__ __forceinline__ void fold(float& h, float& l) const {
+        const T2 a = __hmax2(__hmax2(hi[0], hi[1]), __hmax2(hi[2], hi[3])), b = __hmin2(__hmin2(lo[0], lo[1]), __hmin2(lo[2], lo[3]));
+        h = fmaxf(to_f32<T>(a.x), to_f32<T>(a.y)); l = fminf(to_f32<T>(b.x), to_f32<T>(b.y));
     }
 };
 template <bool SYM> struct RangeAcc<__nv_bfloat16, SYM> : RangeAcc16<__nv_bfloat162, __nv_bfloat16, SYM> {
@@ -146,34 +156,60 @@ template <int SB> __device__ __forceinline__ uint2 pack8(const float (&y)[8]) {
     if constexpr (SB == 8) return make_uint2(pack_fields<8, 4>(y), pack_fields<8, 4>(y + 4));
     else return make_uint2(pack_fields<SB, 8>(y), 0u);
 }
-// PER_VALUE: parameters per value position (columns; scale and zero-point from s_par on the rare path), else one set
-template <int SB, bool SYM, bool PER_VALUE>
-__device__ __forceinline__ uint2 quantize8(const float (&x)[8], float rlen, float length, const float* lo, const float* hi, const float* magic, const float* scale,
+// Where the brackets disagree the quotient lies next to t = k + 1/2, k and k + 1 the two ends, and no division is needed: the residual
+// r = x - t * scale is exact (t has few bits and the difference cancels), so its sign tells on which side of t the exact quotient lies,
+// and the rounded quotient is t itself iff |r| <= scale * ulp(t) / 2; then the even end is the code.  (Below 1/2 floats are twice as
+// dense, but both outcomes give 0 there.)  16-bit inputs of few distinct values hit such ties often.
+__device__ __forceinline__ float settle(float x, float lo, float hi, float magic, float scale) {
+    const float ka = fmaf(x, lo, magic) - magic, kb = fmaf(x, hi, magic) - magic;
+    const float t = 0.5f * (ka + kb);
+    const float r = fmaf(-t, scale, x), half_ulp = __uint_as_float(__float_as_uint(t) & 0x7f800000u) * 5.9604645e-8f;
+    float k = (t + Q_MAGIC) - Q_MAGIC;                  // the ends agree: that integer; a tie: the even end
+    if (ka != kb && fabsf(r) > scale * half_ulp) k = r > 0.f ? fmaxf(ka, kb) : fminf(ka, kb);
+    return magic + k;
+}
+// PER_VALUE: parameters per value position (columns), else one set
+template <int SB, bool SYM, bool NORM, bool PER_VALUE>
+__device__ __forceinline__ uint2 quantize8(const float (&x)[8], float length, const float* lo, const float* hi, const float* magic, const float* scale,
                                            float q_min, float q_max) {
     float y[8];
     bool bad = false;
+    const float rlen = NORM ? __frcp_rn(length) : 1.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int z = PER_VALUE ? j : 0;
-        const float v = length > 0.f ? x[j] * rlen : x[j];       // (`length` is the constant 0 where rows are taken as they are)
+        const float v = NORM ? x[j] * rlen : x[j];
         y[j] = fmaf(v, hi[z], magic[z]);
         bad = bad | (y[j] != fmaf(v, lo[z], magic[z]));
     }
     if (bad) {
-        float t[8];                                    // indexed at run time: local memory, touched on this path only
+        bool divide = NORM;
+        if (!NORM && !SYM) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = x[j];
-#pragma unroll 1
-        for (int j = 0; j < 8; ++j) {
-            float m = magic[0];
-            if (PER_VALUE) {
-#pragma unroll
-                for (int z = 1; z < 8; ++z) m = j == z ? magic[z] : m;
-            }
-            t[j] = exact_code(t[j], length, scale[PER_VALUE ? j : 0], SYM ? 0.f : m - Q_MAGIC, q_min, q_max);
+            for (int z = 0; z < (PER_VALUE ? 8 : 1); ++z) divide = divide | (lo[z] != lo[z]);
         }
+        if (divide) {
+            float t[8];                                // indexed at run time: local memory, touched on this path only
 #pragma unroll
-        for (int j = 0; j < 8; ++j) y[j] = t[j];
+            for (int j = 0; j < 8; ++j) t[j] = x[j];
+#pragma unroll 1
+            for (int j = 0; j < 8; ++j) {
+                float m = magic[0];
+                if (PER_VALUE) {
+#pragma unroll
+                    for (int z = 1; z < 8; ++z) m = j == z ? magic[z] : m;
+                }
+                t[j] = exact_code(t[j], NORM ? length : 0.f, scale[PER_VALUE ? j : 0], SYM ? 0.f : m - Q_MAGIC, q_min, q_max);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) y[j] = t[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int z = PER_VALUE ? j : 0;
+                y[j] = settle(x[j], lo[z], hi[z], magic[z], scale[z]);
+            }
+        }
     }
     if (!SYM) {           // a symmetric code cannot leave its range: |x| <= amax
 #pragma unroll
@@ -195,24 +231,31 @@ template <int SB> __device__ __forceinline__ void store8(int32_t* row, int w, co
 // rows: one (token, head) row of every sample of the batch per D / 8 x bp threads
 // =====================================================================================
 constexpr int ROWS_NV = 4;              // samples per thread
+// (token, head) of group row r
+struct RowAt { long long l, h; };
+__device__ __forceinline__ RowAt row_at(const AppendArgs& a, const AppendJob& jb, unsigned r) {
+    const unsigned q = (unsigned)((__umulhi(r, jb.div_m) + (unsigned long long)r) >> jb.div_s), rem = r - q * (unsigned)(jb.h_fast ? a.H : a.L);
+    return jb.h_fast ? RowAt{(long long)q, (long long)rem} : RowAt{(long long)rem, (long long)q};
+}
+struct RowsShared { uint32_t hi[ROWS_MAX_THREADS], lo[ROWS_MAX_THREADS]; float4 par[ROWS_MAX_THREADS]; };     // per group of the CTA
 template <typename T, int SB, bool SYM, bool NORM>
-__device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& jb, unsigned block, uint32_t* s_stats) {
+__device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& jb, unsigned block, RowsShared& sh) {
     constexpr int NV = ROWS_NV;
-    const int tid = threadIdx.x, tpr = a.D >> 3, lpg = jb.group >> 3, gpr = a.D / jb.group;
-    const int w = tid & (tpr - 1), bl = (tid / tpr) & (jb.bp - 1), g_local = tid / (tpr * jb.bp);
+    const int tid = threadIdx.x, tpr = a.D >> 3, lpg = jb.group >> 3, bsh = __ffs(tpr) - 1, psh = __ffs(jb.bp) - 1;
+    const int w = tid & (tpr - 1), bl = (tid >> bsh) & (jb.bp - 1), g_local = tid >> (bsh + psh);
+    const int gsh = bsh - (__ffs(lpg) - 1), n_groups = jb.ngr << gsh;      // groups per row (log2), of the CTA
     const unsigned n_gr = (unsigned)a.L * (unsigned)a.H, gr_ = block * (unsigned)jb.ngr + g_local;
     const bool in = gr_ < n_gr;
-    const unsigned gr = in ? gr_ : n_gr - 1;              // threads past the last group repeat it and store nothing
-    const unsigned n_in = jb.h_fast ? a.H : a.L, r_out = gr / n_in, r_in = gr - r_out * n_in;
-    const int h = jb.h_fast ? r_in : r_out, l = jb.h_fast ? r_out : r_in;
-    const T* xp = reinterpret_cast<const T*>(jb.x) + (long long)l * jb.xs_l + (long long)h * jb.xs_h + w * 8;
+    // threads past the last group repeat it and store nothing
+    const RowAt at = row_at(a, jb, in ? gr_ : n_gr - 1);
+    const T* xp = reinterpret_cast<const T*>(jb.x) + at.l * jb.xs_l + at.h * jb.xs_h + w * 8;
     Vec8<T> x[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k)
         if (k < jb.nv) x[k].load(xp + (long long)min(bl + k * jb.bp, a.B - 1) * jb.xs_b);      // past the batch: the last sample again
     const bool across_warps = tpr * jb.bp > 32;
     if (across_warps) {
-        for (int i = tid; i < jb.ngr * gpr * 2; i += blockDim.x) s_stats[i] = 0u;
+        if (tid < n_groups) { sh.hi[tid] = 0u; sh.lo[tid] = 0u; }
         __syncthreads();
     }
     typename PickAcc<T, SYM, NORM>::type acc;
@@ -234,11 +277,8 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
             }
         }
     }
-    float h8[8], l8[8];
-    acc.get(h8, l8);
-    float hi = h8[0], lo = l8[0];
-#pragma unroll
-    for (int j = 1; j < 8; ++j) { hi = fmaxf(hi, h8[j]); lo = fminf(lo, l8[j]); }
+    float hi, lo;
+    acc.fold(hi, lo);
     for (int m = 1; m < lpg; m <<= 1) {
         hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, m));
         if (!SYM) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, m));
@@ -247,38 +287,46 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
         hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, m));
         if (!SYM) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, m));
     }
-    Range rg;
-    rg.hi = f2ord(hi);
-    rg.lo = SYM ? 0u : ~f2ord(lo);
-    if (across_warps) {
-        const int slot = (g_local * gpr + (w * 8) / jb.group) * 2;
-        if ((w & (lpg - 1)) == 0 && (tid & 31) < tpr) {
-            atomicMax(&s_stats[slot], rg.hi);
-            if (!SYM) atomicMax(&s_stats[slot + 1], rg.lo);
+    const int g = (g_local << gsh) + (w >> (bsh - gsh));             // this thread's group inside the CTA
+    if ((w & (lpg - 1)) == 0 && (across_warps ? (tid & 31) < tpr : bl == 0)) {
+        if (across_warps) {
+            atomicMax(&sh.hi[g], f2ord(hi));
+            if (!SYM) atomicMax(&sh.lo[g], ~f2ord(lo));
+        } else {
+            sh.hi[g] = f2ord(hi);
+            sh.lo[g] = SYM ? 0u : ~f2ord(lo);
         }
-        __syncthreads();
-        rg.hi = s_stats[slot];
-        rg.lo = s_stats[slot + 1];
     }
-    float scale, zp;
-    params_from_range(rg, jb.bits, SYM, jb.eps, scale, zp);
-    const QPar q = make_qpar<SYM>(scale, zp, ord2f(rg.hi), ord2f(~rg.lo));
+    __syncthreads();
+    // the divisions behind scale, zero-point and reciprocal once per group, by the first warps (done by every thread they were
+    // half of the kernel's instructions)
+    if (tid < n_groups) {
+        const Range rg = {sh.hi[tid], sh.lo[tid]};
+        float scale, zp;
+        params_from_range(rg, jb.bits, SYM, jb.eps, scale, zp);
+        const QPar q = make_qpar<SYM>(scale, zp, ord2f(rg.hi), ord2f(~rg.lo));
+        sh.par[tid] = make_float4(q.lo, q.hi, q.magic, scale);
+        const unsigned r = block * (unsigned)jb.ngr + (unsigned)(tid >> gsh);
+        if (r < n_gr) {
+            const RowAt o = row_at(a, jb, r);
+            const long long pi = o.l * jb.ps_r + o.h * jb.ps_h + (long long)(tid & ((1 << gsh) - 1)) * jb.ps_g;
+            jb.scale[pi] = scale;
+            if (!SYM) jb.zp[pi] = zp;
+        }
+    }
+    __syncthreads();
+    const float4 q = sh.par[g];
     const float q_min = -(float)(1 << (jb.bits - 1)), q_max = (float)((1 << (jb.bits - 1)) - 1);
-    int32_t* cp = jb.codes + (long long)l * jb.cs_l + (long long)h * jb.cs_h + (long long)bl * jb.cs_b;
+    int32_t* cp = jb.codes + at.l * jb.cs_l + at.h * jb.cs_h + (long long)bl * jb.cs_b;
     const long long c_step = (long long)jb.bp * jb.cs_b;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         if (k >= jb.nv) break;
         float v[8];
         x[k].get(v);
-        const uint2 c = quantize8<SB, SYM, false>(v, NORM ? __frcp_rn(len[k]) : 1.f, NORM ? len[k] : 0.f, &q.lo, &q.hi, &q.magic, &scale, q_min, q_max);
+        const uint2 c = quantize8<SB, SYM, NORM, false>(v, NORM ? len[k] : 0.f, &q.x, &q.y, &q.z, &q.w, q_min, q_max);
         store8<SB>(cp, w, c, in && bl + k * jb.bp < a.B);
         cp += c_step;
-    }
-    if (in && bl == 0 && (w & (lpg - 1)) == 0) {
-        const long long pi = (long long)l * jb.ps_r + (long long)h * jb.ps_h + (long long)((w * 8) / jb.group) * jb.ps_g;
-        jb.scale[pi] = scale;
-        if (!SYM) jb.zp[pi] = zp;
     }
 }
 
@@ -294,11 +342,11 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 768 / THREADS) append_rows_kernel(const __grid_constant__ AppendArgs a) {
-    __shared__ uint32_t s_stats[THREADS * 2];
+    __shared__ RowsShared sh;
     const int ji = a.n_jobs > 1 && blockIdx.x >= a.job[0].blocks ? 1 : 0;
     const AppendJob& jb = a.job[ji];
     const unsigned block = blockIdx.x - (ji ? a.job[0].blocks : 0u);
-#define VARQ_BODY(T_, SB_, SYM_, NORM_) rows_body<T_, SB_, SYM_, NORM_>(a, jb, block, s_stats)
+#define VARQ_BODY(T_, SB_, SYM_, NORM_) rows_body<T_, SB_, SYM_, NORM_>(a, jb, block, sh)
     VARQ_AP_SWITCH
 #undef VARQ_BODY
 }
@@ -368,8 +416,8 @@ template <bool SYM> struct ColQuant {
         q_min = -(float)(1 << (jb.bits - 1)); q_max = (float)((1 << (jb.bits - 1)) - 1);
         scale = s_par + 3 * D + w * 8;
     }
-    template <int SB> __device__ __forceinline__ uint2 codes(const float (&v)[8], float rlen, float length) const {
-        return quantize8<SB, SYM, true>(v, rlen, length, lo, hi, m, scale, q_min, q_max);
+    template <int SB, bool NORM> __device__ __forceinline__ uint2 codes(const float (&v)[8], float length) const {
+        return quantize8<SB, SYM, NORM, true>(v, length, lo, hi, m, scale, q_min, q_max);
     }
 };
 // (sample, inner index) of a thread's rows first, first + step, ...: one division at the start, then constant steps with a carry
@@ -448,7 +496,7 @@ __device__ __forceinline__ void cluster_body(const AppendArgs& a, const AppendJo
         if ((unsigned)u * step >= R) break;
         float v[8];
         x[u].get(v);
-        const uint2 c = q.template codes<SB>(v, NORM ? __frcp_rn(len[u]) : 1.f, NORM ? len[u] : 0.f);
+        const uint2 c = q.template codes<SB, NORM>(v, len[u]);
         store8<SB>(ch + (long long)k.b * jb.cs_b + (long long)k.l * jb.cs_in, w, c, k.b < (unsigned)a.B);
         k.next();
     }
@@ -550,7 +598,7 @@ __device__ __forceinline__ void plane_apply_body(const AppendArgs& a, const Appe
         for (int u = 0; u < COL_UNROLL; ++u) {
             float v[8];
             x[u].get(v);
-            const uint2 c = q.template codes<SB>(v, NORM ? __frcp_rn(d[u]) : 1.f, NORM ? d[u] : 0.f);
+            const uint2 c = q.template codes<SB, NORM>(v, d[u]);
             store8<SB>(ch + (long long)kc.b * jb.cs_b + (long long)kc.l * jb.cs_in, w, c, rr + u * nrl + rl < r1);
             kc.next();
         }
@@ -624,6 +672,10 @@ int plan_job(AppendJob& jb, const varq_append_job_t& in, int B, int L, int H, in
     jb.nv = (B + bp - 1) / bp;
     jb.ngr = AP_THREADS / (tpr * bp) < 1 ? 1 : AP_THREADS / (tpr * bp);
     jb.h_fast = jb.xs_h <= jb.xs_l;
+    const unsigned n_in = (unsigned)(jb.h_fast ? H : L);
+    jb.div_s = 0;
+    while ((1ull << jb.div_s) < n_in) ++jb.div_s;
+    jb.div_m = (unsigned)(((1ull << 32) * ((1ull << jb.div_s) - n_in)) / n_in + 1);
     jb.blocks = (unsigned)(((long long)L * H + jb.ngr - 1) / jb.ngr);
     return 1;
 }
