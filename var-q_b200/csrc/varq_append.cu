@@ -141,6 +141,11 @@ __device__ __noinline__ float exact_code(float x, float length, float scale, flo
     if (length > 0.f) x = __fdiv_rn(x, length);
     return fminf(fmaxf(__fadd_rn(rintf(__fdiv_rn(x, scale)), zp), q_min), q_max) + Q_MAGIC;
 }
+// Whether a code of an asymmetric group can leave its range before the clamp: codes grow with x, so the ends of the range decide (they
+// only do when rounding takes zero-point and quotient apart).  Symmetric codes cannot: |x| <= amax.
+__device__ __forceinline__ bool needs_clamp(float mx, float mn, float scale, float zp, int bits) {
+    return !(rintf(__fdiv_rn(mx, scale)) + zp <= (float)((1 << (bits - 1)) - 1) && rintf(__fdiv_rn(mn, scale)) + zp >= -(float)(1 << (bits - 1)));
+}
 // y[8] (1.5 * 2^23 + code) -> packed fields: 8 bits two words, 4 bits one, 2 bits half a word.  The bit patterns are 0x4B400000 + code: a
 // chain of shift-adds sums code << (bits * j) and a known constant, which is replaced by the offset that makes all fields
 // non-negative, and the offset's bits are flipped back to two's complement.
@@ -171,7 +176,7 @@ __device__ __forceinline__ float settle(float x, float lo, float hi, float magic
 // PER_VALUE: parameters per value position (columns), else one set
 template <int SB, bool SYM, bool NORM, bool PER_VALUE>
 __device__ __forceinline__ uint2 quantize8(const float (&x)[8], float length, const float* lo, const float* hi, const float* magic, const float* scale,
-                                           float q_min, float q_max) {
+                                           float q_min, float q_max, bool clamp) {
     float y[8];
     bool bad = false;
     const float rlen = NORM ? __frcp_rn(length) : 1.f;
@@ -211,7 +216,7 @@ __device__ __forceinline__ uint2 quantize8(const float (&x)[8], float length, co
             }
         }
     }
-    if (!SYM) {           // a symmetric code cannot leave its range: |x| <= amax
+    if (!SYM && clamp) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) y[j] = fminf(fmaxf(y[j], Q_MAGIC + q_min), Q_MAGIC + q_max);
     }
@@ -305,7 +310,8 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
         float scale, zp;
         params_from_range(rg, jb.bits, SYM, jb.eps, scale, zp);
         const QPar q = make_qpar<SYM>(scale, zp, ord2f(rg.hi), ord2f(~rg.lo));
-        sh.par[tid] = make_float4(q.lo, q.hi, q.magic, scale);
+        // the sign of the scale says that the codes need their clamp
+        sh.par[tid] = make_float4(q.lo, q.hi, q.magic, !SYM && needs_clamp(ord2f(rg.hi), ord2f(~rg.lo), scale, zp, jb.bits) ? -scale : scale);
         const unsigned r = block * (unsigned)jb.ngr + (unsigned)(tid >> gsh);
         if (r < n_gr) {
             const RowAt o = row_at(a, jb, r);
@@ -315,7 +321,9 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
         }
     }
     __syncthreads();
-    const float4 q = sh.par[g];
+    float4 q = sh.par[g];
+    const bool clamp = !SYM && q.w < 0.f;
+    q.w = fabsf(q.w);
     const float q_min = -(float)(1 << (jb.bits - 1)), q_max = (float)((1 << (jb.bits - 1)) - 1);
     int32_t* cp = jb.codes + at.l * jb.cs_l + at.h * jb.cs_h + (long long)bl * jb.cs_b;
     const long long c_step = (long long)jb.bp * jb.cs_b;
@@ -324,7 +332,7 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
         if (k >= jb.nv) break;
         float v[8];
         x[k].get(v);
-        const uint2 c = quantize8<SB, SYM, NORM, false>(v, NORM ? len[k] : 0.f, &q.x, &q.y, &q.z, &q.w, q_min, q_max);
+        const uint2 c = quantize8<SB, SYM, NORM, false>(v, NORM ? len[k] : 0.f, &q.x, &q.y, &q.z, &q.w, q_min, q_max, clamp);
         store8<SB>(cp, w, c, in && bl + k * jb.bp < a.B);
         cp += c_step;
     }
@@ -377,7 +385,7 @@ __device__ __forceinline__ void fold_columns(float (&hi)[8], float (&lo)[8], int
         s_cta[tid] = a; s_cta[D + tid] = b;
     }
 }
-// scale / zero-point and quantizer constants of column `d` from its range; s_par [4][D]: lo, hi, magic, scale
+// scale / zero-point and quantizer constants of column `d` from its range; s_par [5][D]: lo, hi, magic, scale, clamp
 template <bool SYM>
 __device__ __forceinline__ void column_params(const AppendJob& jb, int D, int plane, int d, float mx, float mn, bool write, float* s_par) {
     Range rg;
@@ -386,6 +394,7 @@ __device__ __forceinline__ void column_params(const AppendJob& jb, int D, int pl
     params_from_range(rg, jb.bits, SYM, jb.eps, scale, zp);
     const QPar q = make_qpar<SYM>(scale, zp, mx, mn);
     s_par[d] = q.lo; s_par[D + d] = q.hi; s_par[2 * D + d] = q.magic; s_par[3 * D + d] = scale;
+    if (!SYM) s_par[4 * D + d] = needs_clamp(mx, mn, scale, zp, jb.bits) ? 1.f : 0.f;
     if (write) {
         const long long pi = (long long)plane * jb.ps_out + (long long)d * jb.ps_g;
         jb.scale[pi] = scale;
@@ -409,15 +418,19 @@ __device__ __forceinline__ void fold_plane(int D, float& mx, float& mn, float* s
 }
 template <bool SYM> struct ColQuant {
     float lo[8], hi[8], m[8], q_min, q_max;
+    bool clamp;
     const float* scale;
     __device__ __forceinline__ void init(const AppendJob& jb, int D, int w, const float* s_par) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) { lo[j] = s_par[w * 8 + j]; hi[j] = s_par[D + w * 8 + j]; m[j] = SYM ? Q_MAGIC : s_par[2 * D + w * 8 + j]; }
         q_min = -(float)(1 << (jb.bits - 1)); q_max = (float)((1 << (jb.bits - 1)) - 1);
         scale = s_par + 3 * D + w * 8;
+        clamp = false;
+        if (!SYM)
+            for (int j = 0; j < 8; ++j) clamp = clamp | (scale[D + j] != 0.f);
     }
     template <int SB, bool NORM> __device__ __forceinline__ uint2 codes(const float (&v)[8], float length) const {
-        return quantize8<SB, SYM, NORM, true>(v, length, lo, hi, m, scale, q_min, q_max);
+        return quantize8<SB, SYM, NORM, true>(v, length, lo, hi, m, scale, q_min, q_max, clamp);
     }
 };
 // (sample, inner index) of a thread's rows first, first + step, ...: one division at the start, then constant steps with a carry
@@ -502,7 +515,7 @@ __device__ __forceinline__ void cluster_body(const AppendArgs& a, const AppendJo
     }
 }
 __global__ void __launch_bounds__(AP_THREADS, 2) append_plane_cluster_kernel(const __grid_constant__ AppendArgs a) {
-    __shared__ float s_red[18 * 128], s_par[4 * 128];
+    __shared__ float s_red[18 * 128], s_par[5 * 128];
     const int csize = (int)cg::this_cluster().num_blocks();
     const int cluster = blockIdx.x / csize, ji = cluster / a.n_out, h = cluster - ji * a.n_out;
     const AppendJob& jb = a.job[ji];
@@ -614,7 +627,7 @@ __global__ void __launch_bounds__(AP_THREADS, 3) append_plane_stats_kernel(const
 #undef VARQ_BODY
 }
 __global__ void __launch_bounds__(AP_THREADS, 2) append_plane_apply_kernel(const __grid_constant__ AppendArgs a) {
-    __shared__ float s_red[2 * AP_THREADS], s_par[4 * 128];
+    __shared__ float s_red[2 * AP_THREADS], s_par[5 * 128];
     const unsigned t = blockIdx.x / (unsigned)a.n_out;
     // chunks in reverse order: the ones read last by the statistics kernel are the likeliest to be in L2
     const int h = blockIdx.x - t * a.n_out, ji = a.n_jobs - 1 - (int)(t / a.chunks), chunk = a.chunks - 1 - (int)(t % a.chunks);

@@ -219,10 +219,128 @@ __global__ void __launch_bounds__(256) unpack_dequant_w32_kernel(DequantArgs a, 
     }
 }
 
+// fp32 output of head_dims with a power-of-two number of 16-byte chunks: four values per thread and row, so that every store
+// instruction writes whole lines whatever the code width, and a thread keeps its head_dim slice: per-dim parameters stay in registers
+// until the appended step changes.  What bounds it: HBM writes (with an index computation, a parameter fetch and integer conversions per
+// word the kernel above issued 62 instructions per four values: 3.8 TB/s of int8 [128,1024,30,64]).
+constexpr int DQ_UNROLL = 4;          // rows in flight per thread
+template <int BITS> __device__ __forceinline__ void codes4(uint32_t w, int sub, float (&v)[4]) {      // fields 4 sub .. 4 sub + 3 of a word
+    // a byte u in the low byte of 0x4B000000 is the float 2^23 + u; codes are offset to unsigned first
+    constexpr float BIAS = 8388608.f + (float)(1 << (BITS - 1));
+    uint32_t b[4];
+    if constexpr (BITS == 8) {
+        const uint32_t x = w ^ 0x80808080u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = __byte_perm(x, 0x4B000000u, 0x7540 + j);
+    } else if constexpr (BITS == 4) {
+        const uint32_t x = (w ^ 0x88888888u) >> (16 * sub), lo = x & 0x0F0Fu, hi = (x >> 4) & 0x0F0Fu;
+        b[0] = __byte_perm(lo, 0x4B000000u, 0x7540); b[1] = __byte_perm(hi, 0x4B000000u, 0x7540);
+        b[2] = __byte_perm(lo, 0x4B000000u, 0x7541); b[3] = __byte_perm(hi, 0x4B000000u, 0x7541);
+    } else {
+        const uint32_t x = (w ^ 0xAAAAAAAAu) >> (8 * sub);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = ((x >> (2 * j)) & 3u) | 0x4B000000u;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(b[j]) - BIAS;
+}
+// PER_VALUE: one parameter pair per value (groups smaller than four), else one per thread and row
+template <int BITS, bool ZP, bool PER_VALUE>
+__global__ void __launch_bounds__(256) dequant_rows_kernel(DequantArgs a, int chunk, int chunks, int tsh) {
+    constexpr int NP = PER_VALUE ? 4 : 1;
+    const int tpr = 1 << tsh, q = threadIdx.x & (tpr - 1), rl = threadIdx.x >> tsh, step = 256 >> tsh;
+    const unsigned bh = blockIdx.x / (unsigned)chunks;
+    const int c = (int)(blockIdx.x - bh * (unsigned)chunks), b = (int)(bh / (unsigned)a.H), h = (int)(bh - (unsigned)b * (unsigned)a.H);
+    const int l1 = min(a.L, (c + 1) * chunk);
+    const int d0 = q * 4;
+    const int32_t* cp = a.codes + b * a.cs_b + h * a.cs_h + d0 / (32 / BITS);
+    float* op = reinterpret_cast<float*>(a.out) + b * a.os_b + h * a.os_h + d0;
+    const int sub = (d0 / 4) & (8 / BITS - 1);
+    const long long pbase = a.p.index(b, 0, h, d0);
+    float s[NP], z[NP];
+    int row = -1;
+    for (int l = c * chunk + rl; l < l1; l += DQ_UNROLL * step) {
+        uint32_t w[DQ_UNROLL];
+        int r[DQ_UNROLL];
+        float su[DQ_UNROLL], zu[DQ_UNROLL];
+#pragma unroll
+        for (int u = 0; u < DQ_UNROLL; ++u) {
+            const int t = min(l + u * step, l1 - 1);          // past the chunk: the last row again, not stored
+            w[u] = (uint32_t)__ldg(cp + (long long)t * a.cs_l);
+            r[u] = a.p.row(t);
+            if (!PER_VALUE) {
+                const long long pi = pbase + r[u] * a.p.sr;
+                su[u] = __ldg(a.p.scale + pi);
+                zu[u] = ZP ? __ldg(a.p.zp + pi) : 0.f;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < DQ_UNROLL; ++u) {
+            const int t = l + u * step;
+            if (PER_VALUE) {
+                if (r[u] != row) {
+                    row = r[u];
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) {
+                        const long long pi = pbase + row * a.p.sr + (long long)((d0 + j) / a.p.group - d0 / a.p.group) * a.p.sg;
+                        s[j] = __ldg(a.p.scale + pi);
+                        z[j] = ZP ? __ldg(a.p.zp + pi) : 0.f;
+                    }
+                }
+            } else {
+                s[0] = su[u]; z[0] = zu[u];
+            }
+            float v[4];
+            codes4<BITS>(w[u], sub, v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (ZP) v[j] = __fsub_rn(v[j], z[PER_VALUE ? j : 0]);
+                v[j] = __fmul_rn(v[j], s[PER_VALUE ? j : 0]);
+            }
+            if (t < l1) *reinterpret_cast<float4*>(op + (long long)t * a.os_l) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+    }
+}
+// true if it took the call
+template <int BITS>
+static bool launch_dequant_rows(const DequantArgs& a, cudaStream_t st) {
+    const int tpr = a.D / 4;
+    if (a.D % 32 || (tpr & (tpr - 1)) || tpr > 256) return false;
+    if ((reinterpret_cast<uintptr_t>(a.out) & 15) || ((a.os_b | a.os_l | a.os_h) & 3)) return false;
+    const long long bh = (long long)a.B * a.H;
+    const int rows = 256 / tpr;                       // of a CTA and pass
+    // tokens of a CTA: enough CTAs for the chip, at least a full unrolled pass each
+    long long chunks = ((long long)sm_count() * 16 + bh - 1) / bh;
+    const long long most = (a.L + rows * DQ_UNROLL - 1) / (rows * DQ_UNROLL);
+    if (chunks > most) chunks = most;
+    if (chunks < 1) chunks = 1;
+    const int chunk = (int)((a.L + chunks - 1) / chunks);
+    if (bh * chunks > 0x7fffffffLL) return false;
+    int tsh = 0;
+    while ((1 << tsh) < tpr) ++tsh;
+    const unsigned grid = (unsigned)(bh * chunks);
+    const bool per_value = a.p.group % 4 != 0;
+    if (a.p.zp) {
+        if (per_value) dequant_rows_kernel<BITS, true, true><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
+        else dequant_rows_kernel<BITS, true, false><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
+    } else {
+        if (per_value) dequant_rows_kernel<BITS, false, true><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
+        else dequant_rows_kernel<BITS, false, false><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
+    }
+    return true;
+}
+
 template <typename T, int BITS>
 static int launch_dequant(const DequantArgs& a, bool vec, cudaStream_t st) {
     const long long total = (long long)a.B * a.L * a.H * a.words;
     if (total == 0) return VARQ_OK;
+    if constexpr (sizeof(T) == 4) {
+        if (launch_dequant_rows<BITS>(a, st)) {
+            VARQ_CUDA_TRY(cudaGetLastError());
+            count_launches(1);
+            return VARQ_OK;
+        }
+    }
     const int threads = 256;
     constexpr int VPW = 32 / BITS;
     if (vec && a.D == a.words * VPW && total < (1ll << 31)) {
