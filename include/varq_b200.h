@@ -213,8 +213,8 @@ int varq_unpack_dequant(const varq_tensor_t* codes, int32_t B, int32_t L, int32_
                         const varq_tensor_t* out, void* stream);
 
 /* Pin the kernel varq_attn_fwd uses for every later call of the process: automatic choice, the general
- * CUDA-core kernel, the streaming CUDA-core kernel, the tcgen05 tensor-core kernel or the warp-level tensor-core
- * kernel of the early scales (MID).  A pinned kernel that cannot take a call (shape, layout, grouping) yields to the
+ * CUDA-core kernel, the streaming CUDA-core kernel, the tcgen05 tensor-core kernel, the warp-level tensor-core
+ * kernel of the early scales (MID) or that of a few queries over a long cache (DECODE).  A pinned kernel that cannot take a call (shape, layout, grouping) yields to the
  * next one in the automatic order and finally to the general kernel.  For tests and measurements that compare the kernels on
  * one input; no counterpart in the reference. */
 #define VARQ_ATTN_PATH_AUTO   0
@@ -222,6 +222,7 @@ int varq_unpack_dequant(const varq_tensor_t* codes, int32_t B, int32_t L, int32_
 #define VARQ_ATTN_PATH_STREAM 2
 #define VARQ_ATTN_PATH_TC     3
 #define VARQ_ATTN_PATH_MID    4
+#define VARQ_ATTN_PATH_DECODE 5
 int varq_attn_force_path(int32_t path);
 
 /* Bytes of scratch varq_attn_fwd needs for this shape, whichever kernel it picks: partial results of the

@@ -98,6 +98,9 @@ bool attn_tc_eligible(const AttnArgs& a, int kb, int vb);
 int attn_tc_run(const AttnArgs& a, int kb, int vb, void* ws, size_t ws_bytes, cudaStream_t st);
 size_t attn_tc_workspace_bytes(int B, int H, int Lq, int Lk, int D);
 int attn_tc_status(int* out);
+bool attn_decode_eligible(const AttnArgs& a, int kb, int vb);
+size_t attn_decode_workspace_bytes(int B, int H, int Lq, int Lk, int D);
+int attn_decode_run(AttnArgs& a, int kb, int vb, void* ws, size_t ws_bytes, cudaStream_t st);
 bool attn_mid_eligible(const AttnArgs& a, int kb, int vb);
 int attn_mid_run(AttnArgs& a, int kb, int vb, cudaStream_t st);
 

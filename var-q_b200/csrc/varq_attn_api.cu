@@ -18,8 +18,9 @@ extern "C" size_t varq_attn_workspace_bytes(int32_t B, int32_t H, int32_t Lq, in
     if (B <= 0 || H <= 0 || Lq <= 0 || Lk <= 0 || D <= 0) return 0;
     const size_t s1 = attn_small_workspace_bytes(B, H, Lq, Lk, D), s2 = attn_stream_workspace_bytes(B, H, Lq, Lk, D);
     const size_t s3 = attn_tc_workspace_bytes(B, H, Lq, Lk, D);
-    const size_t s12 = s1 > s2 ? s1 : s2;
-    return s12 > s3 ? s12 : s3;
+    const size_t s4 = D == 64 || D == 128 ? attn_decode_workspace_bytes(B, H, Lq, Lk, D) : 0;
+    const size_t s12 = s1 > s2 ? s1 : s2, s34 = s3 > s4 ? s3 : s4;
+    return s12 > s34 ? s12 : s34;
 }
 
 static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
@@ -67,6 +68,9 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     // of a schedule, whose caches are a few hundred tokens at most.  Everything else goes to the tensor cores, where a
     // 128-row tile with few live rows still finishes a long cache sooner.
     const int force = __atomic_load_n(&g_forced_path, __ATOMIC_RELAXED);
+    // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key.
+    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : (Lq <= 8 && Lk > 256);
+    if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool small_q = Lq <= 4 || (Lq <= 16 && Lk <= 256);
     // Between the two: tens of queries over at most a few hundred tokens (the early scales of a schedule), where the tcgen05
     // kernel is bound by its per-CTA set-up; a warp-level tensor-core kernel takes them when the parameters are per key.
@@ -95,7 +99,7 @@ extern "C" int varq_attn_fwd_qnorm(const varq_tensor_t* q, const varq_tensor_t* 
 }
 
 extern "C" int varq_attn_force_path(int32_t path) {
-    if (path < VARQ_ATTN_PATH_AUTO || path > VARQ_ATTN_PATH_MID) return fail(VARQ_ERR_ARG, "varq_attn_force_path: unknown path %d", path);
+    if (path < VARQ_ATTN_PATH_AUTO || path > VARQ_ATTN_PATH_DECODE) return fail(VARQ_ERR_ARG, "varq_attn_force_path: unknown path %d", path);
     __atomic_store_n(&g_forced_path, (int)path, __ATOMIC_RELAXED);
     return VARQ_OK;
 }

