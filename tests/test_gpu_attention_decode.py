@@ -22,7 +22,7 @@ def _auto_path_afterwards():
 @pytest.mark.parametrize("kb,vb", [(8, 8), (4, 4), (2, 2), (4, 2), (2, 8), (8, 4)])
 @pytest.mark.parametrize("lq,lk,mode,symmetric,q_dtype", [
     (1, 1, "G_TOKEN_HEAD", True, torch.float32), (4, 15, "G_TOKEN_HEAD", False, torch.float32), (3, 300, "G_TOKEN", False, torch.bfloat16),
-    (5, 1000, "G_TOKEN_HEAD", False, torch.float32), (8, 2049, "G_SCALE", True, torch.float16), (9, 529, "G_TOKEN_HEAD", True, torch.float32)])
+    (5, 1000, "G_TOKEN_HEAD", False, torch.float32), (8, 2049, "G_TOKEN", True, torch.float16), (9, 529, "G_TOKEN_HEAD", True, torch.float32)])
 def test_against_the_oracle(D, kb, vb, lq, lk, mode, symmetric, q_dtype):
     fmt, B, H = "BHLc", 2, 3
     kq, vq = (VAR_Q(b, fmt, mode, symmetric=symmetric) for b in (kb, vb))

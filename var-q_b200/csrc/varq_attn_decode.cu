@@ -15,8 +15,9 @@
 // log-sum-exp rule, partial results of a split in the layout of the small-query kernel.
 // Measured (B64 H16 c128, one bf16 query over 10 521 tokens, int4): 0.95 ms on the CUDA cores (254 instructions per four keys), see the
 // figures at the dispatch rule for this kernel.  Bound by instruction issue at 2 and 4 bits, HBM at 8.
-// Applies to one scale / zero-point per key (per token, per token and head, per appended step) at head_dim 64 and 128.
+// Applies to one scale / zero-point per key (per token, per token and head) at head_dim 64 and 128.
 #include <cfloat>
+#include <type_traits>
 
 #include "varq_attn.cuh"
 #include "varq_codes.cuh"
@@ -48,7 +49,13 @@ __device__ __forceinline__ float dc_ex2(float x) {
 }
 __device__ __forceinline__ float dc_lg2(float x) {
     float y;
-    asm("lg2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float dc_rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -69,16 +76,15 @@ template <int BYTES> struct Raw {
         }
     }
 };
-// 8 pairs of raw halves -> signed codes
+// 8 pairs of raw halves -> signed codes: fp16 pairs of -(1024 / 2^p + bias) by bit position, as bit patterns (a conversion function would
+// not be folded at compile time)
+template <int BITS> __host__ __device__ constexpr uint32_t neg_base_h2(int cls) {
+    return BITS == 8 ? 0xE480E480u : BITS == 4 ? (cls == 0 ? 0xE408E408u : 0xD480D480u)
+                                               : (cls == 0 ? 0xE402E402u : cls == 1 ? 0xDC08DC08u : cls == 2 ? 0xD420D420u : 0xCC80CC80u);
+}
 template <int BITS> __device__ __forceinline__ void to_codes(uint32_t (&h)[8]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        constexpr float b0 = Item<BITS>::neg_base(0), b1 = Item<BITS>::neg_base(1 % Item<BITS>::CLS), b2 = Item<BITS>::neg_base(2 % Item<BITS>::CLS),
-                        b3 = Item<BITS>::neg_base(3 % Item<BITS>::CLS);
-        const int cls = i % Item<BITS>::CLS;
-        const __half2 nz = __float2half2_rn(cls == 0 ? b0 : cls == 1 ? b1 : cls == 2 ? b2 : b3);       // folded at compile time
-        h[i] = Item<BITS>::minus_zp(h[i], i, *reinterpret_cast<const uint32_t*>(&nz));
-    }
+    for (int i = 0; i < 8; ++i) h[i] = Item<BITS>::minus_zp(h[i], i, neg_base_h2<BITS>(i % Item<BITS>::CLS));
 }
 // the words of two keys -> words whose halves (bytes at 8 bits) alternate between the keys, so that unpacking them yields pairs
 // (first key, second key) of one head_dim element each, in element order
@@ -90,9 +96,10 @@ template <int BITS, int NW> __device__ __forceinline__ void join_keys(const uint
     }
 }
 
-template <int KB, int VB, int D, int NT>
+template <int KB, int VB, int D, int NT, bool ZP>
 __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB == 8 || VB == 8 || NT > 1) ? 3 : 4) attn_decode_kernel(AttnArgs a, int keys_per_split, int q_tiles4) {
     constexpr int KBYTES = D / 4 * KB / 8, VBYTES = D / 8 * VB / 8;       // of a row and thread
+    constexpr unsigned KROW = D * KB / 8, VROW = D * VB / 8;             // bytes between tokens
     constexpr int KITEMS = D / 64, VITEMS = D / 64;                       // 16-code items of K per row, 8-pair items of V per key pair
     constexpr int KSTEPS = D / 16, MT = D / 16;                          // contraction steps of S, row tiles of O
     __shared__ float s_part[DC_WARPS][DC_QT * NT][D + 2];
@@ -153,9 +160,16 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
     }
     const unsigned char* kbase = reinterpret_cast<const unsigned char*>(a.kc + b * a.ks_b + h * a.ks_h) + c * KBYTES;
     const unsigned char* vbase = reinterpret_cast<const unsigned char*>(a.vc + b * a.vs_b + h * a.vs_h) + g * VBYTES;
-    const long long kpitch = a.ks_l * 4, vpitch = a.vs_l * 4;
+    CodeMagic<KB> kmagic;
+    CodeMagic<VB> vmagic;
+    kmagic.init();
+    vmagic.init();
+    // per-token parameters of key g; a tensor without zero-points reads its scales in their place and drops them
     const long long kpar = a.kp.index(b, 0, h, 0), vpar = a.vp.index(b, 0, h, 0);
-    const bool kz_on = a.kp.zp != nullptr, vz_on = a.vp.zp != nullptr;
+    const float *ksc = a.kp.scale + kpar, *vsc = a.vp.scale + vpar;
+    const float *kzp = a.kp.zp ? a.kp.zp + kpar : ksc, *vzp = a.vp.zp ? a.vp.zp + vpar : vsc;
+    const float kz_on = a.kp.zp ? 1.f : 0.f, vz_on = a.vp.zp ? 1.f : 0.f;
+    const int ksr = (int)a.kp.sr, vsr = (int)a.vp.sr;
 
     const int k_begin = split * keys_per_split, k_end = min(a.Lk, k_begin + keys_per_split);
     struct Tile {
@@ -163,28 +177,36 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
         Raw<VBYTES> v[4];                  // keys 2c, 2c + 1, 2c + 8, 2c + 9
         float ks[2], kz[2], vs[2], vz[2];  // of keys g, g + 8
     };
-    auto fetch = [&](Tile& t, int k0) {
-        const int last = k_end - 1;
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int key = min(k0 + g + 8 * r, last);
-            t.k[r].load(kbase + key * kpitch);
-            const long long pk = kpar + a.kp.row(key) * a.kp.sr, pv = vpar + a.vp.row(key) * a.vp.sr;
-            t.ks[r] = __ldg(a.kp.scale + pk);
-            t.vs[r] = fmaxf(__ldg(a.vp.scale + pv), 1e-30f);
-            t.kz[r] = kz_on ? __ldg(a.kp.zp + pk) : 0.f;
-            t.vz[r] = vz_on ? __ldg(a.vp.zp + pv) : 0.f;
+    const int last = k_end - 1;
+    // parameters of the two keys; a full tile needs no clamping, and its packed rows lie at constant offsets from one address
+    auto fetch_par = [&](Tile& t, int key0, int key1) {
+        const int k0_ = key0 * ksr, v0_ = key0 * vsr, k1_ = key1 * ksr, v1_ = key1 * vsr;
+        t.ks[0] = __ldg(ksc + k0_); t.ks[1] = __ldg(ksc + k1_);
+        t.vs[0] = __ldg(vsc + v0_); t.vs[1] = __ldg(vsc + v1_);
+        if (ZP) {
+            t.kz[0] = __ldg(kzp + k0_) * kz_on; t.kz[1] = __ldg(kzp + k1_) * kz_on;
+            t.vz[0] = __ldg(vzp + v0_) * vz_on; t.vz[1] = __ldg(vzp + v1_) * vz_on;
         }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) t.v[r].load(vbase + min(k0 + 2 * c + (r & 1) + 8 * (r >> 1), last) * vpitch);
     };
-    Tile cur;
-    int k0 = k_begin + warp * 16;
-    if (k0 < k_end) fetch(cur, k0);
-#pragma unroll 1
-    for (; k0 < k_end; k0 += DC_WARPS * 16) {
-        Tile nxt;
-        if (k0 + DC_WARPS * 16 < k_end) fetch(nxt, k0 + DC_WARPS * 16);
+    auto fetch = [&](Tile& t, int k0) {
+        const unsigned char *kp = kbase + (unsigned)(k0 + g) * KROW, *vp = vbase + (unsigned)(k0 + 2 * c) * VROW;
+        t.k[0].load(kp);
+        t.k[1].load(kp + 8 * KROW);
+        t.v[0].load(vp);
+        t.v[1].load(vp + VROW);
+        t.v[2].load(vp + 8 * VROW);
+        t.v[3].load(vp + 9 * VROW);
+        fetch_par(t, k0 + g, k0 + g + 8);
+    };
+    auto fetch_tail = [&](Tile& t, int k0) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) t.k[r].load(kbase + (unsigned)min(k0 + g + 8 * r, last) * KROW);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) t.v[r].load(vbase + (unsigned)min(k0 + 2 * c + (r & 1) + 8 * (r >> 1), last) * VROW);
+        fetch_par(t, min(k0 + g, last), min(k0 + g + 8, last));
+    };
+    auto process = [&](const Tile& cur, int k0, auto tail) {
+        constexpr bool TAIL = decltype(tail)::value;
         // ---- S^T: 16 keys x 8 columns per tile
         float s[NT][4];
         {
@@ -199,11 +221,11 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
                 uint32_t w[Item<KB>::NW];
 #pragma unroll
                 for (int i = 0; i < Item<KB>::NW; ++i) w[i] = cur.k[0].w[it * Item<KB>::NW + i];
-                Item<KB>::raw(w, ka);
+                Item<KB>::raw(w, ka, kmagic);
                 to_codes<KB>(ka);
 #pragma unroll
                 for (int i = 0; i < Item<KB>::NW; ++i) w[i] = cur.k[1].w[it * Item<KB>::NW + i];
-                Item<KB>::raw(w, kb);
+                Item<KB>::raw(w, kb, kmagic);
                 to_codes<KB>(kb);
 #pragma unroll
                 for (int s4 = 0; s4 < 4; ++s4) {
@@ -224,7 +246,7 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
         uint32_t pf[NT][2];
         float lv[2], rv[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) { lv[r] = dc_lg2(cur.vs[r]); rv[r] = __frcp_rn(cur.vs[r]); }
+        for (int r = 0; r < 2; ++r) { const float vs = fmaxf(cur.vs[r], 1e-30f); lv[r] = dc_lg2(vs); rv[r] = dc_rcp(vs); }
         bool over = false;
 #pragma unroll
         for (int t = 0; t < NT; ++t)
@@ -232,8 +254,8 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
             for (int r = 0; r < 2; ++r)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const float x = fmaf(cur.ks[r], fmaf(s[t][2 * r + e], qfac[t][e], -cur.kz[r] * qsum[t][e]), lv[r]);
-                    s[t][2 * r + e] = k0 + g + 8 * r < k_end ? x : -1e30f;
+                    const float x = fmaf(cur.ks[r], ZP ? fmaf(s[t][2 * r + e], qfac[t][e], -cur.kz[r] * qsum[t][e]) : s[t][2 * r + e] * qfac[t][e], lv[r]);
+                    s[t][2 * r + e] = !TAIL || k0 + g + 8 * r < k_end ? x : -1e30f;
                     over = over | (s[t][2 * r + e] > m[t][e] + DC_LAZY);
                 }
         if (__any_sync(0xffffffffu, over)) {
@@ -258,7 +280,7 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
             for (int r = 0; r < 2; ++r) {
                 const float p0 = dc_ex2(s[t][2 * r] - m[t][0]), p1 = dc_ex2(s[t][2 * r + 1] - m[t][1]);      // softmax weight x V scale
                 l[t][0] = fmaf(p0, rv[r], l[t][0]); l[t][1] = fmaf(p1, rv[r], l[t][1]);
-                corr[t][0] = fmaf(p0, cur.vz[r], corr[t][0]); corr[t][1] = fmaf(p1, cur.vz[r], corr[t][1]);
+                if (ZP) { corr[t][0] = fmaf(p0, cur.vz[r], corr[t][0]); corr[t][1] = fmaf(p1, cur.vz[r], corr[t][1]); }
                 const __half2 hh = __floats2half2_rn(p0, p1);
                 const float2 hf = __half22float2(hh);
                 const __half2 hl = __floats2half2_rn(p0 - hf.x, p1 - hf.y);
@@ -274,11 +296,11 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
             uint32_t w[Item<VB>::NW];
 #pragma unroll
             for (int i = 0; i < Item<VB>::NW; ++i) w[i] = ja[it * Item<VB>::NW + i];
-            Item<VB>::raw(w, va);
+            Item<VB>::raw(w, va, vmagic);
             to_codes<VB>(va);
 #pragma unroll
             for (int i = 0; i < Item<VB>::NW; ++i) w[i] = jb[it * Item<VB>::NW + i];
-            Item<VB>::raw(w, vb_);
+            Item<VB>::raw(w, vb_, vmagic);
             to_codes<VB>(vb_);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -287,7 +309,26 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
                 for (int t = 0; t < NT; ++t) mma16816(o[t][it * 4 + i], af, pf[t][0], pf[t][1]);
             }
         }
-        cur = nxt;
+    };
+    // full tiles in two buffers that take turns, the next one's loads in flight; then the ragged end
+    constexpr int STEP = DC_WARPS * 16;
+    const int full_end = k_begin + ((k_end - k_begin) & ~15);
+    Tile ta, tb;
+    int k0 = k_begin + warp * 16;
+    if (k0 < full_end) fetch(ta, k0);
+#pragma unroll 1
+    while (k0 < full_end) {
+        if (k0 + STEP < full_end) fetch(tb, k0 + STEP);
+        process(ta, k0, std::false_type());
+        k0 += STEP;
+        if (k0 >= full_end) break;
+        if (k0 + STEP < full_end) fetch(ta, k0 + STEP);
+        process(tb, k0, std::false_type());
+        k0 += STEP;
+    }
+    if (k0 < k_end) {
+        fetch_tail(ta, k0);
+        process(ta, k0, std::true_type());
     }
     // ---- a warp's partial result: hi + lo columns, sums over the keys of the lanes
 #pragma unroll
@@ -341,14 +382,19 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
     }
 }
 
-// Key ranges: about eight resident waves of CTAs, so that the last, partial one costs little, of at least 256 keys each
+// Key ranges per (sample, head): the count that makes the whole waves of CTAs (four per SM) shortest, a CTA costing its keys plus about 250
+// keys' worth of set-up and merging.
 int decode_splits(int B, int H, int Lq, int Lk, int& keys_per_split) {
     const int unit = DC_WARPS * 16;
-    const long long base = (long long)B * H * ((Lq + 2 * DC_QT - 1) / (2 * DC_QT));
-    long long s = ((long long)sm_count() * 32 + base - 1) / base;
-    if (s > Lk / 256) s = Lk / 256;
-    if (s < 1) s = 1;
-    keys_per_split = (int)(((Lk + s - 1) / s + unit - 1) / unit) * unit;
+    const long long base = (long long)B * H * ((Lq + 2 * DC_QT - 1) / (2 * DC_QT)), room = (long long)sm_count() * 4;
+    long long best = 0;
+    int splits = 1;
+    for (int s = 1; s <= Lk / 256 || s == 1; ++s) {
+        const long long kps = ((Lk + s - 1) / s + unit - 1) / unit * unit, cost = (base * s + room - 1) / room * (kps + 250);
+        if (best == 0 || cost < best) { best = cost; splits = s; }
+        if (base * s > 16 * room) break;
+    }
+    keys_per_split = (int)(((Lk + splits - 1) / splits + unit - 1) / unit) * unit;
     return (Lk + keys_per_split - 1) / keys_per_split;
 }
 
@@ -358,7 +404,8 @@ int launch_decode(AttnArgs& a, int keys_per_split, cudaStream_t st) {
     a.n_qtiles = (a.Lq + DC_QT * NT - 1) / (DC_QT * NT);
     const long long blocks = (long long)a.B * a.H * a.n_qtiles * a.splits;
     if (blocks > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 thread blocks");
-    attn_decode_kernel<KB, VB, D, NT><<<(unsigned)blocks, DC_WARPS * 32, 0, st>>>(a, keys_per_split, n4);
+    if (a.kp.zp || a.vp.zp) attn_decode_kernel<KB, VB, D, NT, true><<<(unsigned)blocks, DC_WARPS * 32, 0, st>>>(a, keys_per_split, n4);
+    else attn_decode_kernel<KB, VB, D, NT, false><<<(unsigned)blocks, DC_WARPS * 32, 0, st>>>(a, keys_per_split, n4);
     VARQ_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     if (a.splits > 1) {
@@ -373,7 +420,8 @@ int launch_decode(AttnArgs& a, int keys_per_split, cudaStream_t st) {
 
 bool attn_decode_eligible(const AttnArgs& a, int kb, int vb) {
     (void)kb; (void)vb;
-    return (a.D == 64 || a.D == 128) && a.kp.group == a.D && a.vp.group == a.D && a.k16 && a.v16;
+    return (a.D == 64 || a.D == 128) && a.kp.group == a.D && a.vp.group == a.D && a.k16 && a.v16 && a.ks_l == a.wk && a.vs_l == a.wv &&
+           !a.kp.row_of_token && !a.vp.row_of_token && a.Lk * (a.kp.sr > a.vp.sr ? a.kp.sr : a.vp.sr) < (1ll << 31);
 }
 
 size_t attn_decode_workspace_bytes(int B, int H, int Lq, int Lk, int D) {

@@ -306,7 +306,7 @@ struct StepRegs { uint32_t sh[8], sl[8], nz[8]; int step; };
 // clears them (V: their P is zero, but 0 * NaN is not).
 template <int BITS, int D, int NTHR, int MODE, bool SPLIT>
 __device__ __forceinline__ void convert_tile(unsigned char* tile, const unsigned char* packed, const unsigned char* rec, const unsigned char* steptab, StepRegs& sr,
-                                             const ParamRef* ref, int mode, int n_valid, bool zero, int k0, int ptid, int gsh, int grp_shift, int zp_off) {
+                                             const ParamRef* ref, int mode, int n_valid, bool zero, int k0, int ptid, int gsh, int grp_shift, int zp_off, const CodeMagic<BITS>& cm) {
     constexpr int IPK = D / 16, NW = BITS / 2, NIT = TC_N * IPK / NTHR, KSTEP = NTHR / IPK;
     constexpr int LO = SPLIT ? TC_N * D * 2 : 0;
     static_assert(TC_N * IPK % NTHR == 0 && KSTEP % 8 == 0, "items of a tile over the threads");
@@ -325,7 +325,7 @@ __device__ __forceinline__ void convert_tile(unsigned char* tile, const unsigned
         for (int it = 0; it < NIT; ++it) {
             const int key = key0 + it * KSTEP;
             uint32_t d[8], lo[8];
-            Item<BITS>::raw(w[it], d);
+            Item<BITS>::raw(w[it], d, cm);
             if constexpr (MODE == PM_STEP) {
                 const int step = reinterpret_cast<const uint16_t*>(rec)[key];
                 if (step != sr.step) {
@@ -802,6 +802,8 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         if (is_k) {
             auto loop = [&](auto bits_c) {
                 constexpr int BITS = decltype(bits_c)::value;
+                CodeMagic<BITS> cm;
+                cm.init();
 #pragma unroll 1
                 for (int i = 0; i < T; ++i) {
                     const int ps = i % PST, ks = i % KST;
@@ -809,7 +811,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     if (ok && i >= KST) ok = mbar_wait(&bar_kf[ks], ((i - KST) / KST) & 1, abort_flag, 22);    // K stage is free
                     if (!ok) break;
                     convert_tile<BITS, D, KTHR, KM, !KX>(smem + P::OFF_K + ks * P::KT * P::T_BYTES, smem + dy.pkk + ps * dy.k_stage, smem + dy.krec + ps * dy.krec_stage,
-                                                         steptab, sr, ref, mode, tile_n(i), false, (t0 + i) * N, ptid, gsh, grp_shift, zp_off);
+                                                         steptab, sr, ref, mode, tile_n(i), false, (t0 + i) * N, ptid, gsh, grp_shift, zp_off, cm);
                     fence_async_smem();
                     mbar_arrive(&bar_k[ks]);
                 }
@@ -818,6 +820,8 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         } else {
             auto loop = [&](auto bits_c) {
                 constexpr int BITS = decltype(bits_c)::value;
+                CodeMagic<BITS> cm;
+                cm.init();
 #pragma unroll 1
                 for (int i = 0; i < T; ++i) {
                     const int ps = i % PST, vs = i % VST;
@@ -825,7 +829,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     if (ok && i >= VST) ok = mbar_wait(&bar_o[vs], ((i - VST) / VST) & 1, abort_flag, 24);    // V stage is free
                     if (!ok) break;
                     convert_tile<BITS, D, VTHR, VM, false>(smem + P::OFF_V + vs * P::T_BYTES, smem + dy.pkv + ps * dy.v_stage, smem + dy.vrec + ps * dy.vrec_stage,
-                                                           steptab, sr, ref, mode, tile_n(i), true, (t0 + i) * N, ptid, gsh, grp_shift, zp_off);
+                                                           steptab, sr, ref, mode, tile_n(i), true, (t0 + i) * N, ptid, gsh, grp_shift, zp_off, cm);
                     fence_async_smem();
                     mbar_arrive(&bar_v[vs]);
                 }

@@ -26,6 +26,21 @@ __host__ __device__ constexpr int code_at(int bits, int p) {
     return bits == 8 ? p : bits == 4 ? ((p & 8) | ((p & 1) << 2) | ((p & 7) >> 1)) : (((p & 1) << 3) | (p >> 1));
 }
 __host__ __device__ constexpr int code_bias(int bits) { return bits == 8 ? 128 : bits == 4 ? 8 : 2; }
+// The constants of the pairs as register values that the compiler cannot fold: (x & mask) ^ magic is one three-input logic instruction with
+// the mask as its immediate only if the magic is in a register; with two known constants it became two instructions per pair, and
+// logic instructions run at half rate.
+static __constant__ uint32_t c_code_magic[3][4] = {{0x64026402u, 0x64086408u, 0x64206420u, 0x64806480u}, {0x64086408u, 0x64806480u, 0u, 0u}, {0x64646464u, 0u, 0u, 0u}};
+template <int BITS> struct CodeMagic {
+    static constexpr int N = BITS == 8 ? 1 : BITS == 4 ? 2 : 4;
+    uint32_t m[N];
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            m[i] = c_code_magic[BITS == 2 ? 0 : BITS == 4 ? 1 : 2][i];
+            asm volatile("" : "+r"(m[i]));
+        }
+    }
+};
 template <int BITS> struct Item {           // 16 consecutive codes of one key: 4, 2 or 1 packed words -> 8 pairs
     static constexpr int NW = BITS / 2;
     static constexpr int CLS = BITS == 8 ? 1 : BITS == 4 ? 2 : 4;      // classes of bit position: pair i has class i % CLS
@@ -35,29 +50,29 @@ template <int BITS> struct Item {           // 16 consecutive codes of one key: 
         else w[0] = *p;
     }
     // pairs holding 1024 + 2^p (code + bias)
-    static __device__ __forceinline__ void raw(const uint32_t (&w)[NW], uint32_t (&h)[8]) {
+    static __device__ __forceinline__ void raw(const uint32_t (&w)[NW], uint32_t (&h)[8], const CodeMagic<BITS>& cm) {
         if constexpr (BITS == 8) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const uint32_t u = w[i] ^ 0x80808080u;
-                h[2 * i] = __byte_perm(u, 0x64646464u, 0x4140);
-                h[2 * i + 1] = __byte_perm(u, 0x64646464u, 0x4342);
+                h[2 * i] = __byte_perm(u, cm.m[0], 0x4140);
+                h[2 * i + 1] = __byte_perm(u, cm.m[0], 0x4342);
             }
         } else if constexpr (BITS == 4) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const uint32_t x = w[i], y = w[i] >> 8;
-                h[4 * i] = (x & 0x000F000Fu) ^ 0x64086408u;
-                h[4 * i + 1] = (x & 0x00F000F0u) ^ 0x64806480u;
-                h[4 * i + 2] = (y & 0x000F000Fu) ^ 0x64086408u;
-                h[4 * i + 3] = (y & 0x00F000F0u) ^ 0x64806480u;
+                h[4 * i] = (x & 0x000F000Fu) ^ cm.m[0];
+                h[4 * i + 1] = (x & 0x00F000F0u) ^ cm.m[1];
+                h[4 * i + 2] = (y & 0x000F000Fu) ^ cm.m[0];
+                h[4 * i + 3] = (y & 0x00F000F0u) ^ cm.m[1];
             }
         } else {
             const uint32_t x = w[0], y = w[0] >> 8;
-            h[0] = (x & 0x00030003u) ^ 0x64026402u; h[1] = (x & 0x000C000Cu) ^ 0x64086408u;
-            h[2] = (x & 0x00300030u) ^ 0x64206420u; h[3] = (x & 0x00C000C0u) ^ 0x64806480u;
-            h[4] = (y & 0x00030003u) ^ 0x64026402u; h[5] = (y & 0x000C000Cu) ^ 0x64086408u;
-            h[6] = (y & 0x00300030u) ^ 0x64206420u; h[7] = (y & 0x00C000C0u) ^ 0x64806480u;
+            h[0] = (x & 0x00030003u) ^ cm.m[0]; h[1] = (x & 0x000C000Cu) ^ cm.m[1];
+            h[2] = (x & 0x00300030u) ^ cm.m[2]; h[3] = (x & 0x00C000C0u) ^ cm.m[3];
+            h[4] = (y & 0x00030003u) ^ cm.m[0]; h[5] = (y & 0x000C000Cu) ^ cm.m[1];
+            h[6] = (y & 0x00300030u) ^ cm.m[2]; h[7] = (y & 0x00C000C0u) ^ cm.m[3];
         }
     }
     // -(1024 / 2^p + bias) of a class, before the zero-point
