@@ -59,7 +59,8 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     a.scale_log2 = softmax_scale * 1.4426950408889634f;
     a.splits = 1; a.tiles_per_split = 0; a.n_qtiles = 1; a.ws = reinterpret_cast<float*>(workspace);
     a.q_norm = q_norm ? 1 : 0; a.q_mul = q_mul; a.q_eps = q_eps;
-    if (q_norm) {       // the tensor-core kernel normalises queries as it loads them
+    if (q_norm) {       // the tensor-core kernels normalise queries as they load them
+        if (Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
         if (!attn_tc_eligible(a, kb, vb)) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd_qnorm: no kernel normalises the queries of this shape or layout");
         return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     }
@@ -68,8 +69,10 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     // of a schedule, whose caches are a few hundred tokens at most.  Everything else goes to the tensor cores, where a
     // 128-row tile with few live rows still finishes a long cache sooner.
     const int force = __atomic_load_n(&g_forced_path, __ATOMIC_RELAXED);
-    // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key.
-    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : (Lq <= 8 && Lk > 256);
+    // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key
+    // (B64 H16 c128 int4, 10521 tokens, us: 315 / 515 / 906 for 1 / 8 / 16 queries; tcgen05 1354 whatever the count, streaming 954 / 3721 / 7294;
+    // the lead over tcgen05 ends at 16 queries, on short caches too).
+    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : (Lq <= 16 && Lk > 256);
     if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool small_q = Lq <= 4 || (Lq <= 16 && Lk <= 256);
     // Between the two: tens of queries over at most a few hundred tokens (the early scales of a schedule), where the tcgen05

@@ -118,13 +118,20 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
     for (int t = 0; t < NT; ++t) {
         float v[D / 4];
         const int qi = q0 + t * DC_QT + (g & 3);
-        float mx = 0.f, sum = 0.f;
+        float mx = 0.f, sum = 0.f, ss = 0.f;
 #pragma unroll
         for (int j = 0; j < D / 4; j += 8) {
             float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (qi < a.Lq) load_q8(a.q, a.q_dtype, b * a.qs_b + (long long)qi * a.qs_l + h * a.qs_h + c * (D / 4) + j, e);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { v[j + i] = e[i]; mx = fmaxf(mx, fabsf(e[i])); sum += e[i]; }
+            for (int i = 0; i < 8; ++i) { v[j + i] = e[i]; mx = fmaxf(mx, fabsf(e[i])); sum += e[i]; ss = fmaf(e[i], e[i], ss); }
+        }
+        if (a.q_norm) {                 // x / max(||x||_2, eps) * scale_mul[h], on the way in
+            ss += __shfl_xor_sync(0xffffffffu, ss, 1); ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+            const float f = (a.q_mul ? __ldg(a.q_mul + h) : 1.f) / fmaxf(sqrtf(ss), a.q_eps);
+#pragma unroll
+            for (int j = 0; j < D / 4; ++j) v[j] *= f;
+            mx *= fabsf(f); sum *= f;
         }
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         sum += __shfl_xor_sync(0xffffffffu, sum, 1); sum += __shfl_xor_sync(0xffffffffu, sum, 2);
