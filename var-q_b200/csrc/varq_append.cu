@@ -351,6 +351,8 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 768 / THREADS) append_rows_kernel(const __grid_constant__ AppendArgs a) {
     __shared__ RowsShared sh;
+    pdl_trigger();
+    pdl_wait();
     const int ji = a.n_jobs > 1 && blockIdx.x >= a.job[0].blocks ? 1 : 0;
     const AppendJob& jb = a.job[ji];
     const unsigned block = blockIdx.x - (ji ? a.job[0].blocks : 0u);
@@ -516,6 +518,8 @@ __device__ __forceinline__ void cluster_body(const AppendArgs& a, const AppendJo
 }
 __global__ void __launch_bounds__(AP_THREADS, 2) append_plane_cluster_kernel(const __grid_constant__ AppendArgs a) {
     __shared__ float s_red[18 * 128], s_par[5 * 128];
+    pdl_trigger();
+    pdl_wait();
     const int csize = (int)cg::this_cluster().num_blocks();
     const int cluster = blockIdx.x / csize, ji = cluster / a.n_out, h = cluster - ji * a.n_out;
     const AppendJob& jb = a.job[ji];
@@ -619,6 +623,8 @@ __device__ __forceinline__ void plane_apply_body(const AppendArgs& a, const Appe
 }
 __global__ void __launch_bounds__(AP_THREADS, 3) append_plane_stats_kernel(const __grid_constant__ AppendArgs a) {
     __shared__ float s_red[18 * 128];
+    pdl_trigger();
+    pdl_wait();
     const unsigned t = blockIdx.x / (unsigned)a.n_out;
     const int h = blockIdx.x - t * a.n_out, ji = t / a.chunks, chunk = t - ji * a.chunks;
     const AppendJob& jb = a.job[ji];
@@ -628,6 +634,8 @@ __global__ void __launch_bounds__(AP_THREADS, 3) append_plane_stats_kernel(const
 }
 __global__ void __launch_bounds__(AP_THREADS, 2) append_plane_apply_kernel(const __grid_constant__ AppendArgs a) {
     __shared__ float s_red[2 * AP_THREADS], s_par[5 * 128];
+    pdl_trigger();
+    pdl_wait();
     const unsigned t = blockIdx.x / (unsigned)a.n_out;
     // chunks in reverse order: the ones read last by the statistics kernel are the likeliest to be in L2
     const int h = blockIdx.x - t * a.n_out, ji = a.n_jobs - 1 - (int)(t / a.chunks), chunk = a.chunks - 1 - (int)(t % a.chunks);
@@ -746,18 +754,11 @@ int append_fast(const varq_append_job_t* jobs, int n_jobs, int B, int L, int H, 
         if (kind[i] == 1) {
             const int need = D / 8 * a.job[0].bp;            // (the same for both jobs)
             const unsigned blocks = a.job[0].blocks + (a.n_jobs > 1 ? a.job[1].blocks : 0u);
-            if (need > AP_THREADS) append_rows_kernel<ROWS_MAX_THREADS><<<blocks, ROWS_MAX_THREADS, 0, st>>>(a);
-            else append_rows_kernel<AP_THREADS><<<blocks, AP_THREADS, 0, st>>>(a);
-            VARQ_CUDA_TRY(cudaGetLastError());
+            VARQ_CUDA_TRY(need > AP_THREADS ? launch_pdl(append_rows_kernel<ROWS_MAX_THREADS>, blocks, ROWS_MAX_THREADS, 0, st, 1, a)
+                                            : launch_pdl(append_rows_kernel<AP_THREADS>, blocks, AP_THREADS, 0, st, 1, a));
             count_launches(1);
         } else if (cluster_fits(rows, D, cs)) {
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-            cfg.gridDim = dim3((unsigned)(a.n_out * cs * a.n_jobs)); cfg.blockDim = dim3(AP_THREADS); cfg.stream = st;
-            cfg.attrs = at; cfg.numAttrs = 1;
-            VARQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, append_plane_cluster_kernel, a));
+            VARQ_CUDA_TRY(launch_pdl(append_plane_cluster_kernel, (unsigned)(a.n_out * cs * a.n_jobs), AP_THREADS, 0, st, cs, a));
             count_launches(1);
         } else {
             a.chunks = plane_chunks(a.n_jobs, rows, a.n_out);
@@ -766,9 +767,8 @@ int append_fast(const varq_append_job_t* jobs, int n_jobs, int B, int L, int H, 
             for (int j = 0; j < a.n_jobs; ++j) { a.job[j].ranges = p; p += (size_t)a.n_out * a.chunks * 2 * D; }
             a.job[0].norms = p;
             const unsigned blocks = (unsigned)((long long)a.n_out * a.chunks * a.n_jobs);
-            append_plane_stats_kernel<<<blocks, AP_THREADS, 0, st>>>(a);
-            append_plane_apply_kernel<<<blocks, AP_THREADS, 0, st>>>(a);
-            VARQ_CUDA_TRY(cudaGetLastError());
+            VARQ_CUDA_TRY(launch_pdl(append_plane_stats_kernel, blocks, AP_THREADS, 0, st, 1, a));
+            VARQ_CUDA_TRY(launch_pdl(append_plane_apply_kernel, blocks, AP_THREADS, 0, st, 1, a));
             count_launches(2);
         }
     }

@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(DC_WARPS * 32, NT > 1 && D == 128 ? 2 : (KB ==
     constexpr int KSTEPS = D / 16, MT = D / 16;                          // contraction steps of S, row tiles of O
     __shared__ float s_part[DC_WARPS][DC_QT * NT][D + 2];
 
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
     const unsigned blk = blockIdx.x;                        // query tile fastest, then key range, then (sample, head)
     const int qtile = (int)(blk % (unsigned)a.n_qtiles);
@@ -411,9 +413,8 @@ int launch_decode(AttnArgs& a, int keys_per_split, cudaStream_t st) {
     a.n_qtiles = (a.Lq + DC_QT * NT - 1) / (DC_QT * NT);
     const long long blocks = (long long)a.B * a.H * a.n_qtiles * a.splits;
     if (blocks > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 thread blocks");
-    if (a.kp.zp || a.vp.zp) attn_decode_kernel<KB, VB, D, NT, true><<<(unsigned)blocks, DC_WARPS * 32, 0, st>>>(a, keys_per_split, n4);
-    else attn_decode_kernel<KB, VB, D, NT, false><<<(unsigned)blocks, DC_WARPS * 32, 0, st>>>(a, keys_per_split, n4);
-    VARQ_CUDA_TRY(cudaGetLastError());
+    VARQ_CUDA_TRY(a.kp.zp || a.vp.zp ? launch_pdl(attn_decode_kernel<KB, VB, D, NT, true>, (unsigned)blocks, DC_WARPS * 32, 0, st, 1, a, keys_per_split, n4)
+                                     : launch_pdl(attn_decode_kernel<KB, VB, D, NT, false>, (unsigned)blocks, DC_WARPS * 32, 0, st, 1, a, keys_per_split, n4));
     count_launches(1);
     if (a.splits > 1) {
         attn_small_merge_launch(a, n4, st);

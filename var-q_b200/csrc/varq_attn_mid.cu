@@ -92,6 +92,8 @@ __global__ void __launch_bounds__(WARPS * 32, (QSPLIT ? 12 : 16) / WARPS) attn_m
     __shared__ __align__(16) __half sV[MID_KEYS * PITCH];
     __shared__ float sKs[MID_KEYS], sKz[MID_KEYS], sVs[MID_KEYS], sVr[MID_KEYS], sVz[MID_KEYS];    // sVs = log2 (V scale), sVr = 1 / (V scale)
 
+    pdl_trigger();
+    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int qt = (int)(blockIdx.x % (unsigned)a.n_qtiles), bh = (int)(blockIdx.x / (unsigned)a.n_qtiles), b = bh / a.H, h = bh - b * a.H;
     const int q0 = qt * MID_ROWS + warp * 16;            // first query row of this warp
@@ -332,8 +334,8 @@ static int launch_mid(AttnArgs& a, cudaStream_t st) {
     const long long blocks = (long long)a.B * a.H * nqt;
     if (blocks > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 thread blocks");
     a.n_qtiles = nqt;
-    if (a.q_dtype == VARQ_F32) attn_mid_kernel<KB, VB, true, WARPS><<<(unsigned)blocks, MID_THREADS, 0, st>>>(a);
-    else attn_mid_kernel<KB, VB, false, WARPS><<<(unsigned)blocks, MID_THREADS, 0, st>>>(a);
+    if (a.q_dtype == VARQ_F32) launch_pdl(attn_mid_kernel<KB, VB, true, WARPS>, (unsigned)blocks, MID_THREADS, 0, st, 1, a);
+    else launch_pdl(attn_mid_kernel<KB, VB, false, WARPS>, (unsigned)blocks, MID_THREADS, 0, st, 1, a);
     VARQ_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return VARQ_OK;

@@ -54,6 +54,8 @@ __device__ __forceinline__ void stage_tile(uint32_t* dst, int dst_pitch, const i
 
 template <int KB, int VB>
 __global__ void __launch_bounds__(A1_THREADS) attn_small_kernel(AttnArgs a) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int KV = 32 / KB, VV = 32 / VB;   // codes per K / V word
     constexpr int QT = A1_QT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -298,6 +300,8 @@ __global__ void __launch_bounds__(A1_THREADS) attn_small_kernel(AttnArgs a) {
 
 // merge the per-split partials: one thread per output element
 __global__ void attn_small_merge_kernel(AttnArgs a, int n_qtiles) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int QT = A1_QT;
     const long long total = (long long)a.B * a.H * a.Lq * a.D;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -326,7 +330,7 @@ void attn_small_merge_launch(const AttnArgs& a, int n_qtiles, cudaStream_t st) {
     long long blocks = (total + 255) / 256;
     const long long cap = (long long)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    attn_small_merge_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, n_qtiles);
+    launch_pdl(attn_small_merge_kernel, (unsigned)blocks, 256, 0, st, 1, a, n_qtiles);
 }
 
 static int pick_splits(int B, int H, int Lq, int Lk, int& tiles_per_split) {
@@ -372,7 +376,7 @@ static int launch_small(AttnArgs& a, cudaStream_t st) {
     const long long blocks_1d = (long long)a.B * a.H * nqt * a.splits;
     if (blocks_1d > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 thread blocks");
     a.n_qtiles = nqt;
-    attn_small_kernel<KB, VB><<<(unsigned)blocks_1d, A1_THREADS, smem, st>>>(a);
+    launch_pdl(attn_small_kernel<KB, VB>, (unsigned)blocks_1d, A1_THREADS, smem, st, 1, a);
     VARQ_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     if (a.splits > 1) {
@@ -380,7 +384,7 @@ static int launch_small(AttnArgs& a, cudaStream_t st) {
         long long blocks = (total + 255) / 256;
         const long long cap = (long long)sm_count() * 8;
         if (blocks > cap) blocks = cap;
-        attn_small_merge_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, nqt);
+        launch_pdl(attn_small_merge_kernel, (unsigned)blocks, 256, 0, st, 1, a, nqt);
         VARQ_CUDA_TRY(cudaGetLastError());
         count_launches(1);
     }

@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(WARPS * 32) attn_stream_kernel(AttnArgs a, int
     constexpr int KPS = 32 / LPK;             // keys per warp step
     constexpr int KW = 16 * KB / 32, VW = 16 * VB / 32;   // packed words per lane and step
     __shared__ float s_part[WARPS][QT][D + 2];
+    pdl_trigger();
+    pdl_wait();
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned blk = blockIdx.x;            // query tile fastest (tiles of one key range run together and share it in L2)
@@ -303,13 +305,13 @@ static int launch_stream(AttnArgs& a, int keys_per_split, cudaStream_t st) {
     const unsigned grid = (unsigned)blocks_1d;
     const int qmax = a.Lq < ST_QT ? a.Lq : ST_QT;
     if (a.Lk <= ST_SHORT_KEYS) {
-        if (qmax == 1) attn_stream_kernel<KB, VB, D, 1, 1><<<grid, 32, 0, st>>>(a, keys_per_split);
-        else if (qmax == 2) attn_stream_kernel<KB, VB, D, 2, 1><<<grid, 32, 0, st>>>(a, keys_per_split);
-        else attn_stream_kernel<KB, VB, D, 4, 1><<<grid, 32, 0, st>>>(a, keys_per_split);
+        if (qmax == 1) launch_pdl(attn_stream_kernel<KB, VB, D, 1, 1>, grid, 32, 0, st, 1, a, keys_per_split);
+        else if (qmax == 2) launch_pdl(attn_stream_kernel<KB, VB, D, 2, 1>, grid, 32, 0, st, 1, a, keys_per_split);
+        else launch_pdl(attn_stream_kernel<KB, VB, D, 4, 1>, grid, 32, 0, st, 1, a, keys_per_split);
     } else {
-        if (qmax == 1) attn_stream_kernel<KB, VB, D, 1, ST_WARPS><<<grid, ST_WARPS * 32, 0, st>>>(a, keys_per_split);
-        else if (qmax == 2) attn_stream_kernel<KB, VB, D, 2, ST_WARPS><<<grid, ST_WARPS * 32, 0, st>>>(a, keys_per_split);
-        else attn_stream_kernel<KB, VB, D, 4, ST_WARPS><<<grid, ST_WARPS * 32, 0, st>>>(a, keys_per_split);
+        if (qmax == 1) launch_pdl(attn_stream_kernel<KB, VB, D, 1, ST_WARPS>, grid, ST_WARPS * 32, 0, st, 1, a, keys_per_split);
+        else if (qmax == 2) launch_pdl(attn_stream_kernel<KB, VB, D, 2, ST_WARPS>, grid, ST_WARPS * 32, 0, st, 1, a, keys_per_split);
+        else launch_pdl(attn_stream_kernel<KB, VB, D, 4, ST_WARPS>, grid, ST_WARPS * 32, 0, st, 1, a, keys_per_split);
     }
     VARQ_CUDA_TRY(cudaGetLastError());
     count_launches(1);

@@ -5,6 +5,8 @@ namespace varq {
 
 // Partial rows of a split key range: one warp per (query row), lanes over head_dim.
 __global__ void __launch_bounds__(256) attn_tc_merge_kernel(AttnArgs a, int tile_rows) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long row = blockIdx.x * 8ll + (threadIdx.x >> 5);
     if (row >= (long long)a.B * a.H * a.Lq) return;
@@ -103,8 +105,7 @@ int attn_tc_run(const AttnArgs& a0, int kb, int vb, void* ws, size_t ws_bytes, c
     if (int rc = f.launch(a, dy, kb, vb, st)) return rc;
     if (a.splits > 1) {
         const long long q_rows = (long long)a.B * a.H * a.Lq;
-        attn_tc_merge_kernel<<<(unsigned)((q_rows + 7) / 8), 256, 0, st>>>(a, rows);
-        VARQ_CUDA_TRY(cudaGetLastError());
+        VARQ_CUDA_TRY(launch_pdl(attn_tc_merge_kernel, (unsigned)((q_rows + 7) / 8), 256, 0, st, 1, a, rows));
         count_launches(1);
     }
     return VARQ_OK;

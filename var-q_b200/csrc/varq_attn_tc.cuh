@@ -494,11 +494,13 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)P::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();          // global memory is touched from here on only
     if (tid == P::K_WARP0 * 32) *reinterpret_cast<ParamRef*>(smem + P::OFF_PREF) = param_ref(a.kp, b, h);
     if (tid == P::V_WARP0 * 32) *reinterpret_cast<ParamRef*>(smem + P::OFF_PREF + 48) = param_ref(a.vp, b, h);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();       // behind the allocation: a CTA of a next launch must not take tensor memory that one of this launch still asks for
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp < P::K_WARP0) {
@@ -1080,8 +1082,7 @@ template <int D, int NQ, int QT, int KM, int VM> int tc_launch_one(const AttnArg
         VARQ_CUDA_TRY(cudaFuncSetAttribute(attn_tc_kernel<D, NQ, QT, KM, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    attn_tc_kernel<D, NQ, QT, KM, VM><<<(unsigned)((long long)a.B * a.H * a.n_qtiles * a.splits), P::THREADS, smem, st>>>(a, dy, kb, vb);
-    VARQ_CUDA_TRY(cudaGetLastError());
+    VARQ_CUDA_TRY(launch_pdl(attn_tc_kernel<D, NQ, QT, KM, VM>, (unsigned)((long long)a.B * a.H * a.n_qtiles * a.splits), P::THREADS, smem, st, 1, a, dy, kb, vb));
     count_launches(1);
     return VARQ_OK;
 }

@@ -247,6 +247,8 @@ template <int BITS> __device__ __forceinline__ void codes4(uint32_t w, int sub, 
 // PER_VALUE: one parameter pair per value (groups smaller than four), else one per thread and row
 template <int BITS, bool ZP, bool PER_VALUE>
 __global__ void __launch_bounds__(256) dequant_rows_kernel(DequantArgs a, int chunk, int chunks, int tsh) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int NP = PER_VALUE ? 4 : 1;
     const int tpr = 1 << tsh, q = threadIdx.x & (tpr - 1), rl = threadIdx.x >> tsh, step = 256 >> tsh;
     const unsigned bh = blockIdx.x / (unsigned)chunks;
@@ -322,11 +324,11 @@ static bool launch_dequant_rows(const DequantArgs& a, cudaStream_t st) {
     const unsigned grid = (unsigned)(bh * chunks);
     const bool per_value = a.p.group % 4 != 0;
     if (a.p.zp) {
-        if (per_value) dequant_rows_kernel<BITS, true, true><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
-        else dequant_rows_kernel<BITS, true, false><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
+        if (per_value) launch_pdl(dequant_rows_kernel<BITS, true, true>, grid, 256, 0, st, 1, a, chunk, (int)chunks, tsh);
+        else launch_pdl(dequant_rows_kernel<BITS, true, false>, grid, 256, 0, st, 1, a, chunk, (int)chunks, tsh);
     } else {
-        if (per_value) dequant_rows_kernel<BITS, false, true><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
-        else dequant_rows_kernel<BITS, false, false><<<grid, 256, 0, st>>>(a, chunk, (int)chunks, tsh);
+        if (per_value) launch_pdl(dequant_rows_kernel<BITS, false, true>, grid, 256, 0, st, 1, a, chunk, (int)chunks, tsh);
+        else launch_pdl(dequant_rows_kernel<BITS, false, false>, grid, 256, 0, st, 1, a, chunk, (int)chunks, tsh);
     }
     return true;
 }
