@@ -273,7 +273,7 @@ __device__ __forceinline__ void rows_body(const AppendArgs& a, const AppendJob& 
             if constexpr (NORM) {
                 float v[8];
                 x[k].get(v);
-                len[k] = row_length(v, tpr, jb.norm_eps);
+                len[k] = row_length(x[k], tpr, w, jb.norm_eps);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = __fdiv_rn(v[j], len[k]);
                 acc.add(v);
@@ -480,7 +480,7 @@ __device__ __forceinline__ void cluster_body(const AppendArgs& a, const AppendJo
             if constexpr (NORM) {
                 float v[8];
                 x[u].get(v);
-                len[u] = row_length(v, tpr, jb.norm_eps);
+                len[u] = row_length(x[u], tpr, w, jb.norm_eps);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = __fdiv_rn(v[j], len[u]);
                 if (mine) acc.add(v);
@@ -556,7 +556,7 @@ __device__ __forceinline__ void plane_stats_body(const AppendArgs& a, const Appe
             if constexpr (NORM) {
                 float v[8];
                 x[u].get(v);
-                const float d = row_length(v, tpr, jb.norm_eps);
+                const float d = row_length(x[u], tpr, w, jb.norm_eps);
                 if (w == 0 && r < r1) jb.norms[(size_t)r * a.n_out + h] = d;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = __fdiv_rn(v[j], d);

@@ -58,14 +58,62 @@ template <> struct Vec8<__half> {
         for (int i = 0; i < 4; ++i) { const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i])); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
     }
 };
-// max(||x||_2, eps) of a row held by `tpr` neighbouring lanes (8 or 16), eight values each.  Every kernel that normalises rows for the
-// quantizers takes the sum in this order, so that they produce the same bits and the same codes.
-__device__ __forceinline__ float row_length(const float (&v)[8], int tpr, float eps) {
-    float ss = 0.f;
+// max(||x||_2, eps) of a row of 64 or 128 values held by 8 or 16 neighbouring lanes (lane w of the row: values 8w .. 8w + 7).  The order of
+// the sum is that of qk_norm_stats_kernel, in which warp lane i chains the values i, i + 32, ... and the lanes fold by 16, 8, 4, 2, 1: a length
+// that rounds the other way moves the codes of values on a rounding boundary, and with 16-bit rows 1 in 10^4 packed words has one.  The
+// chains take a transposition first, values travelling in pairs (one register per pair of 16-bit inputs), and every fold but the last
+// ones halves what a lane holds: 9 shuffles for 16-bit rows of 128, against 4 for an arbitrary order.
+template <typename T> struct Pair8 { uint32_t v; };
+template <> struct Pair8<float> { float2 v; };
+__device__ __forceinline__ Pair8<float> pair_xor(const Pair8<float>& p, int m) {
+    Pair8<float> r;
+    r.v.x = __shfl_xor_sync(0xffffffffu, p.v.x, m); r.v.y = __shfl_xor_sync(0xffffffffu, p.v.y, m);
+    return r;
+}
+template <typename T> __device__ __forceinline__ Pair8<T> pair_xor(const Pair8<T>& p, int m) { return {__shfl_xor_sync(0xffffffffu, p.v, m)}; }
+__device__ __forceinline__ float2 pair_values(const Pair8<float>& p) { return p.v; }
+__device__ __forceinline__ float2 pair_values(const Pair8<__nv_bfloat16>& p) { return make_float2(__uint_as_float(p.v << 16), __uint_as_float(p.v & 0xffff0000u)); }
+__device__ __forceinline__ float2 pair_values(const Pair8<__half>& p) { return __half22float2(*reinterpret_cast<const __half2*>(&p.v)); }
+template <typename T> __device__ __forceinline__ void get_pairs(const Vec8<T>& x, Pair8<T> (&p)[4]) {
+    if constexpr (sizeof(T) == 4) { p[0].v = {x.a.x, x.a.y}; p[1].v = {x.a.z, x.a.w}; p[2].v = {x.b.x, x.b.y}; p[3].v = {x.b.z, x.b.w}; }
+    else { p[0].v = x.r.x; p[1].v = x.r.y; p[2].v = x.r.z; p[3].v = x.r.w; }
+}
+template <typename T> __device__ __forceinline__ float row_length(const Vec8<T>& x, int tpr, int w, float eps) {
+    auto fold = [](float s, int m) { return s + __shfl_xor_sync(0xffffffffu, s, m); };
+    auto halve = [](float a, float b, bool keep_b, int m) {      // the kept one, plus the partner's (which keeps the other)
+        return (keep_b ? b : a) + __shfl_xor_sync(0xffffffffu, keep_b ? a : b, m);
+    };
+    Pair8<T> p[4], got[2], lo[2], hi[2];
+    get_pairs(x, p);
+    const int far = tpr >> 1;                                    // lanes w and w ^ far: the highest bit of the chain index w / 4
+    const bool up = (w & far) != 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
-    for (int m = 1; m < tpr; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
-    return fmaxf(sqrtf(ss), eps);
+    for (int i = 0; i < 2; ++i) got[i] = pair_xor(up ? p[i] : p[2 + i], far);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { lo[i] = up ? got[i] : p[i]; hi[i] = up ? p[2 + i] : got[i]; }
+    float s;
+    if (tpr == 16) {
+        const bool odd = (w & 4) != 0;
+        const Pair8<T> l_got = pair_xor(odd ? lo[0] : lo[1], 4), h_got = pair_xor(odd ? hi[0] : hi[1], 4);
+        const float2 c[4] = {pair_values(odd ? l_got : lo[0]), pair_values(odd ? lo[1] : l_got), pair_values(odd ? h_got : hi[0]), pair_values(odd ? hi[1] : h_got)};
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { s0 = fmaf(c[e].x, c[e].x, s0); s1 = fmaf(c[e].y, c[e].y, s1); }
+        s = halve(s0, s1, (w & 2) != 0, 2);                      // 16
+        s = fold(fold(fold(fold(s, 1), 8), 4), 2);               // 8, 4, 2, 1
+    } else {
+        float2 t[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float2 c0 = pair_values(lo[i]), c1 = pair_values(hi[i]);
+            t[i] = make_float2(fmaf(c1.x, c1.x, c0.x * c0.x), fmaf(c1.y, c1.y, c0.y * c0.y));
+        }
+        const bool k2 = (w & 2) != 0;
+        const float s0 = halve(t[0].x, t[1].x, k2, 2), s1 = halve(t[0].y, t[1].y, k2, 2);      // 16
+        s = halve(s0, s1, (w & 1) != 0, 1);                      // 8
+        s = fold(fold(fold(s, 4), 2), 1);                        // 4, 2, 1
+    }
+    return fmaxf(sqrtf(s), eps);
 }
 
 // Quantize one or two tensors of a step in one launch where their groupings have a kernel for it (varq_append.cu); VARQ_ERR_UNSUPPORTED
