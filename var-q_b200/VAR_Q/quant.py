@@ -5,8 +5,8 @@ Same constructor, methods and readable attributes as the reference class
 (VAR/models/basic_var.py:104-117,143-147; Infinity/infinity/models/basic.py:254-271,327-330)
 work unchanged.  What differs is underneath:
 
-* ``quant`` is one fused kernel launch (statistics, scale / zero-point, rounding, packing)
-  that writes straight into a pre-allocated packed cache; there is no ``torch.cat`` growth.
+* ``quant`` is one launch (statistics, scale / zero-point, rounding, packing; two for planes
+  too large for the registers of a cluster, more for groupings without such a kernel) that writes straight into a pre-allocated packed cache; there is no ``torch.cat`` growth.
 * the cache is held head-major ``[B, H, L, words]`` with compact parameter tables
   (one row per token, or one row per appended step for the modes whose parameters are
   constant over a step) instead of scales materialised along L;
