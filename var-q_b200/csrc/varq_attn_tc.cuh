@@ -61,10 +61,22 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(TC_WAIT_NS) : "memory");
     return ok != 0;
 }
+// Most waits of a steady loop find their phase complete.  try_wait with a time limit costs a couple of hundred cycles even then
+// (measured per wait site), test_wait a shared-memory round trip: it goes first.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Bounded wait.  Returns false when the limit expires or another thread has already given up.
 // Everything is inline and small: a call here costs a few hundred cycles of register shuffling
 // around it, at every one of the ~20 wait sites, and bloats the loops that hold them.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+    if (mbar_test(bar, parity)) return true;
     uint32_t tries = 0;
 #pragma unroll 1
     while (!mbar_try(bar, parity)) {     // a failed try_wait has already been suspended by the hardware for a while
@@ -76,8 +88,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         }
     }
     return true;
-}// The same by a converged warp, which stays converged: all lanes poll and agree.
+}
+// The same by a converged warp, which stays converged: all lanes poll and agree.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
     uint32_t tries = 0;
 #pragma unroll 1
     while (!__all_sync(0xffffffffu, mbar_try(bar, parity))) {
