@@ -19,7 +19,7 @@
 // The kernel is bound by instruction issue (softmax 4 x ~300 and conversion ~50 warp instructions per 16 codes of 64 keys), so more
 // than 128 queries share each converted tile (QT = 2, head_dim 64, all 512 TMEM columns); up to 128 queries run as two CTAs per
 // SM of 256 columns each, one CTA's set-up and dependent waits under the other's tiles.  At head_dim 128 the tensor pipe
-// is the closer bound (hi + lo operands: 4 products of 256 cycles per tile): one CTA keeps four score tiles in flight.
+// is the closer bound (hi + lo operands: 4 products of 256 cycles per tile): one CTA keeps three or four score tiles in flight.
 // Few CTAs over a long cache: the key range is split across CTAs and a second kernel merges the partial rows.
 // Numerics: integer codes are exact in fp16; an fp32 query is split into hi + lo fp16 halves, a dequantised K likewise (the lo x lo
 // product is below fp32 resolution), so S has fp32-like accuracy; P and a dequantised V are rounded to fp16 once; sums are fp32.
@@ -204,7 +204,13 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr bool KX = KM == PM_EXACT, VX = VM == PM_EXACT;
     static constexpr int CTAS = (D == 64 && QT == 1) ? 2 : 1;  // resident CTAs per SM
     // converter warps: a tile is 64 * D / 16 items of 16 codes
-    static constexpr int KW = D == 128 ? 8 : 2 * QT, VW = D == 128 ? 4 : 2 * QT;
+    // Two threads per query row at head_dim 128.  ALT: they take the even and the odd key tiles, each with its own reference maximum and
+    // accumulator in tensor memory, and meet in the epilogue, so the two warps of a sub-partition hide each other's latencies (score loads,
+    // barriers).  Else each takes half of every tile's keys and they agree on one reference: with two query operands (hi + lo) the second
+    // accumulator would leave room for two score tiles only, and the chain score product -> softmax -> output product then binds (B8 H16
+    // Lq2048 Lk4096 int4, us: one operand 985 -> 814, two operands 1028 -> 1131, so those stay; dequantised K is bound by its converters, 1035 -> 1032).
+    static constexpr bool ALT = D == 128 && NQ == 1 && KX;
+    static constexpr int KW = D == 128 ? (ALT ? 4 : 8) : 2 * QT, VW = D == 128 ? 4 : 2 * QT;
     static constexpr int KTHR = KW * 32, VTHR = VW * 32;
     static constexpr int HV = D == 128 ? 2 : 1;                // threads per query row
     static constexpr int K_WARP0 = 4 * HV * QT, V_WARP0 = K_WARP0 + KW, MMA_WARP = V_WARP0 + VW, LOAD_WARP = MMA_WARP + 2;     // one for K, one for V
@@ -219,7 +225,7 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr int T_BYTES = TC_N * D * 2;              // one fp16 operand tile
     static constexpr int KST = CTAS == 2 ? 2 : 3, VST = KST;  // operand stages
     static constexpr int PST = D == 128 ? 2 : KST;            // packed stages (at most KST)
-    static constexpr int SB = D == 64 ? 2 : 4;                // score tiles in tensor memory, per query tile
+    static constexpr int SB = D == 64 ? 2 : ALT ? 3 : 4;    // score tiles in tensor memory, per query tile
     static constexpr bool TAB = KX || VX;                     // per-key softmax tables
     static constexpr int TS = CTAS == 2 ? 8 : 16;             // table slots: more than PST + KST + SB tiles
     static constexpr int TAB_FLOATS = 4 * TC_N + 4;           // K scale, log2 V scale, 1 / V scale, K zero-point term; flag
@@ -236,7 +242,7 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static_assert(QT * SB <= 4 && KST <= 3 && TS > PST + KST + SB, "barrier plan");
     // TMEM columns: queries, output accumulators, score tiles
     static constexpr int TMEM_COLS = CTAS == 2 ? 256 : 512;
-    static constexpr int COL_Q = 0, COL_O = QT * NQ * D / 2, COL_S = COL_O + QT * D;
+    static constexpr int COL_Q = 0, COL_O = QT * NQ * D / 2, COL_S = COL_O + (ALT ? 2 : QT) * D;
     static_assert(COL_S + QT * SB * TC_N <= TMEM_COLS, "TMEM plan");
 };
 struct TcDyn {          // byte offsets of the launch-sized regions, from the aligned base of dynamic shared memory
@@ -497,7 +503,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
     if (warp == 0) {
         for (int i = lane; i < P::N_BARS; i += 32) {
             const uint32_t count = i >= 32 && i < 38 ? 33u : i < 4 + 3 ? (uint32_t)KTHR : i < 10 ? (uint32_t)VTHR
-                                 : i >= 14 && i < 18 ? (uint32_t)(32 * HV * max(1, i - 14 < SB ? aq0 : aq1)) : i == 21 ? (uint32_t)(32 * HV * aq)
+                                 : i >= 14 && i < 18 ? (uint32_t)(32 * (P::ALT ? 1 : HV) * max(1, i - 14 < SB ? aq0 : aq1)) : i == 21 ? (uint32_t)(32 * HV * aq)
                                  : (i >= 18 && i < 21) || i == 22 || (i >= 24 && i < 27) ? (uint32_t)n_qt : i >= 38 ? 64u : 1u;
             mbar_init(&bars[i], count);
         }
@@ -520,10 +526,11 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
     if (warp < P::K_WARP0) {
         // =============================================================== softmax / epilogue
         set_registers<P::REGS_SOFT, P::REGS>();
-        // Two threads share a query row, each owning 32 of a tile's 64 keys: four (two) softmax warps per SM sub-partition keep the
-        // exponential unit busy where one warp alone leaves it idle half of the time.  The pair (two warps of one sub-partition) agrees on
-        // the reference maximum by one barrier-with-reduction per tile.
-        constexpr int NC = N / HV, DH = D / HV;                 // score columns and head_dim values of a thread
+        // Two threads share a query row at head_dim 128 (TcPlan::ALT says how): four (two) softmax warps per SM sub-partition keep the
+        // exponential unit busy where one warp alone leaves it idle half of the time.  Without ALT the pair (two warps of one sub-partition)
+        // agrees on the reference maximum by one barrier-with-reduction per tile.
+        constexpr bool ALT = P::ALT;
+        constexpr int NC = ALT ? N : N / HV, DH = D / HV;       // score columns and (queries, epilogue) head_dim values of a thread
         const int t = QT == 1 ? 0 : warp / (4 * HV), half = HV == 1 ? 0 : (warp >> 2) & 1, quarter = warp & 3;
         if (quarter < (t ? aq1 : aq0)) {
             const int r = t * TC_M + quarter * 32 + lane;       // query row of the CTA; TMEM lane = r % 128
@@ -535,7 +542,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             const int bar_id = 3 + t * 4 + quarter;
             auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory"); };
             auto pair_any = [&](bool flag) -> bool {
-                if (HV == 1) return __any_sync(0xffffffffu, flag) != 0;
+                if (HV == 1 || ALT) return __any_sync(0xffffffffu, flag) != 0;
                 uint32_t any;
                 asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, %2, 64, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                              : "=r"(any) : "r"((uint32_t)flag), "r"(bar_id) : "memory");
@@ -606,20 +613,23 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 if constexpr (KX) qsum = pair_sum(qsum);
             }
             const float c = tc_factor(a.scale_log2);
-            float m_used = -FLT_MAX;                            // reference maximum (log2 domain), the same in both threads of a row
+            float m_used = -FLT_MAX;                            // reference maximum (log2 domain): with ALT the thread's own, else the same in both threads of a row
             float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;       // row sum of this thread's softmax weights
             bool ok = true;
-            // Once a wait has expired nothing is read or written any more, but the pair's barriers are still taken: both warps run
-            // all iterations.
+            const int first_col = ALT ? 0 : half * NC;          // of the tile's score columns
+            const uint32_t col_acc = lane_base + col_o + (ALT ? half * D : 0);
+            constexpr int STEP = ALT ? 2 : 1;
+            // Once a wait has expired nothing is read or written any more, but a pair's barriers are still taken: without ALT both warps
+            // run all iterations.
 #pragma unroll 1
-            for (int i = 0; i < T; ++i) {
+            for (int i = ALT ? half : 0; i < T; i += STEP) {
                 const int s = i % SB;
                 ok = ok && mbar_wait_warp(&bar_s[t * SB + s], (i / SB) & 1, abort_flag, 11);
                 if (P::TAB) ok = ok && mbar_wait_warp(&bar_t[i % TS], (i / TS) & 1, abort_flag, 12);
                 const uint32_t s_addr = lane_base + col_s + s * N;
-                const float* tab = reinterpret_cast<const float*>(smem + P::OFF_TAB) + (i % TS) * P::TAB_FLOATS + half * NC;
+                const float* tab = reinterpret_cast<const float*>(smem + P::OFF_TAB) + (i % TS) * P::TAB_FLOATS + first_col;
                 if (!ok) {
-                    if (HV == 1) break;
+                    if (HV == 1 || ALT) break;
                     if (pair_any(false)) pair_sync();
                     continue;
                 }
@@ -627,8 +637,8 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 float mx;
                 {
                     tc_fence_after();
-                    tmem_ld32(s_addr + half * NC, x);
-                    if constexpr (HV == 1) tmem_ld32(s_addr + 32, x + 32);
+                    tmem_ld32(s_addr + first_col, x);
+                    if constexpr (NC == 64) tmem_ld32(s_addr + 32, x + 32);
                     tmem_wait_ld();
                     // ---- scores in the log2 domain with the V scale folded in (tables), or raw (their factor c enters with the exponential)
                     if constexpr (KX || VX) {
@@ -647,7 +657,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
 #pragma unroll
                             for (int e = 0; e < 4; ++e) x[j + e] = __float_as_uint(y[e]);
                         }
-                        if (KX && __float_as_int(tab[4 * N - half * NC]) != 0) {        // a zero-point of this tile is too wide for the exact operand: its term in fp32
+                        if (KX && __float_as_int(tab[4 * N - first_col]) != 0) {        // a zero-point of this tile is too wide for the exact operand: its term in fp32
 #pragma unroll
                             for (int j = 0; j < NC; j += 4) {
                                 const float4 z4 = tab4(tab + 3 * N + j);
@@ -658,7 +668,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                             }
                         }
                     }
-                    const int nv = tile_n(i) - half * NC;
+                    const int nv = tile_n(i) - first_col;
                     if (nv < NC) {                                  // the last tile: columns past the cache hold anything
 #pragma unroll
                         for (int j = 0; j < NC; ++j) if (j >= nv) x[j] = __float_as_uint(TC_MASKED);
@@ -678,7 +688,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 if (pair_any(mt > m_used + TC_LAZY)) {
                     // Rare after the first tile: some row of these warps meets a score more than 2^12 above its reference.  Its maximum
                     // becomes the reference and what has been accumulated is rescaled (a factor 1 for the other rows).
-                    if (HV == 2) {
+                    if (HV == 2 && !ALT) {
                         xch[half * XH] = mt;
                         pair_sync();
                         mt = fmaxf(mt, xch[(half ^ 1) * XH]);
@@ -687,27 +697,27 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     const float alpha = ex2(m_used - m_new);    // 0 for a row without a reference yet
                     m_used = m_new;
                     l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
-                    if (i > 0) {
-                        ok = ok && mbar_wait(&bar_o[(i - 1) % VST], ((i - 1) / VST) & 1, abort_flag, 13);      // the accumulator is stable
+                    if (i >= STEP) {
+                        ok = ok && mbar_wait(&bar_o[(i - STEP) % VST], ((i - STEP) / VST) & 1, abort_flag, 13);      // the accumulator is stable
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) continue;
                         {
                             tc_fence_after();
 #pragma unroll 1
-                            for (int c0 = half * DH; c0 < (half + 1) * DH; c0 += 16) {
+                            for (int c0 = ALT ? 0 : half * DH; c0 < (ALT ? D : (half + 1) * DH); c0 += 16) {
                                 uint32_t o[16];
-                                tmem_ld16(lane_base + col_o + c0, o);
+                                tmem_ld16(col_acc + c0, o);
                                 tmem_wait_ld();
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-                                tmem_st16(lane_base + col_o + c0, o);
+                                tmem_st16(col_acc + c0, o);
                             }
                             tmem_wait_st();
                         }
                     }
                 }
                 {
-                    // ---- P = 2^(x - m), fp16 pairs over the score columns (both threads of the row have read theirs)
+                    // ---- P = 2^(x - m), fp16 pairs over the score columns 
                     const float nm = -m_used;
                     uint32_t ph[NC / 2];
 #pragma unroll
@@ -724,7 +734,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                         ph[j / 2] = *reinterpret_cast<const uint32_t*>(&h01);
                         ph[j / 2 + 1] = *reinterpret_cast<const uint32_t*>(&h23);
                     }
-                    if constexpr (HV == 1) tmem_st32(s_addr, ph); else tmem_st16(s_addr + half * 16, *reinterpret_cast<uint32_t (*)[16]>(ph));
+                    if constexpr (NC == 64) tmem_st32(s_addr, ph); else tmem_st16(s_addr + half * 16, *reinterpret_cast<uint32_t (*)[16]>(ph));
                     // the row sum adds up the rounded P that multiplies V: a row dominated by one key stays exact
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) {
@@ -744,7 +754,19 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 }
             }
             // ---- output row: each thread writes half of its head_dim
-            const float l = pair_sum((l0 + l1) + (l2 + l3));
+            // (ALT) the accumulators of the two threads meet: f0 and f1 bring tiles of even and odd index to the common reference (0 where
+            // a thread had no tile; the second accumulator is then not read either).
+            float l = (l0 + l1) + (l2 + l3), f0 = 1.f, f1 = 0.f;
+            if constexpr (!ALT) l = pair_sum(l);
+            else {
+                xch[half * XH] = m_used;
+                pair_sync();
+                const float m0 = xch[0], m1 = xch[XH];
+                m_used = fmaxf(m0, m1);
+                f0 = ex2(m0 - m_used);
+                f1 = ex2(m1 - m_used);
+                l = pair_sum(l * (half ? f1 : f0));
+            }
             ok = ok && mbar_wait(bar_end, 0, abort_flag, 14);
             ok = __all_sync(0xffffffffu, ok);
             if (ok) {
@@ -757,6 +779,20 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     uint32_t o[32];
                     tmem_ld32(lane_base + col_o + c0, o);
                     tmem_wait_ld();
+                    if constexpr (ALT) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f0);
+                        if (T > 1) {
+#pragma unroll
+                            for (int u = 0; u < 32; u += 16) {
+                                uint32_t o1[16];
+                                tmem_ld16(lane_base + col_o + D + c0 + u, o1);
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) o[u + j] = __float_as_uint(fmaf(__uint_as_float(o1[j]), f1, __uint_as_float(o[u + j])));
+                            }
+                        }
+                    }
                     if (live) {
                         auto put = [&](auto bits_c) {
                             float v[32];
@@ -856,7 +892,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         // =============================================================== MMA issue (the whole warp waits; one elected lane issues)
         // Per query tile: S(0) .. S(SB-1), then per key tile i: wait P(i) -> O += P(i) V(i) -> S(i + SB), which overwrites the columns of
         // S(i) / P(i).  A warp spends as long on the waits and the issue of a tile's products as the tensor pipe on the products, so
-        // two warps share the work: one per query tile (QT = 2), or one for S and one for O (head_dim 128, four score tiles deep).
+        // two warps share the work: one per query tile (QT = 2), or one for S and one for O (head_dim 128).
         constexpr bool ROLES = D == 128;
         const int mw = warp - MMA_WARP, t = ROLES ? 0 : mw;
         constexpr uint32_t IDESC_S = instr_desc(TC_M, N, 0), IDESC_O = instr_desc(TC_M, D, 1);
@@ -886,16 +922,16 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         };
         auto issue_o = [&](int i) {
             const uint64_t vd = vd0 + (uint64_t)(((i % VST) * P::T_BYTES) >> 4);
-            const uint32_t pa = col_s + (i % SB) * N;
-            const uint32_t more = i > 0 ? 1u : 0u;
+            const uint32_t pa = col_s + (i % SB) * N, acc = col_o + (P::ALT ? (i & 1) * D : 0);
+            const uint32_t more = i >= (P::ALT ? 2 : 1) ? 1u : 0u;
             const int n = tile_n(i);                     // P columns / V rows past the keys are never read
-            tc_mma_ts(col_o, pa, vd, IDESC_O, more);
+            tc_mma_ts(acc, pa, vd, IDESC_O, more);
             if (n > 48) {
 #pragma unroll
-                for (int kk = 1; kk < N / 16; ++kk) tc_mma_ts(col_o, pa + kk * 8, vd + (uint64_t)((kk * 2048) >> 4), IDESC_O, 1u);
+                for (int kk = 1; kk < N / 16; ++kk) tc_mma_ts(acc, pa + kk * 8, vd + (uint64_t)((kk * 2048) >> 4), IDESC_O, 1u);
             } else {
-                if (n > 16) tc_mma_ts(col_o, pa + 8, vd + (uint64_t)(2048 >> 4), IDESC_O, 1u);
-                if (n > 32) tc_mma_ts(col_o, pa + 16, vd + (uint64_t)(4096 >> 4), IDESC_O, 1u);
+                if (n > 16) tc_mma_ts(acc, pa + 8, vd + (uint64_t)(2048 >> 4), IDESC_O, 1u);
+                if (n > 32) tc_mma_ts(acc, pa + 16, vd + (uint64_t)(4096 >> 4), IDESC_O, 1u);
             }
             tc_commit(&bar_o[i % VST]);
             if (ROLES) tc_commit(&bar_sf[i % SB]);
