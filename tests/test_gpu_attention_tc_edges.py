@@ -1,0 +1,42 @@
+"""The tensor-core kernel, forced, at the edges of its tiles: one, two and three key tiles per row (head_dim 128 gives even and odd tiles to
+different threads), a second query tile, split key ranges, a reference maximum that moves.
+Tolerance: max-abs 2e-3, relative L2 1e-3 (fp32 oracle)."""
+import pytest
+import torch
+
+from oracle import varq_oracle as O
+from VAR_Q import _cabi
+from VAR_Q.attention import attend_cached
+from VAR_Q.quant import VAR_Q
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(autouse=True)
+def _auto_path_afterwards():
+    yield
+    _cabi.force_attn_path(None)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("q_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("kb,vb,options", [(8, 8, {}), (4, 2, dict(symmetric=False)), (4, 4, dict(group_size=32))])
+@pytest.mark.parametrize("lq,lk,gain", [(1, 1, 1.0), (128, 64, 1.0), (129, 65, 1.0), (200, 128, 300.0), (33, 129, 300.0), (20, 1500, 1.0)])
+def test_against_the_oracle(D, q_dtype, kb, vb, options, lq, lk, gain):
+    fmt, B, H = "BHLc", 1, 2
+    kq, vq = (VAR_Q(b, fmt, "G_TOKEN_HEAD", **options) for b in (kb, vb))
+    kr, vr = (O.OracleVARQ(b, fmt, "G_TOKEN_HEAD", **options) for b in (kb, vb))
+    k = O.synthetic_kv((B, H, lk, D), fmt, 3 + lk, n_outlier=0)
+    k = k / k.norm(dim=-1, keepdim=True) * torch.linspace(0.2, 1.0, lk).view(1, 1, lk, 1)        # later keys weigh more
+    v = O.synthetic_kv((B, H, lk, D), fmt, 5 + lk, n_outlier=0)
+    kq.append(k.to(DEV)); vq.append(v.to(DEV))
+    kd, vd = kr.use_var_q(k), vr.use_var_q(v)
+    q = torch.randn((B, H, lq, D), generator=torch.Generator().manual_seed(lq + lk))
+    q = (q / q.norm(dim=-1, keepdim=True) * gain).to(q_dtype)
+    _cabi.force_attn_path("tc")
+    out = attend_cached(q.to(DEV), kq, vq, 1.0, out_dtype=torch.float32).cpu()
+    ref = O.attention(q.float(), kd, vd, fmt, 1.0).transpose(1, 2)
+    err, rel = (out - ref).abs().max().item(), ((out - ref).norm() / ref.norm()).item()
+    assert err <= 2e-3 and rel <= 1e-3, f"max-abs {err:.3e}, rel-L2 {rel:.3e}"
+    assert _cabi.device_status() == 0
