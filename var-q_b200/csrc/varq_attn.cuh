@@ -17,7 +17,7 @@ struct AttnArgs {
     int splits, tiles_per_split;
     int n_qtiles;               // query tiles per (sample, head); grids are 1-D: ((b*H + h) * n_qtiles + qtile) * splits + split
     float* ws;                  // partials: [(b,h,qtile,split)][QT*(2+D)]
-    // Queries normalised on the way in (tensor-core kernel): q / max(||q||_2, q_eps) * q_mul[h]; q_mul may be null (= 1)
+    // Queries normalised on the way in (every kernel but attn_mid_kernel): q / max(||q||_2, q_eps) * q_mul[h]; q_mul may be null (= 1)
     int q_norm = 0;
     const float* q_mul = nullptr;
     float q_eps = 0.f;

@@ -59,27 +59,26 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     a.scale_log2 = softmax_scale * 1.4426950408889634f;
     a.splits = 1; a.tiles_per_split = 0; a.n_qtiles = 1; a.ws = reinterpret_cast<float*>(workspace);
     a.q_norm = q_norm ? 1 : 0; a.q_mul = q_mul; a.q_eps = q_eps;
-    if (q_norm) {       // the tensor-core kernels normalise queries as they load them
-        if (Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
-        if (!attn_tc_eligible(a, kb, vb)) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd_qnorm: no kernel normalises the queries of this shape or layout");
-        return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
-    }
+    if (q_norm && !attn_tc_eligible(a, kb, vb)) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd_qnorm: no kernel normalises the queries of this shape or layout");
     // The CUDA-core streaming kernel is memory-bound only while its arithmetic (queries x keys x head_dim on the FMA pipe)
     // stays below the time to stream the packed cache: up to 4 queries at any cache length, and the 1-16-query first scales
     // of a schedule, whose caches are a few hundred tokens at most.  Everything else goes to the tensor cores, where a
-    // 128-row tile with few live rows still finishes a long cache sooner.
+    // 128-row tile with few live rows still finishes a long cache sooner.  Queries normalised on the way in follow the same rules as
+    // queries that arrive normalised, so that few of them keep fp32 weights: on the tcgen05 kernel (weights and dequantised V in
+    // fp16) the first scales of a per-dim or group-wise cache are 2e-4 away from the exact result, here 2e-7.
     const int force = __atomic_load_n(&g_forced_path, __ATOMIC_RELAXED);
-    // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key
-    // (B64 H16 c128 int4, 10521 tokens, us: 315 / 515 / 906 for 1 / 8 / 16 queries; tcgen05 1354 whatever the count, streaming 954 / 3721 / 7294;
-    // the lead over tcgen05 ends at 16 queries, on short caches too).
-    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : (Lq <= 16 && Lk > 256);
-    if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool small_q = Lq <= 4 || (Lq <= 16 && Lk <= 256);
     // Between the two: tens of queries over at most a few hundred tokens (the early scales of a schedule), where the tcgen05
     // kernel is bound by its per-CTA set-up; a warp-level tensor-core kernel takes them when the parameters are per key.
     const bool mid_q = Lq > 8 && Lq <= 64 && Lk <= 256;          // measured against both neighbours (B64 H16 and B128 H30, c 64)
+    // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key.
+    // (B64 H16 c128 int4, 10521 tokens, us: 315 / 515 / 906 for 1 / 8 / 16 queries; tcgen05 1354 whatever the count, streaming 954 / 3721 / 7294).
+    // It also stands in for the next kernel, which does not normalise (B64 H16 c64 int8, us, decode / streaming: 20 / 45 at 9 queries over
+    // 14 tokens, 22 / 41 at 16 over 30).
+    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (q_norm && mid_q && D == 64));
+    if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : mid_q;
-    if (want_mid && attn_mid_eligible(a, kb, vb)) return attn_mid_run(a, kb, vb, (cudaStream_t)stream);
+    if (want_mid && !q_norm && attn_mid_eligible(a, kb, vb)) return attn_mid_run(a, kb, vb, (cudaStream_t)stream);
     const bool want_tc = force ? (force == VARQ_ATTN_PATH_TC) : !small_q;
     if (want_tc && attn_tc_eligible(a, kb, vb)) return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool want_stream = force ? (force == VARQ_ATTN_PATH_STREAM) : small_q;

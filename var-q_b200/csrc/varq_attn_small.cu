@@ -78,13 +78,25 @@ __global__ void __launch_bounds__(A1_THREADS) attn_small_kernel(AttnArgs a) {
     const int nq = min(QT, a.Lq - q0);
 
     // ---- queries -> shared (scaled), per-group sums
+    const float q_scale = a.q_norm ? 1.f : a.scale_log2;
     for (int i = tid; i < QT * D; i += A1_THREADS) {
         const int qi = i / D, d = i - qi * D;
         float v = 0.f;
-        if (qi < nq) v = load_q_elem(a.q, a.q_dtype, b * a.qs_b + (long long)(q0 + qi) * a.qs_l + h * a.qs_h + d) * a.scale_log2;
+        if (qi < nq) v = load_q_elem(a.q, a.q_dtype, b * a.qs_b + (long long)(q0 + qi) * a.qs_l + h * a.qs_h + d) * q_scale;
         sQ[i] = v;
     }
     __syncthreads();
+    if (a.q_norm) {     // x / max(||x||_2, eps) * scale_mul[h] in fp32: one warp per query, the length summed in the order of qk_norm_stats_kernel
+        static_assert(A1_THREADS == 32 * QT, "one warp per query");
+        float* row = sQ + warp * D;
+        float ss = 0.f;
+        for (int d = lane; d < D; d += 32) ss = fmaf(row[d], row[d], ss);
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+        const float len = fmaxf(sqrtf(ss), a.q_eps), mul = a.q_mul ? __ldg(a.q_mul + h) : 1.f;
+        for (int d = lane; d < D; d += 32) row[d] = __fdiv_rn(row[d], len) * mul * a.scale_log2;
+        __syncthreads();
+    }
     for (int i = tid; i < QT * gk; i += A1_THREADS) {
         const int qi = i / gk, g = i - qi * gk;
         float s = 0.f;

@@ -123,6 +123,16 @@ __global__ void __launch_bounds__(WARPS * 32) attn_stream_kernel(AttnArgs a, int
             load_q8(a.q, a.q_dtype, off, lo8);
             load_q8(a.q, a.q_dtype, off + 8, hi8);
         }
+        if (a.q_norm) {                 // x / max(||x||_2, eps) * scale_mul[h] in fp32, on the way in
+            float ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss = fmaf(hi8[j], hi8[j], fmaf(lo8[j], lo8[j], ss));
+#pragma unroll
+            for (int m = 1; m < LPK; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+            const float len = fmaxf(sqrtf(ss), a.q_eps), mul = a.q_mul ? __ldg(a.q_mul + h) : 1.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { lo8[j] = __fdiv_rn(lo8[j], len) * mul; hi8[j] = __fdiv_rn(hi8[j], len) * mul; }
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             q[qi][j] = lo8[j] * a.scale_log2;
