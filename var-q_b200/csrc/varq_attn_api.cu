@@ -72,9 +72,12 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     // kernel is bound by its per-CTA set-up; a warp-level tensor-core kernel takes them when the parameters are per key.
     const bool mid_q = Lq > 8 && Lq <= 64 && Lk <= 256;          // measured against both neighbours (B64 H16 and B128 H30, c 64)
     // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key.
-    // (B64 H16 c128 int4, 10521 tokens, us: 315 / 515 / 906 for 1 / 8 / 16 queries; tcgen05 1354 whatever the count, streaming 954 / 3721 / 7294).
-    // It also stands in for the next kernel, which does not normalise (B64 H16 c64 int8, us, decode / streaming: 20 / 45 at 9 queries over
-    // 14 tokens, 22 / 41 at 16 over 30).
+    // us at H16, int4, bf16 queries, decode / tcgen05 (the streaming kernel takes 1.8 to 6 times decode's time):
+    //     B64 c64   8 x 300: 22 / 47, 16 x 300: 37 / 47, 16 x 2240: 205 / 179, 8 x 10521: 421 / 754, 16 x 10521: 763 / 757
+    //     B64 c128  8 x 300: 42 / 75, 16 x 300: 73 / 75, 16 x 2240: 325 / 229, 8 x 10521: 660 / 893, 16 x 10521: 1199 / 902
+    //     B2  c128  8 x 300: 10.4 / 10.0, 16 x 2240: 26 / 20, 16 x 10521: 50 / 44;   B2 c64  16 x 2240: 18 / 21, 16 x 10521: 39 / 56
+    // Up to 8 queries (one CTA's worth) it is the faster one; from 9 to 16 it takes 0.6 to 1.4 times as long and stays for its
+    // accuracy (3e-7 against 2e-4 for fp16 weights).  It also stands in for the next kernel, which does not normalise.
     const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (q_norm && mid_q && D == 64));
     if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : mid_q;
