@@ -65,15 +65,24 @@ size_t attn_tc_workspace_bytes(int B, int H, int Lq, int Lk, int D) {
     return (size_t)B * H * splits * ((Lq + rows - 1) / rows) * rows * (D + 2) * sizeof(float) + 256;
 }
 
-// Step tables of at most this many bytes (K and V together) fit behind the fixed part of every plan of the head_dim: 65 steps of K and
-// V at 64, 18 at 128 (the schedules of the models have 10 to 13)
-static int step_table_room(int D) { return D == 64 ? 50 * 1024 : 28 * 1024; }
-static int par_mode(const ParamView& pv, int D, int& room) {
+// Step tables of at most this many bytes (K and V together) fit behind the fixed part of every plan of the head_dim: 66 steps of K and
+// V at 64, 18 at 128 (the schedules of the models have 10 to 13).  Longer histories, and those whose number of steps is not given, have
+// tables that move along (28 KB at both head_dims: at 64 two CTAs then share an SM).  B8 H16 c128, 256 bf16 queries over 2560 tokens in
+// 18 / 40 / 64 steps of K and V, us: 117 / 150 / 180, and 537 for 40 and 64 on the fp32 routine.
+constexpr int STEP_TABLE_BYTES_64 = 50 * 1024, STEP_TABLE_BYTES = 28 * 1024;
+static int par_mode(const ParamView& pv, int D) {
     if (pv.group == D) return PM_EXACT;
     if (pv.group % 16 == 0 && (pv.group & (pv.group - 1)) == 0 && D / pv.group <= 4) return PM_GROUP;
-    const long long bytes = (long long)pv.n_rows * 3 * D * 2;
-    if (pv.row_of_token && pv.n_rows > 0 && bytes <= room) { room -= (int)bytes; return PM_STEP; }
-    return PM_SLOW;
+    return pv.row_of_token ? PM_STEP : PM_SLOW;
+}
+static void step_tables(const AttnArgs& a, TcDyn& dy) {
+    const bool ks = dy.k_mode == PM_STEP, vs = dy.v_mode == PM_STEP;
+    const long long k = ks ? a.kp.n_rows : 0, v = vs ? a.vp.n_rows : 0;
+    const bool known = (!ks || k > 0) && (!vs || v > 0);
+    if (known && (k + v) * 3 * a.D * 2 <= (a.D == 64 ? STEP_TABLE_BYTES_64 : STEP_TABLE_BYTES)) { dy.k_rows = (int)k; dy.v_rows = (int)v; return; }
+    const int room = STEP_TABLE_BYTES / (3 * a.D * 2);
+    if (ks) { dy.k_mode = PM_WINDOW; dy.k_rows = vs ? room / 2 : room; }
+    if (vs) { dy.v_mode = PM_WINDOW; dy.v_rows = room - dy.k_rows; }
 }
 static int bulk_params(const ParamView& pv, int D) {
     const int ng = D / pv.group;
@@ -85,21 +94,23 @@ int attn_tc_run(const AttnArgs& a0, int kb, int vb, void* ws, size_t ws_bytes, c
     AttnArgs a = a0;
     // fp16 queries, and bf16 queries inside fp16's normal range (2^-14 <= |q| <= 65504), are exact in one fp16 term;
     // larger magnitudes saturate, smaller ones lose low bits (both far outside what a softmax can resolve)
-    const bool split_q = a.q_dtype == VARQ_F32 || a.q_norm;
+    bool split_q = a.q_dtype == VARQ_F32 || a.q_norm;
     const size_t need = attn_tc_workspace_bytes(a.B, a.H, a.Lq, a.Lk, a.D);
     if (!ws || ws_bytes < need)
         return fail(VARQ_ERR_WORKSPACE, "varq_attn_fwd: workspace of %zu bytes needed, %zu given", need, ws_bytes);
     a.splits = tc_splits(a.B, a.H, a.Lq, a.Lk, a.D, a.tiles_per_split);
     a.ws = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(ws) + 15) & ~(uintptr_t)15);
-    const int qt = tc_query_tiles(a.Lq, a.D), rows = qt * TC_M;
+    TcDyn dy = {};
+    dy.k_mode = par_mode(a.kp, a.D);
+    dy.v_mode = par_mode(a.vp, a.D);
+    step_tables(a, dy);
+    const bool window = dy.k_mode == PM_WINDOW || dy.v_mode == PM_WINDOW;
+    const int qt = window ? 1 : tc_query_tiles(a.Lq, a.D), rows = qt * TC_M;       // (fewer rows of partials than the workspace is sized for)
     a.n_qtiles = (a.Lq + rows - 1) / rows;
     if ((long long)a.B * a.H * a.n_qtiles * a.splits * rows > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 query rows");
-    TcDyn dy = {};
-    int room = step_table_room(a.D);
-    dy.k_mode = par_mode(a.kp, a.D, room);
-    dy.v_mode = par_mode(a.vp, a.D, room);
     dy.k_bulk = dy.k_mode == PM_GROUP && bulk_params(a.kp, a.D);
     dy.v_bulk = dy.v_mode == PM_GROUP && bulk_params(a.vp, a.D);
+    split_q = split_q || window;
     const TcFile& f = a.D == 128 ? (split_q ? tc_d128_q2 : tc_d128_q1)
                     : qt == 2 ? (split_q ? tc_d64_x2_q2 : tc_d64_x2_q1) : (split_q ? tc_d64_q2 : tc_d64_q1);
     if (int rc = f.launch(a, dy, kb, vb, st)) return rc;

@@ -197,8 +197,12 @@ enum ParMode : int {
     PM_EXACT = 0,     // one scale / zero-point per key: integer codes, scale applied outside the product
     PM_GROUP = 1,     // raw (key, group) parameters of a tile in shared memory: groups of whole 16-code items, at most 4 per key
     PM_STEP = 2,      // per-dim parameters shared by the tokens of an appended step: a table [steps][3][D] in shared memory
-    PM_SLOW = 3,      // anything else: fp32 parameters straight from global memory (runs in the PM_GROUP kernels)
+    PM_WINDOW = 3,    // the same with more steps than such a table holds: it keeps consecutive steps and moves on where a tile needs others.
+                      // A mode of its own, with one query tile and split queries only: in the kernels above the test per tile cost 4 %
+    PM_SLOW = 4,      // anything else: fp32 parameters straight from global memory (runs in the PM_GROUP kernels)
 };
+
+__host__ __device__ constexpr bool per_step(int mode) { return mode == PM_STEP || mode == PM_WINDOW; }
 
 template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr bool KX = KM == PM_EXACT, VX = VM == PM_EXACT;
@@ -248,7 +252,8 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
 struct TcDyn {          // byte offsets of the launch-sized regions, from the aligned base of dynamic shared memory
     int pkk, pkv;       // packed rows: two stages each
     int krec, vrec;     // records: two stages each
-    int ktab, vtab;     // step tables
+    int ktab, vtab;     // step tables ...
+    int k_rows, v_rows; // ... and the steps that they hold (PM_WINDOW: and one more row)
     int k_stage, v_stage, krec_stage, vrec_stage;
     int k_mode, v_mode;
     int k_bulk, v_bulk; // grouped parameters of consecutive tokens are contiguous and 16-byte aligned: bulk copies
@@ -257,6 +262,7 @@ struct TcDyn {          // byte offsets of the launch-sized regions, from the al
 // code - zp stays an exact fp16 integer and its product with the scale inside fp16's range
 __device__ __forceinline__ bool par_in_bounds(float s, float z) { return fabsf(z) <= 512.f && s < 60.f; }
 __device__ __forceinline__ uint32_t half_pair(float v) { return (uint32_t)__half_as_ushort(__float2half_rn(v)) * 0x10001u; }
+constexpr int STEPS_TO_MOVE = 16;                // a table moves for a tile of fewer steps (64 one-token steps per tile, us: 100 when it moved, 62 without)
 constexpr uint32_t PAR_SLOW = 0x7e007e00u;        // NaN in place of a zero-point constant: the item takes the fp32 routine
 
 // What the fp32 routine needs of a ParamView, with the (sample, head) part of the index folded into the pointers.
@@ -318,6 +324,31 @@ __device__ __forceinline__ void scale_pair(uint32_t& d, uint32_t& lo, uint32_t s
 }
 // The per-dim parameters of a thread's 16-wide head_dim slice, kept in registers while consecutive keys belong to one step
 struct StepRegs { uint32_t sh[8], sl[8], nz[8]; int step; };
+// Parameters of n steps from r0 on -> a table fp16 [n][3][D]: scale hi, scale lo, zero-point constant, in operand order (the
+// zero-point constants of a 16-wide slice start with PAR_SLOW when one of its elements is out of bounds).  By nthr threads.
+template <int D>
+__device__ __forceinline__ void fill_steps(unsigned char* steptab, const ParamRef* ref, int r0, int n, int bits, int ptid, int nthr) {
+    __half* tb = reinterpret_cast<__half*>(steptab);
+#pragma unroll 1
+    for (int e = ptid; e < n * (D / 16); e += nthr) {
+        const int slot = e / (D / 16), row = r0 + slot, d0 = (e - slot * (D / 16)) * 16;
+        bool slow = false;
+        __half* t = tb + slot * 3 * D + d0;
+#pragma unroll 8
+        for (int p = 0; p < 16; ++p) {
+            const long long pi = ref->index(row, d0 + (bits == 8 ? code_at(8, p) : bits == 4 ? code_at(4, p) : code_at(2, p)));
+            const float sv = __ldg(ref->scale + pi), zv = ref->zp ? __ldg(ref->zp + pi) : 0.f;
+            slow = slow || !par_in_bounds(sv, zv);
+            const __half s_hi = __float2half_rn(sv);
+            const int cls = p >> 1;
+            const float base = bits == 8 ? Item<8>::neg_base(0) : bits == 4 ? Item<4>::neg_base(cls & 1) : Item<2>::neg_base(cls & 3);
+            t[p] = s_hi;
+            t[D + p] = __float2half_rn(sv - __half2float(s_hi));
+            t[2 * D + p] = __float2half_rn(base - zv);
+        }
+        if (slow) *reinterpret_cast<uint32_t*>(t + 2 * D) = PAR_SLOW;
+    }
+}
 
 // One operand tile by NTHR threads.  SPLIT: hi + lo tiles (K), otherwise one tile.  Neighbouring lanes take the items of one
 // key: contiguous reads, and a quarter-warp's 16-byte stores land in eight different bank groups.  A thread keeps its head_dim slice
@@ -347,7 +378,7 @@ __device__ __forceinline__ void convert_tile(unsigned char* tile, const unsigned
             uint32_t d[8], lo[8];
             Item<BITS>::raw(w[it], d, cm);
             if constexpr (MODE == PM_STEP) {
-                const int step = reinterpret_cast<const uint16_t*>(rec)[key];
+                const int step = reinterpret_cast<const uint16_t*>(rec)[key];        // its slot in the table
                 if (step != sr.step) {
                     const uint4* t = reinterpret_cast<const uint4*>(steptab + (step * 3 * D + d0) * 2);
                     constexpr int TD = D * 2 / 16;      // uint4 per table row
@@ -467,6 +498,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzle atoms need 1024-byte alignment
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P::OFF_BAR);
+    // bars + 0, 1: [PM_WINDOW] the threads of a converter role, K and V, before and after their step table moves
     uint64_t* bar_pk = bars + 32;     // [PST] packed K rows (tx bytes) and records (load warp) of a tile in place
     uint64_t* bar_pv = bars + 35;     // [PST] the same for V
     uint64_t* bar_k = bars + 4;       // [KST] K operand tile written
@@ -497,12 +529,17 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
     const int t0 = split * a.tiles_per_split;                              // first key tile of this CTA
     const int T = min(a.tiles_per_split, (a.Lk + N - 1) / N - t0);         // and how many
     auto tile_n = [&](int i) -> int { return min(N, a.Lk - (t0 + i) * N); };
+    // the steps [x, y) that a step table starts with: from the first tile's on, as many as are known and fit
+    auto first_steps = [&](const ParamView& pv, int tab_rows) {
+        const int r = t0 == 0 ? 0 : pv.row(t0 * N);
+        return make_int2(r, max(r, min(r + tab_rows, pv.n_rows)));
+    };
     const int aq = (nq + 31) >> 5;                  // blocks of 32 rows that hold real queries, ...
     const int aq0 = min(aq, 4), aq1 = max(aq - 4, 0);    // ... per query tile
 
     if (warp == 0) {
         for (int i = lane; i < P::N_BARS; i += 32) {
-            const uint32_t count = i >= 32 && i < 38 ? 33u : i < 4 + 3 ? (uint32_t)KTHR : i < 10 ? (uint32_t)VTHR
+            const uint32_t count = i >= 32 && i < 38 ? 33u : i == 1 ? (uint32_t)VTHR : i < 4 + 3 ? (uint32_t)KTHR : i < 10 ? (uint32_t)VTHR
                                  : i >= 14 && i < 18 ? (uint32_t)(32 * (P::ALT ? 1 : HV) * max(1, i - 14 < SB ? aq0 : aq1)) : i == 21 ? (uint32_t)(32 * HV * aq)
                                  : (i >= 18 && i < 21) || i == 22 || (i >= 24 && i < 27) ? (uint32_t)n_qt : i >= 38 ? 64u : 1u;
             mbar_init(&bars[i], count);
@@ -820,29 +857,15 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         const int mode = is_k ? dy.k_mode : dy.v_mode, bits = is_k ? kb : vb;
         unsigned char* steptab = smem + (is_k ? dy.ktab : dy.vtab);
         if ((is_k ? KM : VM) == PM_STEP) {
-            // table of the steps' parameters: fp16 [steps][3][D] = scale hi, scale lo, zero-point constant, in operand order (the zero-point
-            // constants of a 16-wide slice start with PAR_SLOW when one of its elements is out of bounds)
-            const int n_steps = is_k ? a.kp.n_rows : a.vp.n_rows, nthr = is_k ? KTHR : VTHR;
-            __half* tb = reinterpret_cast<__half*>(steptab);
-#pragma unroll 1
-            for (int e = ptid; e < n_steps * (D / 16); e += nthr) {
-                const int row = e / (D / 16), d0 = (e - row * (D / 16)) * 16;
-                bool slow = false;
-                __half* t = tb + row * 3 * D + d0;
-#pragma unroll 8
-                for (int p = 0; p < 16; ++p) {
-                    const long long pi = ref->index(row, d0 + (bits == 8 ? code_at(8, p) : bits == 4 ? code_at(4, p) : code_at(2, p)));
-                    const float sv = __ldg(ref->scale + pi), zv = ref->zp ? __ldg(ref->zp + pi) : 0.f;
-                    slow = slow || !par_in_bounds(sv, zv);
-                    const __half s_hi = __float2half_rn(sv);
-                    const int cls = p >> 1;
-                    const float base = bits == 8 ? Item<8>::neg_base(0) : bits == 4 ? Item<4>::neg_base(cls & 1) : Item<2>::neg_base(cls & 3);
-                    t[p] = s_hi;
-                    t[D + p] = __float2half_rn(sv - __half2float(s_hi));
-                    t[2 * D + p] = __float2half_rn(base - zv);
-                }
-                if (slow) *reinterpret_cast<uint32_t*>(t + 2 * D) = PAR_SLOW;
-            }
+            fill_steps<D>(steptab, ref, 0, is_k ? a.kp.n_rows : a.vp.n_rows, bits, ptid, is_k ? KTHR : VTHR);
+            if (is_k) asm volatile("bar.sync 1, %0;" ::"n"(KTHR) : "memory");
+            else asm volatile("bar.sync 2, %0;" ::"n"(VTHR) : "memory");
+        }
+        if ((is_k ? KM : VM) == PM_WINDOW) {       // the steps of the first tiles, and the row of the keys whose step is not there: their items take the fp32 routine
+            const int rows = is_k ? dy.k_rows : dy.v_rows, nthr = is_k ? KTHR : VTHR;
+            const int2 w = first_steps(is_k ? a.kp : a.vp, rows);
+            fill_steps<D>(steptab, ref, w.x, w.y - w.x, bits, ptid, nthr);
+            for (int d = ptid; d < D / 2; d += nthr) reinterpret_cast<uint32_t*>(steptab + (rows * 3 + 2) * D * 2)[d] = PAR_SLOW;
             if (is_k) asm volatile("bar.sync 1, %0;" ::"n"(KTHR) : "memory");
             else asm volatile("bar.sync 2, %0;" ::"n"(VTHR) : "memory");
         }
@@ -851,6 +874,17 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         const int zp_off = (is_k ? a.kp.zp : a.vp.zp) ? N * ng : 0;       // raw zero-points behind the raw scales of a tile
         StepRegs sr;
         sr.step = -1;
+        // A tile whose steps are not in the table: the load warp says which steps take their place.  All threads of the role meet before, when
+        // they are through with the old ones, and after; on barriers with a limit, because a thread whose wait has expired does not come.
+        auto move_table = [&](const int2 w, uint64_t* bar, int nthr) -> bool {
+            mbar_arrive(bar);
+            if (!mbar_wait(bar, 0, abort_flag, 25)) return false;
+            fill_steps<D>(steptab, ref, w.x, w.y, bits, ptid, nthr);
+            mbar_arrive(bar);
+            sr = StepRegs{};
+            sr.step = -1;
+            return mbar_wait(bar, 1, abort_flag, 26);
+        };
         if (is_k) {
             auto loop = [&](auto bits_c) {
                 constexpr int BITS = decltype(bits_c)::value;
@@ -862,7 +896,12 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     bool ok = mbar_wait(&bar_pk[ps], (i / PST) & 1, abort_flag, 21);
                     if (ok && i >= KST) ok = mbar_wait(&bar_kf[ks], ((i - KST) / KST) & 1, abort_flag, 22);    // K stage is free
                     if (!ok) break;
-                    convert_tile<BITS, D, KTHR, KM, !KX>(smem + P::OFF_K + ks * P::KT * P::T_BYTES, smem + dy.pkk + ps * dy.k_stage, smem + dy.krec + ps * dy.krec_stage,
+                    const unsigned char* rec = smem + dy.krec + ps * dy.krec_stage;
+                    if constexpr (KM == PM_WINDOW) {
+                        const int2 w = *reinterpret_cast<const int2*>(rec + N * 2);
+                        if (w.y > 0 && !move_table(w, &bars[0], KTHR)) break;
+                    }
+                    convert_tile<BITS, D, KTHR, KM == PM_WINDOW ? PM_STEP : KM, !KX>(smem + P::OFF_K + ks * P::KT * P::T_BYTES, smem + dy.pkk + ps * dy.k_stage, rec,
                                                          steptab, sr, ref, mode, tile_n(i), false, (t0 + i) * N, ptid, gsh, grp_shift, zp_off, cm);
                     fence_async_smem();
                     mbar_arrive(&bar_k[ks]);
@@ -880,7 +919,12 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     bool ok = mbar_wait(&bar_pv[ps], (i / PST) & 1, abort_flag, 23);
                     if (ok && i >= VST) ok = mbar_wait(&bar_o[vs], ((i - VST) / VST) & 1, abort_flag, 24);    // V stage is free
                     if (!ok) break;
-                    convert_tile<BITS, D, VTHR, VM, false>(smem + P::OFF_V + vs * P::T_BYTES, smem + dy.pkv + ps * dy.v_stage, smem + dy.vrec + ps * dy.vrec_stage,
+                    const unsigned char* rec = smem + dy.vrec + ps * dy.vrec_stage;
+                    if constexpr (VM == PM_WINDOW) {
+                        const int2 w = *reinterpret_cast<const int2*>(rec + N * 2);
+                        if (w.y > 0 && !move_table(w, &bars[1], VTHR)) break;
+                    }
+                    convert_tile<BITS, D, VTHR, VM == PM_WINDOW ? PM_STEP : VM, false>(smem + P::OFF_V + vs * P::T_BYTES, smem + dy.pkv + ps * dy.v_stage, rec,
                                                            steptab, sr, ref, mode, tile_n(i), true, (t0 + i) * N, ptid, gsh, grp_shift, zp_off, cm);
                     fence_async_smem();
                     mbar_arrive(&bar_v[vs]);
@@ -971,6 +1015,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         }
     } else {
         // =============================================================== load warps
+        const bool k = warp == P::LOAD_WARP;
         // Tile i goes into the packed stage of tile i - PST once the converters have arrived on that tile's operand barrier.  The table
         // slot of tile i was last read by the softmax of tile i - TS: K(i - PST) converted means S(i - PST - KST) is complete, which was
         // issued after P(i - PST - KST - SB), and TS exceeds that distance (V is converted later still).
@@ -981,7 +1026,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
         const int32_t* vbase = a.vc + b * a.vs_b + h * a.vs_h;
         // one lane: the packed rows of tile i and, where they are contiguous, its raw grouped parameters.  Returns whether the other
         // lanes have to fetch the grouped parameters themselves (a ragged last tile, unaligned tables).
-        auto copy = [&](bool k, int i) {
+        auto copy = [&](int i) {
             const int ps = i % PST, n = tile_n(i);
             uint64_t* bar = k ? &bar_pk[ps] : &bar_pv[ps];
             const uint32_t bytes = (uint32_t)n * (k ? a.wk : a.wv) * 4;
@@ -1022,9 +1067,24 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 zp[u] = pv.zp ? __ldg(pv.zp + pi) : 0.f;
             }
         };
+        // Step record of a tile: the table slots of its keys, then the steps that the converters bring into the table first: (first, count), count
+        // 0 where all are there.  The table moves on to the tile's first step and all that fit behind it.  For a tile of many steps it
+        // stays where it is: keys of steps outside it get the slot of the fp32 routine.
+        const ParamView& my = k ? a.kp : a.vp;
+        const int tab_rows = k ? dy.k_rows : dy.v_rows;
+        int2 win = (k ? KM : VM) == PM_WINDOW ? first_steps(my, tab_rows) : make_int2(0, 0);
+        auto step_record = [&](unsigned char* rec, const float (&row)[2]) {
+            const int r[2] = {__float_as_int(row[0]), __float_as_int(row[1])};
+            const int lo = __reduce_min_sync(0xffffffffu, min(r[0], r[1])), hi = __reduce_max_sync(0xffffffffu, max(r[0], r[1]));
+            const bool move = (lo < win.x || hi >= win.y) && hi - lo < min(tab_rows, STEPS_TO_MOVE);
+            if (move) win = make_int2(lo, min(lo + tab_rows, max(my.n_rows, hi + 1)));
+#pragma unroll
+            for (int u = 0; u < 2; ++u) reinterpret_cast<uint16_t*>(rec)[lane + 32 * u] = (uint16_t)(r[u] >= win.x && r[u] < win.y ? r[u] - win.x : tab_rows);
+            if (lane == 0) *reinterpret_cast<int2*>(rec + N * 2) = make_int2(win.x, move ? win.y - win.x : 0);
+        };
         auto load_k = [&](int i) {
             const int ps = i % PST;
-            if (lane == 0) copy(true, i);
+            if (lane == 0) copy(i);
             float* tab = reinterpret_cast<float*>(smem + P::OFF_TAB) + (i % TS) * P::TAB_FLOATS;
             // ---- K records (and tables)
             unsigned char* krec = smem + dy.krec + ps * dy.krec_stage;
@@ -1046,16 +1106,18 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             } else if constexpr (KM == PM_STEP) {
 #pragma unroll
                 for (int u = 0; u < 2; ++u) reinterpret_cast<uint16_t*>(krec)[lane + 32 * u] = (uint16_t)__float_as_int(ks_[u]);
+            } else if constexpr (KM == PM_WINDOW) {
+                step_record(krec, ks_);
             } else {
                 if (dy.k_mode == PM_GROUP) raw_params(a.kp, k_par, kng, dy.k_bulk != 0, i, reinterpret_cast<float*>(krec));
             }
             mbar_arrive(&bar_pk[ps]);
             if (P::TAB) mbar_arrive(&bar_t[i % TS]);
-            if (KM != PM_GROUP && i + 1 < T) fetch(a.kp, k_par, KM == PM_STEP, i + 1, ks_, kz_);
+            if (KM != PM_GROUP && i + 1 < T) fetch(a.kp, k_par, per_step(KM), i + 1, ks_, kz_);
         };
         auto load_v = [&](int i) {
             const int ps = i % PST;
-            if (lane == 0) copy(false, i);
+            if (lane == 0) copy(i);
             float* tab = reinterpret_cast<float*>(smem + P::OFF_TAB) + (i % TS) * P::TAB_FLOATS;
             // ---- V records (and tables)
             unsigned char* vrec = smem + dy.vrec + ps * dy.vrec_stage;
@@ -1073,16 +1135,17 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             } else if constexpr (VM == PM_STEP) {
 #pragma unroll
                 for (int u = 0; u < 2; ++u) reinterpret_cast<uint16_t*>(vrec)[lane + 32 * u] = (uint16_t)__float_as_int(vs_[u]);
+            } else if constexpr (VM == PM_WINDOW) {
+                step_record(vrec, vs_);
             } else {
                 if (dy.v_mode == PM_GROUP) raw_params(a.vp, v_par, vng, dy.v_bulk != 0, i, reinterpret_cast<float*>(vrec));
             }
             mbar_arrive(&bar_pv[ps]);
             if (P::TAB) mbar_arrive(&bar_t[i % TS]);
-            if (VM != PM_GROUP && i + 1 < T) fetch(a.vp, v_par, VM == PM_STEP, i + 1, vs_, vz_);
+            if (VM != PM_GROUP && i + 1 < T) fetch(a.vp, v_par, per_step(VM), i + 1, vs_, vz_);
         };
-        const bool k = warp == P::LOAD_WARP;
-        if (k) { if (KM != PM_GROUP) fetch(a.kp, k_par, KM == PM_STEP, 0, ks_, kz_); }
-        else if (VM != PM_GROUP) fetch(a.vp, v_par, VM == PM_STEP, 0, vs_, vz_);
+        if (k) { if (KM != PM_GROUP) fetch(a.kp, k_par, per_step(KM), 0, ks_, kz_); }
+        else if (VM != PM_GROUP) fetch(a.vp, v_par, per_step(VM), 0, vs_, vz_);
         int i = 0;
         bool ok = true;
 #pragma unroll 1
@@ -1113,8 +1176,8 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
 // smem layout of a launch, parameter modes, launch of one instantiation
 template <int D, int NQ, int QT, int KM, int VM> int tc_launch_one(const AttnArgs& a, TcDyn dy, int kb, int vb, cudaStream_t st) {
     using P = TcPlan<D, NQ, QT, KM, VM>;
-    constexpr int STEP_BYTES = 3 * D * 2;
-    auto rec_bytes = [](int mode, int ng) { return mode == PM_GROUP ? TC_N * ng * 8 : mode == PM_EXACT ? TC_N * 4 : mode == PM_STEP ? TC_N * 2 : 16; };
+    auto tab_bytes = [](int mode, int rows) { return mode == PM_STEP ? rows * 3 * D * 2 : mode == PM_WINDOW ? (rows + 1) * 3 * D * 2 : 0; };
+    auto rec_bytes = [](int mode, int ng) { return mode == PM_GROUP ? TC_N * ng * 8 : mode == PM_EXACT ? TC_N * 4 : mode == PM_STEP ? TC_N * 2 : mode == PM_WINDOW ? TC_N * 2 + 16 : 16; };
     dy.k_stage = TC_N * a.wk * 4; dy.v_stage = TC_N * a.wv * 4;
     dy.krec_stage = rec_bytes(dy.k_mode, D / a.kp.group); dy.vrec_stage = rec_bytes(dy.v_mode, D / a.vp.group);
     dy.pkk = P::OFF_DYN;
@@ -1122,8 +1185,8 @@ template <int D, int NQ, int QT, int KM, int VM> int tc_launch_one(const AttnArg
     dy.krec = dy.pkv + P::PST * dy.v_stage;
     dy.vrec = dy.krec + P::PST * dy.krec_stage;
     dy.ktab = dy.vrec + P::PST * dy.vrec_stage;
-    dy.vtab = dy.ktab + (KM == PM_STEP ? a.kp.n_rows * STEP_BYTES : 0);
-    const size_t smem = (size_t)dy.vtab + (VM == PM_STEP ? a.vp.n_rows * STEP_BYTES : 0) + 1024;     // slack for the 1024-byte alignment of the swizzled tiles
+    dy.vtab = dy.ktab + tab_bytes(KM, dy.k_rows);
+    const size_t smem = (size_t)dy.vtab + tab_bytes(VM, dy.v_rows) + 1024;     // slack for the 1024-byte alignment of the swizzled tiles
     if (smem > 227 * 1024) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: %zu bytes of shared memory", smem);
     static bool configured[64] = {false};    // per device; the attribute is sticky, set it outside any stream capture
     int dev = 0;
@@ -1142,6 +1205,9 @@ template <int D, int NQ, int QT> int tc_launch_modes(const AttnArgs& a, const Tc
     VARQ_TC_GO(PM_EXACT, PM_EXACT); VARQ_TC_GO(PM_EXACT, PM_GROUP); VARQ_TC_GO(PM_EXACT, PM_STEP);
     VARQ_TC_GO(PM_GROUP, PM_EXACT); VARQ_TC_GO(PM_GROUP, PM_GROUP); VARQ_TC_GO(PM_GROUP, PM_STEP);
     VARQ_TC_GO(PM_STEP, PM_EXACT); VARQ_TC_GO(PM_STEP, PM_GROUP); VARQ_TC_GO(PM_STEP, PM_STEP);
+    if constexpr (NQ == 2 && QT == 1) {
+        VARQ_TC_GO(PM_EXACT, PM_WINDOW); VARQ_TC_GO(PM_GROUP, PM_WINDOW); VARQ_TC_GO(PM_WINDOW, PM_EXACT); VARQ_TC_GO(PM_WINDOW, PM_GROUP); VARQ_TC_GO(PM_WINDOW, PM_WINDOW);
+    }
 #undef VARQ_TC_GO
     return fail(VARQ_ERR_ARG, "varq_attn_fwd: parameter mode");
 }
