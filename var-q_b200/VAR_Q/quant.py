@@ -313,7 +313,8 @@ class VAR_Q(_host.Cache if _host is not None else _Unbuilt):
             self._quantize_into(item, self._codes, self._scale_tbl, self._zp_tbl, self._n_tokens, self._n_rows, stats)
             if share_l:
                 self._row_of_token[self._n_tokens:self._n_tokens + n] = self._n_rows
-                self._row_begin[self._n_rows + 1:self._n_rows + 2].fill_(self._n_tokens + n)   # entry n_rows already holds n_tokens
+                self._row_begin[self._n_rows:self._n_rows + 1].fill_(self._n_tokens)
+                self._row_begin[self._n_rows + 1:self._n_rows + 2].fill_(self._n_tokens + n)
             self._pending = (n, rows, False)
         self._pack_meta = meta
 
