@@ -59,11 +59,12 @@ typedef struct {
  * row_of_token[token] when that table is given (modes whose parameters are constant
  * over the tokens of one appended step keep one row per step).
  * zp == NULL means symmetric quantization.
- * row_begin (optional, only read together with row_of_token): row_begin[r] is the first token of row r and
- * row_begin[n_rows] the number of tokens described, i.e. the inverse of row_of_token for rows that cover
- * consecutive tokens (one row per appended step).  Attention uses it to cut its key tiles at step boundaries,
- * which lets per-dim scales that are constant over a step be folded into the queries; without it such
- * groupings are dequantised element by element. */
+ * n_rows (only read together with row_of_token): rows 0 .. n_rows - 1 exist; 0 if their number is not known.  Attention
+ * keeps the rows of per-dim groupings in shared memory: all of them when n_rows says that they fit, otherwise a
+ * part that moves along with the keys.
+ * row_begin: row_begin[r] is the first token of row r and row_begin[n_rows] the number of tokens described, i.e. the
+ * inverse of row_of_token for rows that cover consecutive tokens (one row per appended step).  Part of a cache's
+ * tables (varq_append maintains it); no kernel reads it, and it may be NULL here. */
 typedef struct {
     float*         scale;
     float*         zp;

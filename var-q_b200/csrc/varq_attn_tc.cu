@@ -103,6 +103,8 @@ int attn_tc_run(const AttnArgs& a0, int kb, int vb, void* ws, size_t ws_bytes, c
     TcDyn dy = {};
     dy.k_mode = par_mode(a.kp, a.D);
     dy.v_mode = par_mode(a.vp, a.D);
+    for (ParamView* pv : {&a.kp, &a.vp})
+        if (pv->n_rows > a.Lk) pv->n_rows = 0;         // more rows than keys: read those that the keys name
     step_tables(a, dy);
     const bool window = dy.k_mode == PM_WINDOW || dy.v_mode == PM_WINDOW;
     const int qt = window ? 1 : tc_query_tiles(a.Lq, a.D), rows = qt * TC_M;       // (fewer rows of partials than the workspace is sized for)
