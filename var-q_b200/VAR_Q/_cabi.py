@@ -131,24 +131,10 @@ def tensor_desc(ptr: int, dtype_code: int, sb: int, sl: int, sh: int) -> Tensor:
     return Tensor(ptr, dtype_code, 0, sb, sl, sh)
 
 
-_workspaces = {}
-
-
 def workspace(device, nbytes: int) -> torch.Tensor:
-    """Scratch buffer of the current stream on `device`; it only grows.
-
-    Kernels on one stream are ordered and may share scratch; kernels on two streams may overlap, so
-    every stream gets its own buffer.  A buffer that is outgrown goes back to torch's caching
-    allocator, which reuses a block only in the order of the stream it was allocated on.
-    """
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        with torch.cuda.device(index):
-            buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+    """Scratch of one call on the current stream of `device`.  From torch's caching allocator, which reuses a block only in the order of
+    the stream it was allocated on, and keeps what a captured call used for the lifetime of the graph."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 ATTN_PATHS = {None: 0, "auto": 0, "small": 1, "stream": 2, "tc": 3, "mid": 4, "decode": 5}

@@ -17,9 +17,6 @@
 #include <torch/csrc/DynamicTypes.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <list>
-#include <mutex>
-
 #include "varq_b200.h"
 
 namespace {
@@ -57,28 +54,14 @@ PyObject* raise(int rc) {
     return nullptr;
 }
 
-// Scratch of a (device, stream): grows, at most 16 are kept (the least recently used goes back to the caching allocator, which reuses
-// a block only in the order of its stream).
-struct Scratch { int dev; cudaStream_t st; at::Tensor buf; };
-std::list<Scratch> scratch_pool;
-std::mutex scratch_lock;
 at::Tensor empty(at::IntArrayRef shape, at::ScalarType s, c10::DeviceIndex dev) {
     return at::detail::empty_cuda(shape, s, c10::Device(c10::kCUDA, dev), c10::nullopt);
 }
-void* scratch(const c10::cuda::CUDAStream& st, size_t bytes) {
-    std::lock_guard<std::mutex> guard(scratch_lock);
-    auto it = scratch_pool.begin();
-    while (it != scratch_pool.end() && !(it->dev == st.device_index() && it->st == st.stream())) ++it;
-    if (it == scratch_pool.end()) {
-        if (scratch_pool.size() >= 16) scratch_pool.pop_back();
-        scratch_pool.push_front({st.device_index(), st.stream(), at::Tensor()});
-    } else if (it != scratch_pool.begin()) {
-        scratch_pool.splice(scratch_pool.begin(), scratch_pool, it);
-    }
-    at::Tensor& buf = scratch_pool.front().buf;
-    if (!buf.defined() || (size_t)buf.numel() < bytes) buf = empty({(long long)std::max(bytes, (size_t)1 << 16)}, at::kByte, st.device_index());
-    return buf.data_ptr();
-}
+// Scratch of one call, from the caching allocator on the current stream: it goes back when the call returns and is reused in the order of
+// that stream, and what a captured call used belongs to the graph's pool for the graph's lifetime.  (A buffer kept between calls would have to
+// outlive every graph that holds its address, and would be shared by a replay and by calls on the stream that it was captured on.)
+at::Tensor scratch(size_t bytes, c10::DeviceIndex dev) { return bytes ? empty({(long long)bytes}, at::kByte, dev) : at::Tensor(); }
+void* scratch_ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 // (B, L, H, D) strides of a 4-D tensor in the cache's item layout; false if the call does not handle it
 bool view4(const at::Tensor& x, bool bhlc, varq_tensor_t& d, long long& B, long long& L, long long& H, long long& D) {
@@ -205,11 +188,13 @@ int append_n(Cache** c, const at::Tensor** x, int n, float norm_eps, bool commit
         fill_job(c[i], d[i], jobs[i]);
     }
     size_t ws = varq_append_workspace_bytes(jobs, n, (int)B, (int)L, (int)H, (int)D, norm_eps);
-    int rc = varq_append(jobs, n, (int)B, (int)L, (int)H, (int)D, norm_eps, ws ? scratch(st, ws) : nullptr, ws, st.stream());
+    at::Tensor buf = scratch(ws, dev);
+    int rc = varq_append(jobs, n, (int)B, (int)L, (int)H, (int)D, norm_eps, scratch_ptr(buf), ws, st.stream());
     if (rc == VARQ_ERR_UNSUPPORTED && norm_eps >= 0.f) return 0;
     if (rc == VARQ_ERR_WORKSPACE) {
         for (int i = 0; i < n; ++i) ws = std::max(ws, varq_quant_workspace_bytes((int)B, (int)L, (int)H, (int)D, jobs[i].x.dtype, jobs[i].store_bits, &jobs[i].p));
-        rc = varq_append(jobs, n, (int)B, (int)L, (int)H, (int)D, norm_eps, scratch(st, ws), ws, st.stream());
+        buf = scratch(ws, dev);
+        rc = varq_append(jobs, n, (int)B, (int)L, (int)H, (int)D, norm_eps, scratch_ptr(buf), ws, st.stream());
     }
     if (rc != VARQ_OK) { raise(rc); return -1; }
     for (int i = 0; i < n; ++i) { set_pending(c[i], L); if (commit_too) commit(c[i]); }
@@ -250,7 +235,8 @@ PyObject* attend_impl(const at::Tensor& q, Cache* k, Cache* v, double scale, PyO
     cache_desc(v, vc, vp);
     const long long Lk = k->n_tokens;
     const size_t ws = varq_attn_workspace_bytes((int)B, (int)H, (int)Lq, (int)Lk, (int)D, store_bits(k), store_bits(v));
-    void* wp = ws ? scratch(st, ws) : nullptr;
+    const at::Tensor buf = scratch(ws, dev);
+    void* const wp = scratch_ptr(buf);
     int rc;
     if (norm)
         rc = varq_attn_fwd_qnorm(&qd, &kc, &vc, &kp, &vp, (int)B, (int)H, (int)Lq, (int)Lk, (int)D, store_bits(k), store_bits(v), (float)scale,
