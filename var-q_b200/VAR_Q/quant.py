@@ -24,6 +24,7 @@ Known deviations, both deliberate: ``G_TENSOR`` replaces the cache after re-quan
 duplicates tokens); ``qkv_format`` may be re-assigned after construction and takes effect
 (in the reference the derived dims go stale, VAR_Q/quant.py:75-95).
 """
+import os
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -32,7 +33,11 @@ from . import _cabi
 
 try:
     from . import _host                 # native state and call path (csrc_host/)
-except ImportError:                     # not built yet: construction and configuration work, device calls say what is missing
+except ImportError as e:
+    # Nothing is built: construction and configuration work, device calls say what is missing.  With the library in place the host path
+    # has to load, too (it links against the torch it was built with): without it every step would quietly take its slow Python form.
+    if os.path.exists(_cabi.LIB_PATH):
+        raise ImportError(f"VAR_Q/_host.so is missing or does not load ({e}): build it with `python var-q_b200/build.py --force`") from e
     _host = None
 
 _METHODS = ('G_TENSOR', 'G_SCALE_HEAD_DIM', 'G_HEAD_DIM', 'G_SCALE', 'G_TOKEN', 'G_TOKEN_HEAD')
