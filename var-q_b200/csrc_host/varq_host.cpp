@@ -243,14 +243,6 @@ PyObject* attend_impl(const at::Tensor& q, Cache* k, Cache* v, double scale, PyO
                                  mul ? mul->data_ptr<float>() : nullptr, (float)eps, &od, wp, ws, st.stream());
     else
         rc = varq_attn_fwd(&qd, &kc, &vc, &kp, &vp, (int)B, (int)H, (int)Lq, (int)Lk, (int)D, store_bits(k), store_bits(v), (float)scale, &od, wp, ws, st.stream());
-    if (norm && rc == VARQ_ERR_UNSUPPORTED) {       // no kernel normalises this call's queries: do it here
-        at::Tensor qf = q.to(at::kFloat);
-        qf = qf / at::linalg_vector_norm(qf, 2, at::IntArrayRef({-1}), true).clamp_min(eps);
-        if (mul) qf = qf * (k->bhlc ? mul->view({1, H, 1, 1}) : mul->view({1, 1, H, 1}));
-        const at::Tensor qc = qf.contiguous();
-        PyObject* dt = out_dtype != Py_None ? out_dtype : reinterpret_cast<PyObject*>(torch::getTHPDtype(at::kFloat));
-        return attend_impl(qc, k, v, scale, dt, false, nullptr, 0.0);
-    }
     if (rc != VARQ_OK) return raise(rc);
     return THPVariable_Wrap(out);
 }
