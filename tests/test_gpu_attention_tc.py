@@ -54,7 +54,7 @@ def test_bit_widths(D, kb, vb, symmetric):
     kq, vq, kd, vd = make("BHLc", 2, 3, (1, 4, 9, 16, 25, 36, 64, 100, 169, 256), D, kb, vb, seed=kb * 10 + vb, symmetric=symmetric)
     q = torch.randn((2, 3, 256, D), generator=torch.Generator().manual_seed(D + kb))
     out, launches = run("tc", q.to(DEV), kq, vq, 1.0 / D ** 0.5)
-    assert launches == 2          # per-key parameter preparation + the attention kernel
+    assert launches == 2          # six (sample, head) pairs: the key range is split, the second launch merges the parts
     check(out, O.attention(q, kd, vd, "BHLc", 1.0 / D ** 0.5).transpose(1, 2), f"D={D} k{kb} v{vb} sym={symmetric}")
 
 
@@ -132,7 +132,7 @@ def test_full_size_last_scale_is_linear_in_v_and_permutation_invariant():
 ])
 @pytest.mark.parametrize("kb,vb", [(8, 8), (4, 2)])
 def test_groupings_whose_k_scale_varies_along_head_dim(D, q_dtype, kkw, vkw, kb, vb):
-    """Per-dim and group-wise K: the kernel dequantises K into hi + lo fp16 tiles (two MMAs)."""
+    """Per-dim and group-wise K: the kernel dequantises K into hi + lo fp16 tiles (two score products, three with fp32 queries)."""
     fmt, B, H = "BLHc", 2, 3
     steps = (1, 4, 9, 16, 25, 36, 64, 100, 169)
     kkw, vkw = dict(kkw), dict(vkw)
@@ -147,7 +147,7 @@ def test_groupings_whose_k_scale_varies_along_head_dim(D, q_dtype, kkw, vkw, kb,
     q = torch.randn((B, 169, H, D), generator=torch.Generator().manual_seed(D + kb)).to(q_dtype)
     scale = 1.0 / D ** 0.5
     out, launches = run("tc", q.to(DEV), kq, vq, scale)
-    assert launches == 2          # per-key (or per-step) parameter preparation + the attention kernel
+    assert launches == 2          # the attention kernel on a split key range, and the merge
     check(out, O.attention(q, kd, vd, fmt, scale), f"D={D} {q_dtype} K{kkw} V{vkw} {kb}/{vb}")
 
 
@@ -177,8 +177,8 @@ def test_all_zero_and_tiny_value_tokens_keep_their_attention_weight(D, symmetric
 
 @pytest.mark.parametrize("D,kb,vb", [(64, 8, 8), (128, 4, 4)])
 def test_per_dim_scales_over_a_long_history_of_steps(D, kb, vb):
-    """More appended steps than the step tables of the dequantising mode hold (64): per-dim K scales are then folded
-    into the queries step by step, with key tiles cut at the step boundaries (one launch, no preparation)."""
+    """More appended steps of K and V than the step tables hold (66 at head_dim 64, 18 at 128): the tables move along with the key
+    tiles, still in one launch (too few tiles here for a split key range)."""
     fmt, B, H = "BLHc", 1, 2
     steps = (1, 2, 3) * 22 + (40, 130)          # 68 steps, 302 tokens
     kq, vq = VAR_Q(kb, fmt, "G_SCALE_HEAD_DIM", symmetric=False), VAR_Q(vb, fmt, "G_SCALE_HEAD_DIM")
@@ -202,7 +202,7 @@ def test_per_dim_scales_over_a_long_history_of_steps(D, kb, vb):
 ])
 def test_parameters_outside_the_packed_half_converters_bounds(D, kkw, vkw):
     """K values far from zero with a narrow range give zero-points below -512; V scaled up gives scales above 60: the
-    preparation kernel flags such tiles and the converters take their fp32 routine (first step only: the second one is
+    converters find such parameters and take their fp32 routine (first step only: the second one is
     ordinary data, so flagged and unflagged tiles alternate inside one launch where the parameters are per key)."""
     fmt, B, H = "BLHc", 2, 2
     kkw, vkw = dict(kkw), dict(vkw)
@@ -229,8 +229,8 @@ def test_parameters_outside_the_packed_half_converters_bounds(D, kkw, vkw):
 
 
 def test_tensor_core_path_refuses_a_missing_workspace():
-    """The preparation streams live in the caller's workspace: without one the call fails with VARQ_ERR_WORKSPACE and
-    launches nothing."""
+    """Partial rows of a split key range go through the caller's workspace, which is asked for whether the range is split or not:
+    without one the call fails with VARQ_ERR_WORKSPACE and launches nothing."""
     fmt, B, H, D, lq, lk = "BLHc", 1, 2, 64, 40, 100
     kq, vq = VAR_Q(8, fmt, "G_TOKEN_HEAD"), VAR_Q(8, fmt, "G_TOKEN_HEAD")
     kq.append(torch.randn(B, lk, H, D, device=DEV)); vq.append(torch.randn(B, lk, H, D, device=DEV))
