@@ -347,10 +347,10 @@ def kernel_rooflines(device, peaks):
     ph8 = (8, "G_TOKEN_HEAD", {})
     for bits in (8, 4, 2):
         a = (bits, "G_TOKEN_HEAD", {})
-        attn_case(f"attention, streaming CUDA-core kernel (per-head INT{bits})", 64, 16, 128, 1, 10521, a, a, torch.bfloat16)
+        attn_case(f"attention, few-query tensor-core kernel (per-head INT{bits})", 64, 16, 128, 1, 10521, a, a, torch.bfloat16)
     g32 = lambda b: (b, "G_TOKEN_HEAD", dict(symmetric=False, group_size=32))
     attn_case("attention, streaming CUDA-core kernel (group-32 INT4 K / INT2 V)", 64, 16, 128, 1, 10521, g32(4), g32(2), torch.bfloat16)
-    attn_case("attention, streaming CUDA-core kernel, 16 queries (per-head INT8)", 64, 16, 128, 16, 10521, ph8, ph8, torch.bfloat16)
+    attn_case("attention, few-query tensor-core kernel, 16 queries (per-head INT8)", 64, 16, 128, 16, 10521, ph8, ph8, torch.bfloat16)
     attn_case("attention, warp-level tensor-core kernel for the early scales (per-head INT8)", 64, 16, 64, 25, 55, ph8, ph8, torch.float32, fmt="BLHc", reps=20)
     attn_case("attention, tensor-core kernel, exact-code K (per-head INT8)", 64, 16, 64, 256, 680, ph8, ph8, torch.float32, fmt="BLHc", reps=20)
     attn_case("attention, tensor-core kernel, exact-code K (per-head INT8)", 64, 16, 64, 1024, 2240, ph8, ph8, torch.bfloat16, fmt="BLHc")
@@ -515,17 +515,19 @@ def load_traffic(kernel_key, launch_bytes):
     """DRAM bytes of one launch of the dominant kernel, from the ncu capture recorded in profiles/ncu_traffic.json: the
     capture ran a smaller case of the same kernel and settings (the full launch is too large to capture), so its DRAM
     bytes are scaled by the ratio of the algorithmic bytes of the two launches.  Valid only while the kernel's source
-    file is the one the capture was taken on."""
+    files are those the capture was taken on."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if not os.path.exists(path):
         return None, "no ncu capture recorded"
     rec = json.load(open(path)).get(kernel_key)
     if not rec:
         return None, f"no ncu capture recorded for {kernel_key}"
-    src = os.path.join(ROOT, rec["source"])
-    sha = hashlib.sha256(open(src, "rb").read()).hexdigest()[:16] if os.path.exists(src) else None
-    if sha != rec["source_sha256_16"]:
-        return None, f"the ncu capture in {rec['summary']} predates the current {rec['source']}"
+    paths = [os.path.join(ROOT, p) for p in rec["sources"]]
+    digest = hashlib.sha256()
+    for p in paths:
+        digest.update(open(p, "rb").read() if os.path.exists(p) else b"")
+    if digest.hexdigest()[:16] != rec["sources_sha256_16"]:
+        return None, f"the ncu capture in {rec['summary']} predates the current {', '.join(rec['sources'])}"
     ratio = rec["dram_bytes"] / rec["algorithmic_bytes_of_capture"]
     return int(ratio * launch_bytes), (f"ncu capture of a smaller launch ({rec['capture']}; {rec['dram_bytes']} DRAM bytes for "
                                        f"{rec['algorithmic_bytes_of_capture']} algorithmic bytes, summary in {rec['summary']}), scaled by algorithmic bytes")
@@ -711,7 +713,7 @@ def run_ours(args):
         if kind == "attn":
             roof = roof_entry(f"attn[scale {si}: l={lq}, cached={lk}]", w["desc"].split(":")[0], top_ms, peaks,
                               nbytes=attn_bytes(w, b2, lq, lk), flops=attn_flops(w, b2, lq, lk), kernels=top_launches)
-            key = "attn_tc_kernel" if lq > 16 else "attn_stream_kernel"
+            key = "attn_tc_kernel" if lq > 16 else "attn_decode_kernel"
         else:
             bits, mode, kw = w["k"] if kind == "quant_k" else w["v"]
             n_el = b2 * lq * w["heads"] * w["head_dim"]
@@ -853,7 +855,7 @@ def run_reference(args):
 
 # --------------------------------------------------------------------------- single-kernel cases (what ncu captures)
 def run_case(name):
-    """One kernel on a small, larger-than-L2 case, a few launches: the command the ncu summaries under profiles/ cite."""
+    """One kernel on a small, larger-than-L2 case (or one layer), a few launches: the command the ncu summaries under profiles/ cite."""
     from VAR_Q.attention import attend_cached
     from VAR_Q.quant import VAR_Q
     dev = torch.device("cuda", 0)
@@ -883,18 +885,26 @@ def run_case(name):
         qshape = (B, lq, H, D) if fmt == "BLHc" else (B, H, lq, D)
         q = torch.nn.functional.normalize(torch.randn(qshape, generator=g, device=dev), dim=-1) * Q_GAIN
         fn = lambda: attend_cached(q, kq, vq, 1.0, out_dtype=torch.bfloat16)
-    elif name == "stream":    # one query per (sample, head) over 10 521 packed tokens, INT4 K and V, head_dim 128: 1.4 GB of codes
-        B, H, D, lk = 64, 16, 128, 10521
-        kq, vq = VAR_Q(4, "BHLc", "G_TOKEN_HEAD", max_tokens=lk), VAR_Q(4, "BHLc", "G_TOKEN_HEAD", max_tokens=lk)
+    elif name in ("decode", "stream"):     # one query per (sample, head) over 10 521 packed tokens, head_dim 128: INT4 per head / INT4 and INT2 in groups of 32
+        B, H, D, lk = 16, 16, 128, 10521
+        ka, va = (4, {}), (4, {})
+        if name == "stream":
+            ka, va = (4, dict(symmetric=False, group_size=32)), (2, dict(symmetric=False, group_size=32))
+        kq, vq = (VAR_Q(b, "BHLc", "G_TOKEN_HEAD", max_tokens=lk, **kw) for b, kw in (ka, va))
         kq.append(torch.nn.functional.normalize(torch.randn((B, H, lk, D), generator=g, device=dev), dim=-1))
         vq.append(torch.randn((B, H, lk, D), generator=g, device=dev).to(torch.bfloat16))
         q = (torch.nn.functional.normalize(torch.randn((B, H, 1, D), generator=g, device=dev), dim=-1) * Q_GAIN).to(torch.bfloat16)
         fn = lambda: attend_cached(q, kq, vq, 1.0, out_dtype=torch.bfloat16)
-        nbytes = 2 * B * H * lk * D // 2
-    else:                     # "quant": 252 MB of fp32 K, per-head INT8, batch-shared groups; "quant2": per-dim groups (two passes)
+        nbytes = B * H * lk * D * (ka[0] + va[0]) // 8
+    elif name.startswith("layer_"):        # one attention layer of a workload, every scale: what the launch lists show
+        w = dict(WORKLOADS[name[len("layer_"):]], depth=1)
+        inputs = make_inputs(w, dev, seed=1)
+        fn = lambda: hot_path_step(w, inputs)
+    else:                     # "quant": 252 MB of fp32 K, per-head INT8, batch-shared groups; "quant2": per-dim groups (two passes); "dequant": back to fp32
         x = torch.randn((128, 256, 30, 64), generator=g, device=dev)
-        qz = VAR_Q(8, "BLHc", "G_TOKEN_HEAD" if name == "quant" else "G_SCALE_HEAD_DIM", max_tokens=256)
-        fn = lambda: qz.quant(x)
+        qz = VAR_Q(8, "BLHc", "G_SCALE_HEAD_DIM" if name == "quant2" else "G_TOKEN_HEAD", max_tokens=256)
+        qz.quant(x)
+        fn = qz.dequant_current if name == "dequant" else lambda: qz.quant(x)
         nbytes = x.numel() * 5
     for _ in range(3):
         fn()
@@ -917,7 +927,8 @@ def main():
     ap.add_argument("--no-sweep", action="store_true", help="skip the isolated dequant-attention sweep")
     ap.add_argument("--quick", action="store_true", help="headline measurement only (no per-kernel rooflines, sweep, other workloads, CPU leg)")
     ap.add_argument("--no-graph", action="store_true", help="launch every kernel from Python instead of replaying a CUDA graph")
-    ap.add_argument("--case", choices=("attn", "attn_early", "attn_perdim", "attn_group", "stream", "quant", "quant2"),
+    ap.add_argument("--case", choices=("attn", "attn_early", "attn_perdim", "attn_group", "decode", "stream", "quant", "quant2", "dequant") +
+                    tuple("layer_" + n for n in sorted(WORKLOADS)),
                     help="run one kernel on a small case and exit (profiling aid)")
     args = ap.parse_args()
     if args.case:

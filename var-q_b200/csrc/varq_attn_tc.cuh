@@ -16,10 +16,17 @@
 //   load warps one for K, one for V: a lane requests packed rows (and the raw scales of grouped parameters) up to three tiles ahead by
 //              1-D bulk copies; all lanes fetch per-key parameters one tile ahead into registers and write them as records and
 //              softmax tables.
-// The kernel is bound by instruction issue (softmax 4 x ~300 and conversion ~50 warp instructions per 16 codes of 64 keys), so more
-// than 128 queries share each converted tile (QT = 2, head_dim 64, all 512 TMEM columns); up to 128 queries run as two CTAs per
-// SM of 256 columns each, one CTA's set-up and dependent waits under the other's tiles.  At head_dim 128 the tensor pipe
-// is the closer bound (hi + lo operands: 4 products of 256 cycles per tile): one CTA keeps three or four score tiles in flight.
+// More than 128 queries share each converted tile (QT = 2, head_dim 64, all 512 TMEM columns); up to 128 queries run as two CTAs per SM of
+// 256 columns each, one CTA's set-up and dependent waits under the other's tiles.  At head_dim 128 one CTA keeps three or four score
+// tiles in flight.
+// What bounds it, from builds in which one role skips its arithmetic (us a call: all / no conversion / no softmax / one score product):
+//   c 64   B64 H16 256 x 10521, int2 group 32, bf16 queries      1306 / 1340 /  724 / 1271
+//          B64 H16 256 x 680, int8 per head, fp32 queries         182 /  179 /  103 /  175
+//          B32 H30 1024 x 2240, int4, K per dim, fp32 queries    1426 / 1546 /  851 / 1410
+//   c 128  B4 H16 4096 x 10521, int4 and int2 group 32, fp32     2395 / 2412 / 2221 / 2335     (neither conversion nor softmax: 1814)
+//          B6 H16 1600 x 6000, int8 per dim, fp32                1040 /  936 /  953 /  962     (neither: 730)
+// At head_dim 64 the softmax warps, two per sub-partition, each a serial chain of score load, exponentials and P store.  At 128 no role by
+// itself: conversion and softmax share the issue slots, the tensor pipe is behind both (hi + lo operands, 4 products of 256 cycles a tile).
 // Few CTAs over a long cache: the key range is split across CTAs and a second kernel merges the partial rows.
 // Numerics: integer codes are exact in fp16; an fp32 query is split into hi + lo fp16 halves, a dequantised K likewise (the lo x lo
 // product is below fp32 resolution), so S has fp32-like accuracy; P and a dequantised V are rounded to fp16 once; sums are fp32.
@@ -212,7 +219,7 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     // accumulator in tensor memory, and meet in the epilogue, so the two warps of a sub-partition hide each other's latencies (score loads,
     // barriers).  Else each takes half of every tile's keys and they agree on one reference: with two query operands (hi + lo) the second
     // accumulator would leave room for two score tiles only, and the chain score product -> softmax -> output product then binds (B8 H16
-    // Lq2048 Lk4096 int4, us: one operand 985 -> 814, two operands 1028 -> 1131, so those stay; dequantised K is bound by its converters, 1035 -> 1032).
+    // Lq2048 Lk4096 int4, us: one operand 985 -> 814, two operands 1028 -> 1131, so those stay; dequantised K, 1035 -> 1032, is not bound by its softmax warps alone).
     static constexpr bool ALT = D == 128 && NQ == 1 && KX;
     static constexpr int KW = D == 128 ? (ALT ? 4 : 8) : 2 * QT, VW = D == 128 ? 4 : 2 * QT;
     static constexpr int KTHR = KW * 32, VTHR = VW * 32;
