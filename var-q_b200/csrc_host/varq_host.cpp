@@ -1,8 +1,8 @@
 // Host path of the package as a CPython extension over ATen: cache state, append, attention and dequantisation calls.
 //
 // A step of an attention layer is three calls of the C ABI on small operands; written in Python (descriptors through ctypes, device
-// context managers, tensor allocations) it cost about 75 us per step, several times the kernels of the early scales.  Here it is one
-// call per step (about 10 us): the quantizers' state lives in a C++ object (the base class of VAR_Q.quant.VAR_Q), descriptors are
+// context managers, tensor allocations) it cost about 72 us per step, several times the kernels of the early scales.  Here it is one
+// call per step (about 9 us): the quantizers' state lives in a C++ object (the base class of VAR_Q.quant.VAR_Q), descriptors are
 // filled in place and tensors come straight from the caching allocator.  Every function declines (returns None / False) what it does
 // not handle -- unusual dtypes and layouts, the whole-cache modes after their first step, anything erroneous -- and the Python code
 // next to it takes over, so that errors and rare modes have one implementation.
