@@ -516,7 +516,8 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
     uint64_t* bar_q = bars + 21;      // queries in tensor memory
     uint64_t* bar_end = bars + 22;    // all products complete
     uint64_t* bar_kf = bars + 24;     // [KST] every product that reads a K stage complete
-    uint64_t* bar_sf = bars + 28;     // [SB] O += P V complete: the score columns are free (head_dim 128, where another warp issues S)
+    uint64_t* bar_sf = bars + 28;     // [SB] O += P V complete: the score columns are free (head_dim 128, where another warp issues S); QT = 2: [QT][2], the same
+                                      // per query tile, for the softmax threads
     uint64_t* bar_t = bars + 38;      // [TS] softmax tables of tile i in place (slot i % TS)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + P::OFF_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + P::OFF_MISC + 4);
@@ -742,7 +743,10 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     m_used = m_new;
                     l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
                     if (i >= STEP) {
-                        ok = ok && mbar_wait(&bar_o[(i - STEP) % VST], ((i - STEP) / VST) & 1, abort_flag, 13);      // the accumulator is stable
+                        // The accumulator is stable.  With two query tiles bar_o waits for both, and the other may be so far behind that the parity
+                        // of an earlier phase answers: each has barriers of its own.
+                        const int o = i - STEP;
+                        ok = ok && (QT == 2 ? mbar_wait(&bar_sf[2 * t + (o & 1)], (o >> 1) & 1, abort_flag, 13) : mbar_wait(&bar_o[o % VST], (o / VST) & 1, abort_flag, 13));
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) continue;
                         {
@@ -986,6 +990,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             }
             tc_commit(&bar_o[i % VST]);
             if (ROLES) tc_commit(&bar_sf[i % SB]);
+            else if (QT == 2) tc_commit(&bar_sf[2 * t + (i & 1)]);
         };
         if (t < n_qt && (mw == 0 || QT == 2 || ROLES)) {
             bool ok = mbar_wait_warp(bar_q, 0, abort_flag, 30);
