@@ -453,9 +453,10 @@ __device__ __forceinline__ void convert_tile(unsigned char* tile, const unsigned
 }
 
 // ---- softmax arithmetic
-// A row keeps its reference maximum until a score exceeds it by more than this (log2 units): P stays below
-// 2^12 in fp16 and the accumulators are rescaled rarely.
-constexpr float TC_LAZY = 12.f;
+// A row keeps its reference until the weights of a tile add up to more than this: P stays below it in fp16 (largest finite value 65504)
+// and the accumulators are rescaled rarely.
+constexpr float TC_SUM_MAX = 32768.f;
+constexpr float TC_LAZY = 12.f;       // the same for a maximum (log2 units)
 constexpr float TC_VS_MIN = 9.5367431640625e-07f;     // 2^-20: smallest V scale folded into P as is
 constexpr float TC_MASKED = -1e30f;
 // |softmax scale| * log2(e) multiplies the scores; below this (a zero scale among them) it goes into the queries instead, so that
@@ -658,87 +659,70 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 if constexpr (KX) qsum = pair_sum(qsum);
             }
             const float c = tc_factor(a.scale_log2);
-            float m_used = -FLT_MAX;                            // reference maximum (log2 domain): with ALT the thread's own, else the same in both threads of a row
+            float m_used = -FLT_MAX;                            // reference (log2 domain): with ALT the thread's own, else the same in both threads of a row
             float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;       // row sum of this thread's softmax weights
             bool ok = true;
             const int first_col = ALT ? 0 : half * NC;          // of the tile's score columns
             const uint32_t col_acc = lane_base + col_o + (ALT ? half * D : 0);
             constexpr int STEP = ALT ? 2 : 1;
+            // scores and tables of a tile in place?  Asked for the next tile while P of this one is on its way: the answer takes 130 cycles
+            auto tile_ready = [&](int i) -> bool {
+                const bool r = mbar_test(&bar_s[t * SB + i % SB], (i / SB) & 1);
+                return P::TAB ? mbar_test(&bar_t[i % TS], (i / TS) & 1) && r : r;
+            };
+            bool ready = false;
+            bool behind = true;        // the reference has to follow this tile's scores before its P is computed
             // Once a wait has expired nothing is read or written any more, but a pair's barriers are still taken: without ALT both warps
             // run all iterations.
 #pragma unroll 1
-            for (int i = ALT ? half : 0; i < T; i += STEP) {
+            for (int i = ALT ? half : 0; i < T;) {
                 const int s = i % SB;
-                ok = ok && mbar_wait_warp(&bar_s[t * SB + s], (i / SB) & 1, abort_flag, 11);
-                if (P::TAB) ok = ok && mbar_wait_warp(&bar_t[i % TS], (i / TS) & 1, abort_flag, 12);
+                if (!__all_sync(0xffffffffu, ready)) {
+                    ok = ok && mbar_wait_warp(&bar_s[t * SB + s], (i / SB) & 1, abort_flag, 11);
+                    if (P::TAB) ok = ok && mbar_wait_warp(&bar_t[i % TS], (i / TS) & 1, abort_flag, 12);
+                    if (!ok) {
+                        if (HV == 1 || ALT) break;
+                        if (behind) pair_sync();
+                        const bool again = !behind && pair_any(false);
+                        behind = again;
+                        if (!again) i += STEP;
+                        continue;
+                    }
+                }
                 const uint32_t s_addr = lane_base + col_s + s * N;
                 const float* tab = reinterpret_cast<const float*>(smem + P::OFF_TAB) + (i % TS) * P::TAB_FLOATS + first_col;
-                if (!ok) {
-                    if (HV == 1 || ALT) break;
-                    if (pair_any(false)) pair_sync();
-                    continue;
+                uint32_t x[NC], ph[NC / 2];
+                const int nv = tile_n(i) - first_col;
+                const bool wide = KX && __float_as_int(tab[4 * N - first_col]) != 0;        // a zero-point of this tile is too wide for the exact operand: its term in fp32
+                tc_fence_after();
+                tmem_ld32(s_addr + first_col, x);
+                if constexpr (NC == 64) tmem_ld32(s_addr + 32, x + 32);
+                tmem_wait_ld();
+                if (wide || nv < NC) {          // and columns past the cache (the last tile) hold anything
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) {
+                        if (wide) x[j] = __float_as_uint(fmaf(-tab[3 * N + j], qsum, __uint_as_float(x[j])));
+                        if (j >= nv) x[j] = __float_as_uint(TC_MASKED);
+                    }
                 }
-                uint32_t x[NC];
-                float mx;
-                {
-                    tc_fence_after();
-                    tmem_ld32(s_addr + first_col, x);
-                    if constexpr (NC == 64) tmem_ld32(s_addr + 32, x + 32);
-                    tmem_wait_ld();
-                    // ---- scores in the log2 domain with the V scale folded in (tables), or raw (their factor c enters with the exponential)
-                    if constexpr (KX || VX) {
+                const bool settled = behind;       // (both threads of a row have read their scores before either stores P over them: here and where they vote below)
+                if (behind) {
+                    // The first tile, and where some row of these warps meets scores far above its reference: the tile's maximum becomes the
+                    // reference and what has been accumulated is rescaled (a factor 1 for the other rows).
+                    float mt = -FLT_MAX;
 #pragma unroll
-                        for (int j = 0; j < NC; j += 4) {
-                            const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c);
-                            float y[4];
-                            if constexpr (VX) {
-                                const float4 b4 = tab4(tab + N + j);
-                                fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), k4.x, k4.y, b4.x, b4.y);
-                                fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), k4.z, k4.w, b4.z, b4.w);
-                            } else {
-                                mul2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), k4.x, k4.y);
-                                mul2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), k4.z, k4.w);
-                            }
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) x[j + e] = __float_as_uint(y[e]);
-                        }
-                        if (KX && __float_as_int(tab[4 * N - first_col]) != 0) {        // a zero-point of this tile is too wide for the exact operand: its term in fp32
-#pragma unroll
-                            for (int j = 0; j < NC; j += 4) {
-                                const float4 z4 = tab4(tab + 3 * N + j);
-                                x[j] = __float_as_uint(fmaf(-z4.x, qsum, __uint_as_float(x[j])));
-                                x[j + 1] = __float_as_uint(fmaf(-z4.y, qsum, __uint_as_float(x[j + 1])));
-                                x[j + 2] = __float_as_uint(fmaf(-z4.z, qsum, __uint_as_float(x[j + 2])));
-                                x[j + 3] = __float_as_uint(fmaf(-z4.w, qsum, __uint_as_float(x[j + 3])));
-                            }
-                        }
+                    for (int j = 0; j < NC; j += 4) {
+                        const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c), b4 = VX ? tab4(tab + N + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        mt = max3(mt, fmaf(__uint_as_float(x[j]), k4.x, b4.x), fmaf(__uint_as_float(x[j + 1]), k4.y, b4.y));
+                        mt = max3(mt, fmaf(__uint_as_float(x[j + 2]), k4.z, b4.z), fmaf(__uint_as_float(x[j + 3]), k4.w, b4.w));
                     }
-                    const int nv = tile_n(i) - first_col;
-                    if (nv < NC) {                                  // the last tile: columns past the cache hold anything
-#pragma unroll
-                        for (int j = 0; j < NC; ++j) if (j >= nv) x[j] = __float_as_uint(TC_MASKED);
-                    }
-                    float ma = -FLT_MAX, mb = -FLT_MAX, mc = -FLT_MAX, md = -FLT_MAX;
-#pragma unroll
-                    for (int j = 0; j < NC; j += 8) {
-                        ma = max3(ma, __uint_as_float(x[j]), __uint_as_float(x[j + 1]));
-                        mb = max3(mb, __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]));
-                        mc = max3(mc, __uint_as_float(x[j + 4]), __uint_as_float(x[j + 5]));
-                        md = max3(md, __uint_as_float(x[j + 6]), __uint_as_float(x[j + 7]));
-                    }
-                    mx = fmaxf(max3(ma, mb, mc), md);
-                    if constexpr (!KX && !VX) mx *= c;
-                }
-                float mt = mx;
-                if (pair_any(mt > m_used + TC_LAZY)) {
-                    // Rare after the first tile: some row of these warps meets a score more than 2^12 above its reference.  Its maximum
-                    // becomes the reference and what has been accumulated is rescaled (a factor 1 for the other rows).
                     if (HV == 2 && !ALT) {
                         xch[half * XH] = mt;
                         pair_sync();
                         mt = fmaxf(mt, xch[(half ^ 1) * XH]);
                     }
-                    const float m_new = mt > m_used + TC_LAZY ? mt : m_used;
+                    behind = false;
+                    const float m_new = fmaxf(mt, m_used);
                     const float alpha = ex2(m_used - m_new);    // 0 for a row without a reference yet
                     m_used = m_new;
                     l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
@@ -748,58 +732,96 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                         const int o = i - STEP;
                         ok = ok && (QT == 2 ? mbar_wait(&bar_sf[2 * t + (o & 1)], (o >> 1) & 1, abort_flag, 13) : mbar_wait(&bar_o[o % VST], (o / VST) & 1, abort_flag, 13));
                         ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) continue;
-                        {
-                            tc_fence_after();
+                        if (!ok) { ready = false; i += STEP; continue; }
+                        tc_fence_after();
 #pragma unroll 1
-                            for (int c0 = ALT ? 0 : half * DH; c0 < (ALT ? D : (half + 1) * DH); c0 += 16) {
-                                uint32_t o[16];
-                                tmem_ld16(col_acc + c0, o);
-                                tmem_wait_ld();
+                        for (int c0 = ALT ? 0 : half * DH; c0 < (ALT ? D : (half + 1) * DH); c0 += 16) {
+                            uint32_t o[16];
+                            tmem_ld16(col_acc + c0, o);
+                            tmem_wait_ld();
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-                                tmem_st16(col_acc + c0, o);
-                            }
-                            tmem_wait_st();
+                            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+                            tmem_st16(col_acc + c0, o);
                         }
+                        tmem_wait_st();
                     }
                 }
-                {
-                    // ---- P = 2^(x - m), fp16 pairs over the score columns 
-                    const float nm = -m_used;
-                    uint32_t ph[NC / 2];
+                // ---- P = 2^(score - reference), with the V scale where V keeps exact codes: fp16 pairs.  The row sum adds up the rounded P
+                // that multiplies V, so that a row dominated by one key stays exact.
+                const float nm = -m_used;
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+                auto to_half = [&](int j, const float (&y)[4]) {
+                    const __half2 h01 = __floats2half2_rn(ex2(y[0]), ex2(y[1])), h23 = __floats2half2_rn(ex2(y[2]), ex2(y[3]));
+                    ph[j / 2] = *reinterpret_cast<const uint32_t*>(&h01);
+                    ph[j / 2 + 1] = *reinterpret_cast<const uint32_t*>(&h23);
+                };
+                auto sum_up = [&](int j) {
+                    if constexpr (VX) {       // P carries the V scale: the softmax weight is P / V scale
+                        const float4 v4 = tab4(tab + 2 * N + j);
+                        const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&ph[j / 2])), f23 = __half22float2(*reinterpret_cast<const __half2*>(&ph[j / 2 + 1]));
+                        fma2(s0, s1, f01.x, f01.y, v4.x, v4.y, s0, s1);
+                        fma2(s2, s3, f23.x, f23.y, v4.z, v4.w, s2, s3);
+                    } else {
+                        add_halves(s0, s1, ph[j / 2]);
+                        add_halves(s2, s3, ph[j / 2 + 1]);
+                    }
+                };
+                if constexpr (ALT) {
+                    // The maximum first and the sum behind the store of P: two warps of a sub-partition on tiles of different age fill each
+                    // other's gaps already (B8 H16 Lq2048 Lk4096 int8, bf16 queries: 872 us, 937 us as the block below).  Nothing of it may move up
+                    // into the waits for the scores (910 us).
+                    asm volatile("" ::: "memory");
+                    float ma = -FLT_MAX, mb = -FLT_MAX;
+#pragma unroll
+                    for (int j = 0; j < NC; j += 4) {
+                        const float4 k4 = tab4(tab + j), b4 = VX ? tab4(tab + N + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        float y[4];
+                        fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), k4.x, k4.y, b4.x, b4.y);
+                        fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), k4.z, k4.w, b4.z, b4.w);
+                        ma = max3(ma, y[0], y[1]);
+                        mb = max3(mb, y[2], y[3]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[j + e] = __float_as_uint(y[e]);
+                    }
+                    if (!settled && __any_sync(0xffffffffu, fmaxf(ma, mb) > m_used + TC_LAZY)) { ready = behind = true; continue; }
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) {
                         float y[4];
-                        if constexpr (KX || VX) {
-                            add2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), nm, nm);
-                            add2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), nm, nm);
-                        } else {
-                            fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), c, c, nm, nm);
-                            fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), c, c, nm, nm);
-                        }
-                        const __half2 h01 = __floats2half2_rn(ex2(y[0]), ex2(y[1])), h23 = __floats2half2_rn(ex2(y[2]), ex2(y[3]));
-                        ph[j / 2] = *reinterpret_cast<const uint32_t*>(&h01);
-                        ph[j / 2 + 1] = *reinterpret_cast<const uint32_t*>(&h23);
+                        add2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), nm, nm);
+                        add2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), nm, nm);
+                        to_half(j, y);
                     }
-                    if constexpr (NC == 64) tmem_st32(s_addr, ph); else tmem_st16(s_addr + half * 16, *reinterpret_cast<uint32_t (*)[16]>(ph));
-                    // the row sum adds up the rounded P that multiplies V: a row dominated by one key stays exact
+                    tmem_st32(s_addr, ph);
+#pragma unroll
+                    for (int j = 0; j < NC; j += 4) sum_up(j);
+                } else {
+                    // One block of straight code: the exponential unit takes most of it, everything else fits in between
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) {
-                        if constexpr (VX) {       // P carries the V scale: the softmax weight is P / V scale
-                            const float4 v4 = tab4(tab + 2 * N + j);
-                            const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&ph[j / 2])), f23 = __half22float2(*reinterpret_cast<const __half2*>(&ph[j / 2 + 1]));
-                            fma2(l0, l1, f01.x, f01.y, v4.x, v4.y, l0, l1);
-                            fma2(l2, l3, f23.x, f23.y, v4.z, v4.w, l2, l3);
-                        } else {
-                            add_halves(l0, l1, ph[j / 2]);
-                            add_halves(l2, l3, ph[j / 2 + 1]);
+                        const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c);
+                        float b0 = nm, b1 = nm, b2 = nm, b3 = nm, y[4];
+                        if constexpr (VX) {
+                            const float4 b4 = tab4(tab + N + j);
+                            add2(b0, b1, b4.x, b4.y, nm, nm);
+                            add2(b2, b3, b4.z, b4.w, nm, nm);
                         }
+                        fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), k4.x, k4.y, b0, b1);
+                        fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), k4.z, k4.w, b2, b3);
+                        to_half(j, y);
+                        sum_up(j);
                     }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(&bar_p[t * SB + s]);
+                    // P has room up to 65504: the sum of the tile's weights shows that none came close, without their maximum
+                    const float limit = VX ? tab[4 * N + 1 - first_col] : TC_SUM_MAX;
+                    const bool high = !((s0 + s1) + (s2 + s3) <= limit);
+                    if (!settled && pair_any(high)) { ready = behind = true; continue; }
+                    if constexpr (NC == 64) tmem_st32(s_addr, ph); else tmem_st16(s_addr + half * 16, *reinterpret_cast<uint32_t (*)[16]>(ph));
                 }
+                l0 += s0; l1 += s1; l2 += s2; l3 += s3;
+                i += STEP;
+                ready = !ALT && i < T && tile_ready(i);       // (ALT: the next tile of a warp is seldom there yet)
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(&bar_p[t * SB + s]);
             }
             // ---- output row: each thread writes half of its head_dim
             // (ALT) the accumulators of the two threads meet: f0 and f1 bring tiles of even and odd index to the common reference (0 where
@@ -1095,7 +1117,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             if (lane == 0) *reinterpret_cast<int2*>(rec + N * 2) = make_int2(win.x, move ? win.y - win.x : 0);
         };
         auto load_k = [&](int i) {
-            const int ps = i % PST;
+            const int ps = i % PST, n = tile_n(i);
             if (lane == 0) copy(i);
             float* tab = reinterpret_cast<float*>(smem + P::OFF_TAB) + (i % TS) * P::TAB_FLOATS;
             // ---- K records (and tables)
@@ -1107,10 +1129,9 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 for (int u = 0; u < 2; ++u) {
                     const int key = lane + 32 * u;
                     const bool w = !(fabsf(kz_[u]) <= 512.f);       // code - zp is not exact in fp16: its term goes to the scores in fp32
-                    const float s = ks_[u] * c;
                     reinterpret_cast<uint32_t*>(krec)[key] = half_pair(kbase0 - (w ? 0.f : kz_[u]));
-                    tab[key] = s;
-                    tab[3 * N + key] = w ? kz_[u] * s : 0.f;
+                    tab[key] = key < n ? ks_[u] * c : 1.f;          // a masked score stays masked
+                    tab[3 * N + key] = w ? kz_[u] : 0.f;
                     wide = wide || w;
                 }
                 wide = __any_sync(0xffffffffu, wide);
@@ -1134,6 +1155,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             // ---- V records (and tables)
             unsigned char* vrec = smem + dy.vrec + ps * dy.vrec_stage;
             if constexpr (VM == PM_EXACT) {
+                float least = FLT_MAX;          // of the weights' factors: P = weight / factor stays below TC_SUM_MAX while their sum is below that times this
                 const float vbase0 = vb == 8 ? Item<8>::neg_base(0) : vb == 4 ? Item<4>::neg_base(0) : Item<2>::neg_base(0);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
@@ -1142,8 +1164,12 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     const float s = w ? 1.f : fmaxf(vs_[u], TC_VS_MIN);
                     reinterpret_cast<uint32_t*>(vrec)[key] = w ? PAR_SLOW : half_pair(vbase0 - vz_[u]);
                     tab[N + key] = __log2f(s);
-                    tab[2 * N + key] = __frcp_rn(s);
+                    const float r = __frcp_rn(s);
+                    tab[2 * N + key] = r;
+                    least = fminf(least, r);
                 }
+                least = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(least)));
+                if (lane == 0) tab[4 * N + 1] = TC_SUM_MAX * least;
             } else if constexpr (VM == PM_STEP) {
 #pragma unroll
                 for (int u = 0; u < 2; ++u) reinterpret_cast<uint16_t*>(vrec)[lane + 32 * u] = (uint16_t)__float_as_int(vs_[u]);
