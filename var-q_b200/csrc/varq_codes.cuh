@@ -25,6 +25,10 @@ __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
 __host__ __device__ constexpr int code_at(int bits, int p) {
     return bits == 8 ? p : bits == 4 ? ((p & 8) | ((p & 1) << 2) | ((p & 7) >> 1)) : (((p & 1) << 3) | (p >> 1));
 }
+// and the operand position of head_dim index e
+__host__ __device__ constexpr int code_pos(int bits, int e) {
+    return bits == 8 ? e : bits == 4 ? ((e & 8) | ((e & 3) << 1) | ((e >> 2) & 1)) : (((e & 7) << 1) | (e >> 3));
+}
 __host__ __device__ constexpr int code_bias(int bits) { return bits == 8 ? 128 : bits == 4 ? 8 : 2; }
 // The constants of the pairs as register values that the compiler cannot fold: (x & mask) ^ magic is one three-input logic instruction with
 // the mask as its immediate only if the magic is in a register; with two known constants it became two instructions per pair, and
