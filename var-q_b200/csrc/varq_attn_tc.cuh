@@ -323,11 +323,16 @@ template <bool SPLIT>
 __device__ __forceinline__ void scale_pair(uint32_t& d, uint32_t& lo, uint32_t sh, uint32_t sl) {
     if constexpr (SPLIT) {
         const uint32_t hi = h2_mul(d, sh);
-        lo = h2_fma(d, sl, h2_fma(d, sh, hi ^ 0x80008000u));
+        lo = h2_fma(d, sl, h2_fma(d, sh, h2_neg(hi)));
         d = hi;
     } else {
         d = h2_fma(d, sh, h2_mul(d, sl));
     }
+}
+template <int N> __device__ __forceinline__ void load_words(const uint32_t* p, uint32_t* w) {
+    if constexpr (N == 4) { const uint4 v = *reinterpret_cast<const uint4*>(p); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
+    else if constexpr (N == 2) { const uint2 v = *reinterpret_cast<const uint2*>(p); w[0] = v.x; w[1] = v.y; }
+    else w[0] = *p;
 }
 // The per-dim parameters of a thread's 16-wide head_dim slice, kept in registers while consecutive keys belong to one step
 struct StepRegs { uint32_t sh[8], sl[8], nz[8]; int step; };
@@ -366,97 +371,107 @@ __device__ __forceinline__ void fill_steps(unsigned char* steptab, const ParamRe
     }
 }
 
-// One operand tile by NTHR threads.  SPLIT: hi + lo tiles (K), otherwise one tile.  Neighbouring lanes take the items of one
-// key: contiguous reads, and a quarter-warp's 16-byte stores land in eight different bank groups.  A thread keeps its head_dim slice
-// and its place inside the swizzled rows (NTHR is a multiple of 8 keys' items), so its addresses advance by constants, and its
-// packed words are all loaded before the first is used.  Rows past the keys are computed from whatever the stage holds; `zero`
-// clears them (V: their P is zero, but 0 * NaN is not).
+// One operand tile by NTHR threads.  SPLIT: hi + lo tiles (K), otherwise one tile.  A thread keeps its head_dim slice and its place inside the
+// swizzled rows (NTHR is a multiple of 8 keys' items), so its addresses advance by constants, and its packed words are all loaded before
+// the first is used.  Rows past the keys are computed from whatever the stage holds; `zero` clears them (V: their P is zero, but 0 * NaN is not).
+// An item is 16 codes of a key; with grouped parameters of narrow codes it is 32, which share a scale where the group has that many (the
+// preparation of a scale is a third of a 16-code item's instructions).  Neighbouring lanes take the items of one key: contiguous reads, and
+// a quarter-warp's 16-byte stores land in eight different bank groups; 32-code items do so when it takes two items of four keys.
 template <int BITS, int D, int NTHR, int MODE, bool SPLIT>
 __device__ __forceinline__ void convert_tile(unsigned char* tile, const unsigned char* packed, const unsigned char* rec, const unsigned char* steptab, StepRegs& sr,
                                              const ParamRef* ref, int mode, int n_valid, bool zero, int k0, int ptid, int gsh, int grp_shift, int zp_off, const CodeMagic<BITS>& cm) {
-    constexpr int IPK = D / 16, NW = BITS / 2, NIT = TC_N * IPK / NTHR, KSTEP = NTHR / IPK;
+    constexpr int W = MODE == PM_GROUP && BITS < 8 ? 2 : 1;
+    constexpr int IPK = D / (16 * W), NW = BITS / 2, NIT = TC_N * IPK / NTHR, KSTEP = NTHR / IPK;
     constexpr int LO = SPLIT ? TC_N * D * 2 : 0;
+    constexpr int STEP_BYTES = KSTEP * 128;      // KSTEP keys further in the tile
     static_assert(TC_N * IPK % NTHR == 0 && KSTEP % 8 == 0, "items of a tile over the threads");
-    const int item = ptid & (IPK - 1), d0 = item * 16, key0 = ptid / IPK;
-    unsigned char* dst0 = tile + chunk_off(key0, 2 * item);
-    unsigned char* dst1 = tile + chunk_off(key0, 2 * item + 1);
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(packed) + ptid * NW;
-    uint32_t slow = 0;                       // items to redo in fp32
+    const int item = W == 2 && IPK == 4 ? (ptid & 1) | (ptid >> 2 & 2) : ptid & (IPK - 1);
+    const int key0 = W == 2 && IPK == 4 ? (ptid >> 1 & 3) | (ptid >> 2 & 4) | (ptid >> 5) * 8 : ptid / IPK, d0 = item * 16 * W;
+    const uint32_t off0 = chunk_off(key0, 2 * W * item);
+    auto dst = [&](int it, int ch) -> unsigned char* { return tile + (off0 ^ (uint32_t)(ch << 4)) + it * STEP_BYTES; };
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(packed) + (key0 * IPK + item) * (W * NW);
+    uint32_t slow = 0;                       // 16-code slices to redo in fp32
     if (MODE == PM_GROUP && mode == PM_SLOW) {
-        slow = (1u << NIT) - 1u;
+        slow = (1u << (NIT * W)) - 1u;
     } else {
-        uint32_t w[NIT][NW];
+        uint32_t w[NIT][W * NW];
 #pragma unroll
-        for (int it = 0; it < NIT; ++it) Item<BITS>::load(src + it * NTHR * NW, w[it]);
+        for (int it = 0; it < NIT; ++it) load_words<W * NW>(src + it * NTHR * (W * NW), w[it]);
 #pragma unroll
         for (int it = 0; it < NIT; ++it) {
             const int key = key0 + it * KSTEP;
-            uint32_t d[8], lo[8];
-            Item<BITS>::raw(w[it], d, cm);
-            if constexpr (MODE == PM_STEP) {
-                const int step = reinterpret_cast<const uint16_t*>(rec)[key];        // its slot in the table
-                if (step != sr.step) {
-                    const uint4* t = reinterpret_cast<const uint4*>(steptab + (step * 3 * D + d0) * 2);
-                    constexpr int TD = D * 2 / 16;      // uint4 per table row
+            uint32_t sh = 0, sl = 0, nz[Item<BITS>::CLS];
+            bool out = false;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const uint4 a = t[i], b = t[TD + i], c = t[2 * TD + i];
-                        sr.sh[4 * i] = a.x; sr.sh[4 * i + 1] = a.y; sr.sh[4 * i + 2] = a.z; sr.sh[4 * i + 3] = a.w;
-                        sr.sl[4 * i] = b.x; sr.sl[4 * i + 1] = b.y; sr.sl[4 * i + 2] = b.z; sr.sl[4 * i + 3] = b.w;
-                        sr.nz[4 * i] = c.x; sr.nz[4 * i + 1] = c.y; sr.nz[4 * i + 2] = c.z; sr.nz[4 * i + 3] = c.w;
+            for (int u = 0; u < W; ++u) {
+                uint32_t d[8], lo[8];
+                Item<BITS>::raw(w[it] + u * NW, d, cm);
+                if constexpr (MODE == PM_STEP) {
+                    const int step = reinterpret_cast<const uint16_t*>(rec)[key];        // its slot in the table
+                    if (step != sr.step) {
+                        const uint4* t = reinterpret_cast<const uint4*>(steptab + (step * 3 * D + d0) * 2);
+                        constexpr int TD = D * 2 / 16;      // uint4 per table row
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint4 a = t[i], b = t[TD + i], c = t[2 * TD + i];
+                            sr.sh[4 * i] = a.x; sr.sh[4 * i + 1] = a.y; sr.sh[4 * i + 2] = a.z; sr.sh[4 * i + 3] = a.w;
+                            sr.sl[4 * i] = b.x; sr.sl[4 * i + 1] = b.y; sr.sl[4 * i + 2] = b.z; sr.sl[4 * i + 3] = b.w;
+                            sr.nz[4 * i] = c.x; sr.nz[4 * i + 1] = c.y; sr.nz[4 * i + 2] = c.z; sr.nz[4 * i + 3] = c.w;
+                        }
+                        sr.step = step;
                     }
-                    sr.step = step;
-                }
-                if (sr.nz[0] == PAR_SLOW) slow |= 1u << it;
+                    if (sr.nz[0] == PAR_SLOW) slow |= 1u << it;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    d[i] = Item<BITS>::minus_zp(d[i], i, sr.nz[i]);
-                    scale_pair<SPLIT>(d[i], lo[i], sr.sh[i], sr.sl[i]);
-                }
-            } else if constexpr (MODE == PM_GROUP) {
-                const float* par = reinterpret_cast<const float*>(rec) + (key << gsh) + (d0 >> grp_shift);
-                const float s = par[0], z = zp_off ? par[zp_off] : 0.f;
-                if (!par_in_bounds(s, z)) slow |= 1u << it;
-                const __half s_hi = __float2half_rn(s);
-                const uint32_t sh = (uint32_t)__half_as_ushort(s_hi) * 0x10001u, sl = half_pair(s - __half2float(s_hi));
-                uint32_t nz[Item<BITS>::CLS];
-                Item<BITS>::spread(half_pair(Item<BITS>::neg_base(0) - z), nz);
+                    for (int i = 0; i < 8; ++i) {
+                        d[i] = Item<BITS>::minus_zp(d[i], i, sr.nz[i]);
+                        scale_pair<SPLIT>(d[i], lo[i], sr.sh[i], sr.sl[i]);
+                    }
+                } else if constexpr (MODE == PM_GROUP) {
+                    if (u == 0 || grp_shift == 4) {
+                        const float* par = reinterpret_cast<const float*>(rec) + (key << gsh) + ((d0 + 16 * u) >> grp_shift);
+                        const float s = par[0], z = zp_off ? par[zp_off] : 0.f;
+                        out = !par_in_bounds(s, z);
+                        const __half s_hi = __float2half_rn(s);
+                        sh = (uint32_t)__half_as_ushort(s_hi) * 0x10001u;
+                        sl = half_pair(s - __half2float(s_hi));
+                        Item<BITS>::spread(half_pair(Item<BITS>::neg_base(0) - z), nz);
+                    }
+                    if (out) slow |= 1u << (it * W + u);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    d[i] = Item<BITS>::minus_zp(d[i], i, nz[i % Item<BITS>::CLS]);
-                    scale_pair<SPLIT>(d[i], lo[i], sh, sl);
-                }
-            } else {
-                const uint32_t nz0 = reinterpret_cast<const uint32_t*>(rec)[key];
-                if (nz0 == PAR_SLOW) slow |= 1u << it;
-                uint32_t nz[Item<BITS>::CLS];
-                Item<BITS>::spread(nz0, nz);
+                    for (int i = 0; i < 8; ++i) {
+                        d[i] = Item<BITS>::minus_zp(d[i], i, nz[i % Item<BITS>::CLS]);
+                        scale_pair<SPLIT>(d[i], lo[i], sh, sl);
+                    }
+                } else {
+                    const uint32_t nz0 = reinterpret_cast<const uint32_t*>(rec)[key];
+                    if (nz0 == PAR_SLOW) slow |= 1u << it;
+                    Item<BITS>::spread(nz0, nz);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) d[i] = Item<BITS>::minus_zp(d[i], i, nz[i % Item<BITS>::CLS]);
-            }
-            constexpr int STEP_BYTES = KSTEP * 128;      // KSTEP keys further in the tile
-            sts128(dst0 + it * STEP_BYTES, d[0], d[1], d[2], d[3]);
-            sts128(dst1 + it * STEP_BYTES, d[4], d[5], d[6], d[7]);
-            if constexpr (SPLIT) {
-                sts128(dst0 + it * STEP_BYTES + LO, lo[0], lo[1], lo[2], lo[3]);
-                sts128(dst1 + it * STEP_BYTES + LO, lo[4], lo[5], lo[6], lo[7]);
+                    for (int i = 0; i < 8; ++i) d[i] = Item<BITS>::minus_zp(d[i], i, nz[i % Item<BITS>::CLS]);
+                }
+                sts128(dst(it, 2 * u), d[0], d[1], d[2], d[3]);
+                sts128(dst(it, 2 * u + 1), d[4], d[5], d[6], d[7]);
+                if constexpr (SPLIT) {
+                    sts128(dst(it, 2 * u) + LO, lo[0], lo[1], lo[2], lo[3]);
+                    sts128(dst(it, 2 * u + 1) + LO, lo[4], lo[5], lo[6], lo[7]);
+                }
             }
         }
     }
     if (slow) {
 #pragma unroll 1
-        for (int it = 0; it < NIT; ++it) {
-            const int key = key0 + it * KSTEP;
-            if ((slow >> it & 1u) && key < n_valid)
-                slow_item<BITS>(dst0 + it * KSTEP * 128, dst1 + it * KSTEP * 128, LO, src + it * NTHR * NW, ref, k0 + key, d0);
+        for (int e = 0; e < NIT * W; ++e) {
+            const int it = e / W, u = e - it * W, key = key0 + it * KSTEP;
+            if ((slow >> e & 1u) && key < n_valid)
+                slow_item<BITS>(dst(it, 2 * u), dst(it, 2 * u + 1), LO, src + it * NTHR * (W * NW) + u * NW, ref, k0 + key, d0 + 16 * u);
         }
     }
     if (zero && n_valid < TC_N) {
 #pragma unroll 1
         for (int it = 0; it < NIT; ++it)
             if (key0 + it * KSTEP >= n_valid) {
-                sts128(dst0 + it * KSTEP * 128, 0u, 0u, 0u, 0u);
-                sts128(dst1 + it * KSTEP * 128, 0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int ch = 0; ch < 2 * W; ++ch) sts128(dst(it, ch), 0u, 0u, 0u, 0u);
             }
     }
 }

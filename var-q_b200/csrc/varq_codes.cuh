@@ -21,6 +21,10 @@ __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
     __half2 r = __hfma2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b), *reinterpret_cast<__half2*>(&c));
     return *reinterpret_cast<uint32_t*>(&r);
 }
+__device__ __forceinline__ uint32_t h2_neg(uint32_t a) {       // an operand modifier of the instruction that takes it
+    __half2 r = __hneg2(*reinterpret_cast<__half2*>(&a));
+    return *reinterpret_cast<uint32_t*>(&r);
+}
 // head_dim index (inside a 16-code item) at operand position p
 __host__ __device__ constexpr int code_at(int bits, int p) {
     return bits == 8 ? p : bits == 4 ? ((p & 8) | ((p & 1) << 2) | ((p & 7) >> 1)) : (((p & 1) << 3) | (p >> 1));
@@ -54,7 +58,7 @@ template <int BITS> struct Item {           // 16 consecutive codes of one key: 
         else w[0] = *p;
     }
     // pairs holding 1024 + 2^p (code + bias)
-    static __device__ __forceinline__ void raw(const uint32_t (&w)[NW], uint32_t (&h)[8], const CodeMagic<BITS>& cm) {
+    static __device__ __forceinline__ void raw(const uint32_t* w, uint32_t (&h)[8], const CodeMagic<BITS>& cm) {
         if constexpr (BITS == 8) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
