@@ -215,7 +215,8 @@ int varq_unpack_dequant(const varq_tensor_t* codes, int32_t B, int32_t L, int32_
 
 /* Pin the kernel varq_attn_fwd uses for every later call of the process: automatic choice, the general
  * CUDA-core kernel, the streaming CUDA-core kernel, the tcgen05 tensor-core kernel, the warp-level tensor-core
- * kernel of the early scales (MID) or that of a few queries over a long cache (DECODE).  A pinned kernel that cannot take a call (shape, layout, grouping) yields to the
+ * kernel of the early scales (MID), that of a few queries over a long cache (DECODE) or the fp32 kernel of the first scales (EARLY).
+ * A pinned kernel that cannot take a call (shape, layout, grouping) yields to the
  * next one in the automatic order and finally to the general kernel.  For tests and measurements that compare the kernels on
  * one input; no counterpart in the reference. */
 #define VARQ_ATTN_PATH_AUTO   0
@@ -224,6 +225,7 @@ int varq_unpack_dequant(const varq_tensor_t* codes, int32_t B, int32_t L, int32_
 #define VARQ_ATTN_PATH_TC     3
 #define VARQ_ATTN_PATH_MID    4
 #define VARQ_ATTN_PATH_DECODE 5
+#define VARQ_ATTN_PATH_EARLY  6
 int varq_attn_force_path(int32_t path);
 
 /* Bytes of scratch varq_attn_fwd needs for this shape, whichever kernel it picks: partial results of the

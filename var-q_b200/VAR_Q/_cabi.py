@@ -137,11 +137,11 @@ def workspace(device, nbytes: int) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
-ATTN_PATHS = {None: 0, "auto": 0, "small": 1, "stream": 2, "tc": 3, "mid": 4, "decode": 5}
+ATTN_PATHS = {None: 0, "auto": 0, "small": 1, "stream": 2, "tc": 3, "mid": 4, "decode": 5, "early": 6}
 
 
 def force_attn_path(name):
-    """Pin the attention kernel for later calls ("small", "stream", "tc", "mid", "decode"; None = automatic).  Test hook."""
+    """Pin the attention kernel for later calls ("small", "stream", "tc", "mid", "decode", "early"; None = automatic).  Test hook."""
     check(lib().varq_attn_force_path(ATTN_PATHS[name]))
 
 

@@ -103,5 +103,7 @@ size_t attn_decode_workspace_bytes(int B, int H, int Lq, int Lk, int D);
 int attn_decode_run(AttnArgs& a, int kb, int vb, void* ws, size_t ws_bytes, cudaStream_t st);
 bool attn_mid_eligible(const AttnArgs& a, int kb, int vb);
 int attn_mid_run(AttnArgs& a, int kb, int vb, cudaStream_t st);
+bool attn_early_eligible(const AttnArgs& a);
+int attn_early_run(AttnArgs& a, int kb, int vb, cudaStream_t st);
 
 }  // namespace varq

@@ -86,6 +86,11 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     if (want_tc && attn_tc_eligible(a, kb, vb)) return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool want_stream = force ? (force == VARQ_ATTN_PATH_STREAM) : small_q;
     if (want_stream && attn_stream_eligible(a, kb, vb)) return attn_stream_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
+    // Parameters that vary inside 16 head_dim values: up to 16 queries over at most 256 tokens have a kernel of their own.  us, general kernel /
+    // early, int8 per dim, 4 / 9 / 16 queries over 5 / 14 / 30 tokens: B2 H16 c64 11.9 / 5.6, 12.5 / 7.0, 13.4 / 9.2; B64 H16 c64 24.8 / 8.4, 62 / 12,
+    // 85 / 17; 16 queries over 256 tokens 283 / 84; c128 B6 H16 20.5 / 8.0 (4), 23.4 / 11.7 (16).  Relative L2 error 1.3e-7 / 1.1e-7.
+    const bool want_early = force ? (force == VARQ_ATTN_PATH_EARLY) : Lq <= 16 && Lk <= 256;
+    if (want_early && attn_early_eligible(a)) return attn_early_run(a, kb, vb, (cudaStream_t)stream);
     return attn_small_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -104,7 +109,7 @@ extern "C" int varq_attn_fwd_qnorm(const varq_tensor_t* q, const varq_tensor_t* 
 }
 
 extern "C" int varq_attn_force_path(int32_t path) {
-    if (path < VARQ_ATTN_PATH_AUTO || path > VARQ_ATTN_PATH_DECODE) return fail(VARQ_ERR_ARG, "varq_attn_force_path: unknown path %d", path);
+    if (path < VARQ_ATTN_PATH_AUTO || path > VARQ_ATTN_PATH_EARLY) return fail(VARQ_ERR_ARG, "varq_attn_force_path: unknown path %d", path);
     __atomic_store_n(&g_forced_path, (int)path, __ATOMIC_RELAXED);
     return VARQ_OK;
 }
