@@ -75,3 +75,21 @@ def test_normalised_queries_and_strided_rows(D):
         qn = q.double() / q.double().norm(dim=-1, keepdim=True).clamp_min(1e-12) * mul.double()
         ref = _reference(qn, kv.k_quant, kv.v_quant, 1.0, "BLHc")
         assert ((out - ref).norm() / ref.norm()).item() <= 2e-6
+
+
+@pytest.mark.parametrize("kw", [dict(quant_bits=8, quant_method="G_TOKEN_HEAD"), dict(quant_bits=4, quant_method="G_TOKEN_HEAD", symmetric=False),
+                                dict(quant_bits=2, quant_method="G_TOKEN")], ids=["int8_head", "int4_head_asym", "int2_token"])
+@pytest.mark.parametrize("heads", [512, 544])
+@pytest.mark.parametrize("lq,lk,fp32", [(9, 14, True), (12, 32, True), (13, 32, False), (12, 33, True), (16, 30, False), (25, 55, False), (33, 60, False)])
+def test_choice_with_one_scale_per_key(kw, heads, lq, lk, fp32):
+    """Both sides of the lines of the automatic choice: fp32-like accuracy wherever the decode or the early kernel takes the call (on 512 pairs
+    decode takes 13 and 16 queries too), fp16 weights elsewhere."""
+    B, H = heads // 16, 16
+    gen = torch.Generator(device=DEV).manual_seed(lq * lk)
+    kq, vq = (_cache(kw, (lk,), "BLHc", B, H, 64, gen, i == 0) for i in range(2))
+    q = torch.randn((B, lq, H, 64), generator=gen, device=DEV)
+    q = q / q.norm(dim=-1, keepdim=True) * 4.0
+    out = attend_cached(q, kq, vq, 0.7, out_dtype=torch.float32).double()
+    ref = _reference(q, kq, vq, 0.7, "BLHc")
+    limit = 2e-6 if fp32 or (lq <= 16 and heads <= 512) else 1e-3
+    assert ((out - ref).norm() / ref.norm()).item() <= limit

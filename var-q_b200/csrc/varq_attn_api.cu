@@ -68,19 +68,31 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     // fp16) the first scales of a per-dim or group-wise cache are 2e-4 away from the exact result, here 2e-7.
     const int force = __atomic_load_n(&g_forced_path, __ATOMIC_RELAXED);
     const bool small_q = Lq <= 4 || (Lq <= 16 && Lk <= 256);
-    // Between the two: tens of queries over at most a few hundred tokens (the early scales of a schedule), where the tcgen05
-    // kernel is bound by its per-CTA set-up; a warp-level tensor-core kernel takes them when the parameters are per key.
-    const bool mid_q = Lq > 8 && Lq <= 64 && Lk <= 256;          // measured against both neighbours (B64 H16 and B128 H30, c 64)
+    // head_dim 64 with one scale per key over at most 256 tokens (the early scales of a schedule), us at H16 (H30 for B128), int8, fp32 queries:
+    //              9 queries over 14 tokens         16 over 30                       25 over 55     36 over 91     64 over 155
+    //     batch    mid / decode / tcgen05 / early   mid / decode / tcgen05 / early   mid / tcgen05  mid / tcgen05  mid / tcgen05
+    //       2     10.0 /   4.3  /   7.1   /  7.4    9.9 /   4.3  /   7.2   / 10.3   10.5 /  7.2    11.6 /  8.0    14.3 /  8.8
+    //      16     10.4 /   7.4  /   8.7   /  8.6   10.7 /   8.3  /   8.8   / 12.3   11.3 /  9.0    14.1 / 10.3    18.9 / 11.7
+    //      32     11.0 /  10.6  /  16.6   / 10.5   11.5 /  12.5  /  16.7   / 14.5   12.9 / 16.9    24.0 / 19.0    32.8 / 21.5
+    //      64     19.5 /  17.6  /  30.6   / 13.5   20.0 /  20.1  /  30.7   / 20.7   22.7 / 30.9    36.4 / 35.8    49.7 / 40.6
+    //     128     48.8 /  58.1  /  96.5   / 41.8   50.8 /  67.8  /  96.9   / 66.8   58.8 / 98.2   139.9 / 115.6  187.8 / 133.9
+    // decode and early keep weights to fp32's accuracy (1e-7 against 2e-4 of the other two).  Up to 512 (sample, head) pairs decode takes 9 to 16 queries;
+    // beyond, early takes up to 12 of them over one chunk of keys, mid the rest, decode again over more keys (16 queries over 256 tokens at B64: mid 43.8,
+    // decode 30.7).  Up to 32 queries mid is the faster of the last two where the tcgen05 kernel needs more than one wave (two CTAs per SM).
+    // mid does not normalise queries: decode or tcgen05 stand in.
+    const long long heads = (long long)B * H;
+    const bool key_scale = D == 64 && kp->group == D && vp->group == D, few = Lq > 8 && Lq <= 16 && Lk <= 256, crowded = heads > 512 && Lk <= 32;
+    if (!force && key_scale && few && crowded && Lq <= 12 && attn_early_eligible(a)) return attn_early_run(a, kb, vb, (cudaStream_t)stream);
     // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key.
     // us at H16, int4, bf16 queries, decode / tcgen05 (the streaming kernel takes 1.8 to 6 times decode's time):
     //     B64 c64   8 x 300: 22 / 47, 16 x 300: 37 / 47, 16 x 2240: 205 / 179, 8 x 10521: 421 / 754, 16 x 10521: 763 / 757
     //     B64 c128  8 x 300: 42 / 75, 16 x 300: 73 / 75, 16 x 2240: 325 / 229, 8 x 10521: 660 / 893, 16 x 10521: 1199 / 902
     //     B2  c128  8 x 300: 10.4 / 10.0, 16 x 2240: 26 / 20, 16 x 10521: 50 / 44;   B2 c64  16 x 2240: 18 / 21, 16 x 10521: 39 / 56
     // Up to 8 queries (one CTA's worth) it is the faster one; from 9 to 16 it takes 0.6 to 1.4 times as long and stays for its
-    // accuracy (3e-7 against 2e-4 for fp16 weights).  It also stands in for the next kernel, which does not normalise.
-    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (q_norm && mid_q && D == 64));
+    // accuracy (3e-7 against 2e-4 for fp16 weights).
+    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (few && D == 64 && (q_norm || !crowded)));
     if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
-    const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : mid_q;
+    const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : few || (Lq > 16 && Lq <= 32 && Lk <= 256 && heads > 2 * sm_count());
     if (want_mid && !q_norm && attn_mid_eligible(a, kb, vb)) return attn_mid_run(a, kb, vb, (cudaStream_t)stream);
     const bool want_tc = force ? (force == VARQ_ATTN_PATH_TC) : !small_q;
     if (want_tc && attn_tc_eligible(a, kb, vb)) return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
