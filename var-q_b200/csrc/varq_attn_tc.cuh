@@ -249,6 +249,9 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr int OFF_PREF = OFF_MISC + 16;            // ParamRef [2]
     static constexpr int OFF_XCH = OFF_PREF + 2 * 48;         // float [4][QT * 128]: the two threads of a row, maxima and sums
     static constexpr int OFF_DYN = OFF_XCH + (HV == 2 ? 4 * QT * TC_M * 4 : 0);   // packed stages, records, step tables: sizes known at launch (TcDyn)
+    static constexpr bool Q_STAGED = NQ == 2;      // queries come in through shared memory:
+    static constexpr int Q_STAGE = 32 * 80;                   // bytes per softmax warp, in the V stages
+    static_assert(K_WARP0 * Q_STAGE <= VST * T_BYTES, "query staging");
     static_assert(OFF_DYN % 16 == 0 && (OFF_TAB % 1024) == 0, "alignment");
     static_assert(QT * SB <= 4 && KST <= 3 && TS > PST + KST + SB, "barrier plan");
     // TMEM columns: queries, output accumulators, score tiles
@@ -521,6 +524,38 @@ template <int N, int AT_LAUNCH> __device__ __forceinline__ void set_registers() 
 }
 template <int V> struct IntC { static constexpr int value = V; };
 
+// 16 bytes of a query row from element `off` on (ES: bytes of an element); rows that do not lie on 16 bytes come element by element
+template <int ES> __device__ __forceinline__ uint4 load_q16(const void* q, long long off) {
+    const uintptr_t addr = reinterpret_cast<uintptr_t>(q) + (unsigned long long)off * ES;
+    if ((addr & 15u) == 0) return __ldg(reinterpret_cast<const uint4*>(addr));
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if constexpr (ES == 4) w[i] = __ldg(reinterpret_cast<const uint32_t*>(addr) + i);
+        else w[i] = (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(addr) + 2 * i) | (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(addr) + 2 * i + 1) << 16;
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// eight elements, as fp32
+template <int ES> __device__ __forceinline__ void q8_floats(const uint4 (&r)[ES / 2], int dtype, float (&v)[8]) {
+    if constexpr (ES == 4) {
+        v[0] = __uint_as_float(r[0].x); v[1] = __uint_as_float(r[0].y); v[2] = __uint_as_float(r[0].z); v[3] = __uint_as_float(r[0].w);
+        v[4] = __uint_as_float(r[1].x); v[5] = __uint_as_float(r[1].y); v[6] = __uint_as_float(r[1].z); v[7] = __uint_as_float(r[1].w);
+    } else {
+        const uint32_t w[4] = {r[0].x, r[0].y, r[0].z, r[0].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (dtype == VARQ_F16) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+                v[2 * j] = f.x; v[2 * j + 1] = f.y;
+            } else {                         // a bf16 is the upper half of an fp32
+                v[2 * j] = __uint_as_float(w[j] << 16);
+                v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+            }
+        }
+    }
+}
+
 template <int D, int NQ, int QT, int KM, int VM>
 __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, NQ, QT, KM, VM>::CTAS) attn_tc_kernel(AttnArgs a, TcDyn dy, int kb, int vb) {
     using P = TcPlan<D, NQ, QT, KM, VM>;
@@ -629,7 +664,51 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             // ---- queries -> tensor memory as fp16 hi [, lo]; the sign of the softmax scale goes with them
             float qsum = 0.f;
             {
-                const long long qoff = b * a.qs_b + (long long)(q0 + (live ? r : 0)) * a.qs_l + h * a.qs_h + half * DH;
+                // fp32 and normalised queries: a warp reads 64 (16-bit: 32) contiguous bytes of a row with four (two) lanes and hands each lane its own
+                // row through shared memory (the V stages, which the V converters leave alone until the queries are in place).  Every lane
+                // reading its row took 32 sectors an instruction and 7000 cycles of a CTA.  us per call, before / after: int8 B64 H16 256 x 680
+                // 155 / 149, int8 per dim B100 H16 228 / 217, int4 B64 H30 324 x 645 526 / 498; c128 group 32 400 x 921 171 / 165, 64 x 121 21 / 20, fp32 int8
+                // 1040 / 1012.  One operand (16-bit queries, half of the bytes) is read directly: the loop behind lost more to its changed
+                // schedule (c64 int2 1237 / 1278, c128 int8 886 / 985).
+                const long long q_own = b * a.qs_b + (long long)(q0 + (live ? r : 0)) * a.qs_l + h * a.qs_h + half * DH;
+                const long long q_first = b * a.qs_b + (long long)q0 * a.qs_l + h * a.qs_h + half * DH;
+                unsigned char* stage = smem + P::OFF_V + warp * P::Q_STAGE;
+                uint4 raw[8];
+                auto fetch = [&](auto es_c, int c0) {
+                    constexpr int ES = decltype(es_c)::value;       // bytes of an element = lanes of a row segment of 16 elements
+#pragma unroll
+                    for (int p = 0; p < 2 * ES; ++p) {
+                        const int row = t * TC_M + quarter * 32 + (p & (ES - 1)) * (32 / ES) + lane / ES;
+                        raw[p] = load_q16<ES>(a.q, q_first + (long long)(row < nq ? row : 0) * a.qs_l + c0 + (p / ES) * 16 + (lane & (ES - 1)) * (16 / ES));
+                    }
+                };
+                auto spread = [&](auto es_c, float (&v)[4][8]) {
+                    constexpr int ES = decltype(es_c)::value, PITCH = 16 * ES + 16;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        __syncwarp();
+#pragma unroll
+                        for (int p = 0; p < ES; ++p) *reinterpret_cast<uint4*>(stage + (p * (32 / ES) + lane / ES) * PITCH + (lane & (ES - 1)) * 16) = raw[u * ES + p];
+                        __syncwarp();
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            uint4 w[ES / 2];
+#pragma unroll
+                            for (int p = 0; p < ES / 2; ++p) w[p] = *reinterpret_cast<const uint4*>(stage + lane * PITCH + (e * (ES / 2) + p) * 16);
+                            q8_floats<ES>(w, a.q_dtype, v[2 * u + e]);
+                        }
+                    }
+                };
+                auto rows_at = [&](int c0, float (&v)[4][8]) {      // 32 head_dim values from c0 on; the next ones are requested
+                    if constexpr (!P::Q_STAGED) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) load_q8(a.q, a.q_dtype, q_own + c0 + 8 * u, v[u]);
+                        return;
+                    }
+                    const int next = c0 + 32;
+                    if (a.q_dtype == VARQ_F32) { if (c0 == 0) fetch(IntC<4>(), 0); spread(IntC<4>(), v); if (next < DH) fetch(IntC<4>(), next); }
+                    else { if (c0 == 0) fetch(IntC<2>(), 0); spread(IntC<2>(), v); if (next < DH) fetch(IntC<2>(), next); }
+                };
                 float mul = a.scale_log2 < 0.f ? -1.f : 1.f;
                 if (fabsf(a.scale_log2) < TC_MIN_SCALE) mul *= fabsf(a.scale_log2);
                 if (a.q_norm) {       // x / max(||x||_2, eps) * scale_mul[h], on the way in
@@ -637,8 +716,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
 #pragma unroll 1
                     for (int c0 = 0; c0 < DH; c0 += 32) {
                         float v[4][8];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) load_q8(a.q, a.q_dtype, qoff + c0 + 8 * u, v[u]);
+                        rows_at(c0, v);
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -651,8 +729,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
 #pragma unroll 1
                 for (int c0 = 0; c0 < DH; c0 += 32) {
                     float v[4][8];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) load_q8(a.q, a.q_dtype, qoff + c0 + 8 * u, v[u]);
+                    rows_at(c0, v);
                     uint32_t hi[16], lo[16];
                     auto pack = [&](auto bits_c) {
 #pragma unroll
@@ -973,7 +1050,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
 #pragma unroll 1
                 for (int i = 0; i < T; ++i) {
                     const int ps = i % PST, vs = i % VST;
-                    bool ok = mbar_wait(&bar_pv[ps], (i / PST) & 1, abort_flag, 23);
+                    bool ok = (!P::Q_STAGED || i > 0 || mbar_wait(bar_q, 0, abort_flag, 27)) && mbar_wait(&bar_pv[ps], (i / PST) & 1, abort_flag, 23);
                     if (ok && i >= VST) ok = mbar_wait(&bar_o[vs], ((i - VST) / VST) & 1, abort_flag, 24);    // V stage is free
                     if (!ok) break;
                     const unsigned char* rec = smem + dy.vrec + ps * dy.vrec_stage;
