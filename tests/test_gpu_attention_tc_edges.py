@@ -40,3 +40,16 @@ def test_against_the_oracle(D, q_dtype, kb, vb, options, lq, lk, gain):
     err, rel = (out - ref).abs().max().item(), ((out - ref).norm() / ref.norm()).item()
     assert err <= 2e-3 and rel <= 1e-3, f"max-abs {err:.3e}, rel-L2 {rel:.3e}"
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,lq,lk", [(2, 16, 169, 424), (4, 16, 256, 680), (5, 16, 256, 680), (1, 16, 169, 424), (2, 16, 256, 1024), (2, 16, 256, 1025), (1, 12, 400, 300)])
+def test_query_tiles_per_cta(B, H, lq, lk):
+    """Both sides of the line between one and two query tiles per CTA (few CTAs, short caches), with and without key splits."""
+    g = torch.Generator(device="cuda").manual_seed(lq + lk)
+    kq, vq = (VAR_Q(qkv_format="BHLc", quant_bits=8, quant_method="G_TOKEN_HEAD", max_tokens=lk) for _ in range(2))
+    for qz in (kq, vq):
+        qz.append(torch.randn((B, H, lk, 64), generator=g, device="cuda"))
+    q = torch.randn((B, H, lq, 64), generator=g, device="cuda")
+    out = attend_cached(q, kq, vq, 0.125, out_dtype=torch.float32).transpose(1, 2).double()
+    ref = torch.softmax(q.double() @ kq.dequant_all().double().transpose(-1, -2) * 0.125, -1) @ vq.dequant_all().double()
+    assert ((out - ref).norm() / ref.norm()).item() <= 1e-3        # fp16 weights

@@ -40,13 +40,20 @@ bool attn_tc_eligible(const AttnArgs& a, int kb, int vb) {
     return true;
 }
 
-// Two query tiles per CTA share every converted K / V tile; a second tile needs queries to fill it.
-static int tc_query_tiles(int Lq, int D) { return D == 64 && Lq > TC_M ? 2 : 1; }
+// Two query tiles per CTA share every converted K / V tile; a second tile needs queries to fill it.  Where such CTAs would fill less than half
+// of the SMs and the cache is short, single tiles occupy twice as many, and need no key splits and no merge.  us, two / one tile, int8 per head
+// H16: 169 queries over 424 tokens B2 18.8 / 13.5, B4 15.3 / 14.1; 256 over 680 B2 22.3 / 17.2, B4 21.1 / 18.0.  Over long caches the splits are worth
+// more (256 over 8000 int4 group 32 B2 50 / 98), and with fewer CTAs still both are split (169 over 424, per dim, B1 15.3 / 16.7).
+static int tc_query_tiles(int B, int H, int Lq, int Lk, int D) {
+    if (D != 64 || Lq <= TC_M) return 1;
+    const long long heads = (long long)B * H, one = heads * ((Lq + TC_M - 1) / TC_M), two = heads * ((Lq + 2 * TC_M - 1) / (2 * TC_M));
+    return Lk <= 16 * TC_N && two * 2 <= sm_count() && one * 4 > sm_count() ? 1 : 2;
+}
 
 // Key range of a CTA.  Splitting pays when the CTAs of the unsplit grid leave most of the chip idle and every part still has a few
 // tiles to hide its set-up behind (the merge is a second launch).
 static int tc_splits(int B, int H, int Lq, int Lk, int D, int& tiles_per_split) {
-    const int tiles = (Lk + TC_N - 1) / TC_N, rows = tc_query_tiles(Lq, D) * TC_M;
+    const int tiles = (Lk + TC_N - 1) / TC_N, rows = tc_query_tiles(B, H, Lq, Lk, D) * TC_M;
     const long long ctas = (long long)B * H * ((Lq + rows - 1) / rows);
     tiles_per_split = tiles;
     if (ctas * 4 > sm_count()) return 1;
@@ -60,7 +67,7 @@ static int tc_splits(int B, int H, int Lq, int Lk, int D, int& tiles_per_split) 
 size_t attn_tc_workspace_bytes(int B, int H, int Lq, int Lk, int D) {
     if (D != 64 && D != 128) return 0;
     int tps;
-    const int splits = tc_splits(B, H, Lq, Lk, D, tps), rows = tc_query_tiles(Lq, D) * TC_M;
+    const int splits = tc_splits(B, H, Lq, Lk, D, tps), rows = tc_query_tiles(B, H, Lq, Lk, D) * TC_M;
     if (splits == 1) return 256;
     return (size_t)B * H * splits * ((Lq + rows - 1) / rows) * rows * (D + 2) * sizeof(float) + 256;
 }
@@ -107,7 +114,7 @@ int attn_tc_run(const AttnArgs& a0, int kb, int vb, void* ws, size_t ws_bytes, c
         if (pv->n_rows > a.Lk) pv->n_rows = 0;         // more rows than keys: read those that the keys name
     step_tables(a, dy);
     const bool window = dy.k_mode == PM_WINDOW || dy.v_mode == PM_WINDOW;
-    const int qt = window ? 1 : tc_query_tiles(a.Lq, a.D), rows = qt * TC_M;       // (fewer rows of partials than the workspace is sized for)
+    const int qt = window ? 1 : tc_query_tiles(a.B, a.H, a.Lq, a.Lk, a.D), rows = qt * TC_M;       // (fewer rows of partials than the workspace is sized for)
     a.n_qtiles = (a.Lq + rows - 1) / rows;
     if ((long long)a.B * a.H * a.n_qtiles * a.splits * rows > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 query rows");
     dy.k_bulk = dy.k_mode == PM_GROUP && bulk_params(a.kp, a.D);
