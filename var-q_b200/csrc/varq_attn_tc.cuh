@@ -5,9 +5,9 @@
 // over the S columns they came from, the A operand of O += P V) and the output accumulators.  Shared memory then only feeds the
 // B operands: with A in shared memory a 128 x 64 x 16 product costs 48 cycles of its bandwidth against 32 of the tensor pipe
 // (measured), with A in tensor memory it runs at the pipe's rate.  Warps:
-//   softmax    eight per query tile, two threads per query row (= TMEM lane).  A thread reads 32 scores of a key tile, applies the per-key
-//              tables where K or V keep exact codes, exponentiates against its lazily updated reference maximum, sums the rounded
-//              P in registers and writes P back to tensor memory;
+//   softmax    one thread per query row (= TMEM lane) at head_dim 64, two at 128.  A thread reads the scores of a key tile, applies the per-key
+//              tables where K or V keep exact codes, exponentiates against a lazily updated reference, sums the rounded P in registers
+//              and writes P back to tensor memory;
 //   K and V converters: turn a tile's packed rows into 128B-swizzled fp16 operand tiles in shared memory.  K: exact integer codes
 //              minus zero-point (one scale per key, applied to S in fp32), or an fp16 hi + lo pair of (code - zp) * scale when the scale
 //              varies along head_dim.  V: codes minus zero-point (the per-key scale is folded into P through the exponent and taken out
@@ -19,14 +19,10 @@
 // More than 128 queries share each converted tile (QT = 2, head_dim 64, all 512 TMEM columns); up to 128 queries run as two CTAs per SM of
 // 256 columns each, one CTA's set-up and dependent waits under the other's tiles.  At head_dim 128 one CTA keeps three or four score
 // tiles in flight.
-// What bounds it, from builds in which one role skips its arithmetic (us a call: all / no conversion / no softmax / one score product):
-//   c 64   B64 H16 256 x 10521, int2 group 32, bf16 queries      1306 / 1340 /  724 / 1271
-//          B64 H16 256 x 680, int8 per head, fp32 queries         182 /  179 /  103 /  175
-//          B32 H30 1024 x 2240, int4, K per dim, fp32 queries    1426 / 1546 /  851 / 1410
-//   c 128  B4 H16 4096 x 10521, int4 and int2 group 32, fp32     2395 / 2412 / 2221 / 2335     (neither conversion nor softmax: 1814)
-//          B6 H16 1600 x 6000, int8 per dim, fp32                1040 /  936 /  953 /  962     (neither: 730)
-// At head_dim 64 the softmax warps, two per sub-partition, each a serial chain of score load, exponentials and P store.  At 128 no role by
-// itself: conversion and softmax share the issue slots, the tensor pipe is behind both (hi + lo operands, 4 products of 256 cycles a tile).
+// What bounds it: at head_dim 64 the softmax warps, two per sub-partition (64 x 256 scores: 1024 cycles of the exponential unit, 1900 to 2300 in
+// all beside conversion and tensor pipe; 2800 while the maximum came before the exponentials).  Without exponentials 1299 -> 923 us (B64 H16
+// 256 x 10521, int2 group 32), without tables 1279 -> 1180 (B32 H30 1024 x 2240, int4, K per dim).  At 128 softmax and conversion share the issue slots
+// (1650 and 1800 cycles a tile, tensor pipe 1024), and long calls run into the power limit: what fewer cycles save the clock gives back in part.
 // Few CTAs over a long cache: the key range is split across CTAs and a second kernel merges the partial rows.
 // Numerics: integer codes are exact in fp16; an fp32 query is split into hi + lo fp16 halves, a dequantised K likewise (the lo x lo
 // product is below fp32 resolution), so S has fp32-like accuracy; P and a dequantised V are rounded to fp16 once; sums are fp32.
@@ -249,7 +245,7 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr int OFF_PREF = OFF_MISC + 16;            // ParamRef [2]
     static constexpr int OFF_XCH = OFF_PREF + 2 * 48;         // float [4][QT * 128]: the two threads of a row, maxima and sums
     static constexpr int OFF_DYN = OFF_XCH + (HV == 2 ? 4 * QT * TC_M * 4 : 0);   // packed stages, records, step tables: sizes known at launch (TcDyn)
-    static constexpr bool Q_STAGED = NQ == 2;      // queries come in through shared memory:
+    static constexpr bool Q_STAGED = NQ == 2 || (D == 64 && KX);      // queries come in through shared memory:
     static constexpr int Q_STAGE = 32 * 80;                   // bytes per softmax warp, in the V stages
     static_assert(K_WARP0 * Q_STAGE <= VST * T_BYTES, "query staging");
     static_assert(OFF_DYN % 16 == 0 && (OFF_TAB % 1024) == 0, "alignment");
@@ -664,12 +660,12 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             // ---- queries -> tensor memory as fp16 hi [, lo]; the sign of the softmax scale goes with them
             float qsum = 0.f;
             {
-                // fp32 and normalised queries: a warp reads 64 (16-bit: 32) contiguous bytes of a row with four (two) lanes and hands each lane its own
+                // A warp reads 64 (16-bit: 32) contiguous bytes of a row with four (two) lanes and hands each lane its own
                 // row through shared memory (the V stages, which the V converters leave alone until the queries are in place).  Every lane
                 // reading its row took 32 sectors an instruction and 7000 cycles of a CTA.  us per call, before / after: int8 B64 H16 256 x 680
                 // 155 / 149, int8 per dim B100 H16 228 / 217, int4 B64 H30 324 x 645 526 / 498; c128 group 32 400 x 921 171 / 165, 64 x 121 21 / 20, fp32 int8
-                // 1040 / 1012.  One operand (16-bit queries, half of the bytes) is read directly: the loop behind lost more to its changed
-                // schedule (c64 int2 1237 / 1278, c128 int8 886 / 985).
+                // 1040 / 1012.  16-bit queries come so over exact K at head_dim 64 (int2, 1044 x 505 85 / 80; 244 x 258 27.0 / 25.4); in the other kernels of one
+                // operand the loop behind lost more to its changed schedule (c64 int2 group 32 1237 / 1278, c128 int8 886 / 985).
                 const long long q_own = b * a.qs_b + (long long)(q0 + (live ? r : 0)) * a.qs_l + h * a.qs_h + half * DH;
                 const long long q_first = b * a.qs_b + (long long)q0 * a.qs_l + h * a.qs_h + half * DH;
                 unsigned char* stage = smem + P::OFF_V + warp * P::Q_STAGE;
