@@ -233,6 +233,10 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr int KST = CTAS == 2 ? 2 : 3, VST = KST;  // operand stages
     static constexpr int PST = D == 128 ? 2 : KST;            // packed stages (at most KST)
     static constexpr int SB = D == 64 ? 2 : ALT ? 3 : 4;    // score tiles in tensor memory, per query tile
+    // The softmax of a tile: one block of exponentials, conversion and sum, behind which the reference may turn out to be too low, or the maximum
+    // first.  At head_dim 128 the block takes issue slots from the converters of a dequantised K and from the other tile of ALT.  us, block / maximum
+    // first, B2 H16 4096 x 10521: int8 in groups of 32 1460 / 1253, int8 per dim 1298 / 1285, ALT int8 per head 1050 / 986; exact K, two operands 1216 / 1490.
+    static constexpr bool BLOCK = D == 64 || (KX && !ALT);
     static constexpr bool TAB = KX || VX;                     // per-key softmax tables
     static constexpr int TS = CTAS == 2 ? 8 : 16;             // table slots: more than PST + KST + SB tiles
     static constexpr int TAB_FLOATS = 4 * TC_N + 4;           // K scale, log2 V scale, 1 / V scale, K zero-point term; flag
@@ -768,7 +772,39 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 return P::TAB ? mbar_test(&bar_t[i % TS], (i / TS) & 1) && r : r;
             };
             bool ready = false;
-            bool behind = true;        // the reference has to follow this tile's scores before its P is computed
+            // The reference becomes `mt` (log2 domain) where that is higher, and what has been accumulated is rescaled (a factor 1 for the other rows)
+            auto move_reference = [&](int i, float mt, float margin) -> bool {
+                if (HV == 2 && !ALT) {
+                    xch[half * XH] = mt;
+                    pair_sync();
+                    mt = fmaxf(mt, xch[(half ^ 1) * XH]);
+                }
+                const float m_new = mt > m_used + margin ? mt : m_used;
+                const float alpha = ex2(m_used - m_new);    // 0 for a row without a reference yet
+                m_used = m_new;
+                l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
+                if (i < STEP) return true;
+                // The accumulator is stable.  With two query tiles bar_o waits for both, and the other may be so far behind that the parity
+                // of an earlier phase answers: each has barriers of its own.
+                const int o = i - STEP;
+                ok = ok && (QT == 2 ? mbar_wait(&bar_sf[2 * t + (o & 1)], (o >> 1) & 1, abort_flag, 13) : mbar_wait(&bar_o[o % VST], (o / VST) & 1, abort_flag, 13));
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) return false;
+                tc_fence_after();
+#pragma unroll 1
+                for (int c0 = ALT ? 0 : half * DH; c0 < (ALT ? D : (half + 1) * DH); c0 += 16) {
+                    uint32_t acc[16];
+                    tmem_ld16(col_acc + c0, acc);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[j] = __float_as_uint(__uint_as_float(acc[j]) * alpha);
+                    tmem_st16(col_acc + c0, acc);
+                }
+                tmem_wait_st();
+                return true;
+            };
+            constexpr bool block = P::BLOCK;
+            bool behind = true;        // (block) the reference has to follow this tile's scores before its P is computed
             // Once a wait has expired nothing is read or written any more, but a pair's barriers are still taken: without ALT both warps
             // run all iterations.
 #pragma unroll 1
@@ -779,10 +815,15 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     if (P::TAB) ok = ok && mbar_wait_warp(&bar_t[i % TS], (i / TS) & 1, abort_flag, 12);
                     if (!ok) {
                         if (HV == 1 || ALT) break;
-                        if (behind) pair_sync();
-                        const bool again = !behind && pair_any(false);
-                        behind = again;
-                        if (!again) i += STEP;
+                        if constexpr (block) {
+                            if (behind) pair_sync();
+                            const bool again = !behind && pair_any(false);
+                            behind = again;
+                            if (!again) i += STEP;
+                        } else {
+                            if (pair_any(false)) pair_sync();
+                            i += STEP;
+                        }
                         continue;
                     }
                 }
@@ -802,56 +843,13 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                         if (j >= nv) x[j] = __float_as_uint(TC_MASKED);
                     }
                 }
-                const bool settled = behind;       // (both threads of a row have read their scores before either stores P over them: here and where they vote below)
-                if (behind) {
-                    // The first tile, and where some row of these warps meets scores far above its reference: the tile's maximum becomes the
-                    // reference and what has been accumulated is rescaled (a factor 1 for the other rows).
-                    float mt = -FLT_MAX;
-#pragma unroll
-                    for (int j = 0; j < NC; j += 4) {
-                        const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c), b4 = VX ? tab4(tab + N + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        mt = max3(mt, fmaf(__uint_as_float(x[j]), k4.x, b4.x), fmaf(__uint_as_float(x[j + 1]), k4.y, b4.y));
-                        mt = max3(mt, fmaf(__uint_as_float(x[j + 2]), k4.z, b4.z), fmaf(__uint_as_float(x[j + 3]), k4.w, b4.w));
-                    }
-                    if (HV == 2 && !ALT) {
-                        xch[half * XH] = mt;
-                        pair_sync();
-                        mt = fmaxf(mt, xch[(half ^ 1) * XH]);
-                    }
-                    behind = false;
-                    const float m_new = fmaxf(mt, m_used);
-                    const float alpha = ex2(m_used - m_new);    // 0 for a row without a reference yet
-                    m_used = m_new;
-                    l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
-                    if (i >= STEP) {
-                        // The accumulator is stable.  With two query tiles bar_o waits for both, and the other may be so far behind that the parity
-                        // of an earlier phase answers: each has barriers of its own.
-                        const int o = i - STEP;
-                        ok = ok && (QT == 2 ? mbar_wait(&bar_sf[2 * t + (o & 1)], (o >> 1) & 1, abort_flag, 13) : mbar_wait(&bar_o[o % VST], (o / VST) & 1, abort_flag, 13));
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) { ready = false; i += STEP; continue; }
-                        tc_fence_after();
-#pragma unroll 1
-                        for (int c0 = ALT ? 0 : half * DH; c0 < (ALT ? D : (half + 1) * DH); c0 += 16) {
-                            uint32_t o[16];
-                            tmem_ld16(col_acc + c0, o);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-                            tmem_st16(col_acc + c0, o);
-                        }
-                        tmem_wait_st();
-                    }
-                }
-                // ---- P = 2^(score - reference), with the V scale where V keeps exact codes: fp16 pairs.  The row sum adds up the rounded P
-                // that multiplies V, so that a row dominated by one key stays exact.
-                const float nm = -m_used;
                 float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
                 auto to_half = [&](int j, const float (&y)[4]) {
                     const __half2 h01 = __floats2half2_rn(ex2(y[0]), ex2(y[1])), h23 = __floats2half2_rn(ex2(y[2]), ex2(y[3]));
                     ph[j / 2] = *reinterpret_cast<const uint32_t*>(&h01);
                     ph[j / 2 + 1] = *reinterpret_cast<const uint32_t*>(&h23);
                 };
+                // The row sum adds up the rounded P that multiplies V, so that a row dominated by one key stays exact
                 auto sum_up = [&](int j) {
                     if constexpr (VX) {       // P carries the V scale: the softmax weight is P / V scale
                         const float4 v4 = tab4(tab + 2 * N + j);
@@ -863,36 +861,63 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                         add_halves(s2, s3, ph[j / 2 + 1]);
                     }
                 };
-                if constexpr (ALT) {
-                    // The maximum first and the sum behind the store of P: two warps of a sub-partition on tiles of different age fill each
-                    // other's gaps already (B8 H16 Lq2048 Lk4096 int8, bf16 queries: 872 us, 937 us as the block below).  Nothing of it may move up
-                    // into the waits for the scores (910 us).
+                auto store_p = [&]() {
+                    if constexpr (NC == 64) tmem_st32(s_addr, ph); else tmem_st16(s_addr + half * 16, *reinterpret_cast<uint32_t (*)[16]>(ph));
+                };
+                // ---- P = 2^(score - reference), with the V scale where V keeps exact codes: fp16 pairs.
+                if constexpr (!block) {
+                    // The maximum first and the sum behind the store of P.  Nothing of it may move up into the waits for the scores (ALT, B8 H16 Lq2048 Lk4096
+                    // int8: 872 us, 910 us where it did).
                     asm volatile("" ::: "memory");
                     float ma = -FLT_MAX, mb = -FLT_MAX;
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) {
-                        const float4 k4 = tab4(tab + j), b4 = VX ? tab4(tab + N + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        float y[4];
-                        fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), k4.x, k4.y, b4.x, b4.y);
-                        fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), k4.z, k4.w, b4.z, b4.w);
-                        ma = max3(ma, y[0], y[1]);
-                        mb = max3(mb, y[2], y[3]);
+                        if constexpr (P::TAB) {
+                            const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c), b4 = VX ? tab4(tab + N + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            float y[4];
+                            fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), k4.x, k4.y, b4.x, b4.y);
+                            fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), k4.z, k4.w, b4.z, b4.w);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) x[j + e] = __float_as_uint(y[e]);
+                            for (int e = 0; e < 4; ++e) x[j + e] = __float_as_uint(y[e]);
+                        }
+                        ma = max3(ma, __uint_as_float(x[j]), __uint_as_float(x[j + 1]));
+                        mb = max3(mb, __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]));
                     }
-                    if (!settled && __any_sync(0xffffffffu, fmaxf(ma, mb) > m_used + TC_LAZY)) { ready = behind = true; continue; }
+                    const float mt = fmaxf(ma, mb) * (P::TAB ? 1.f : c);
+                    // (the vote: both threads of a row have read their scores before either stores P over them)
+                    if (pair_any(mt > m_used + TC_LAZY) && !move_reference(i, mt, TC_LAZY)) { i += STEP; continue; }
+                    const float nm = -m_used;
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) {
                         float y[4];
-                        add2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), nm, nm);
-                        add2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), nm, nm);
+                        if constexpr (P::TAB) {
+                            add2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), nm, nm);
+                            add2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), nm, nm);
+                        } else {
+                            fma2(y[0], y[1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]), c, c, nm, nm);
+                            fma2(y[2], y[3], __uint_as_float(x[j + 2]), __uint_as_float(x[j + 3]), c, c, nm, nm);
+                        }
                         to_half(j, y);
                     }
-                    tmem_st32(s_addr, ph);
+                    store_p();
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) sum_up(j);
                 } else {
+                    const bool settled = behind;       // (both threads of a row have read their scores before either stores P over them: here and where they vote below)
+                    if (behind) {
+                        // The first tile, and where some row of these warps meets scores far above its reference
+                        float mt = -FLT_MAX;
+#pragma unroll
+                        for (int j = 0; j < NC; j += 4) {
+                            const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c), b4 = VX ? tab4(tab + N + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            mt = max3(mt, fmaf(__uint_as_float(x[j]), k4.x, b4.x), fmaf(__uint_as_float(x[j + 1]), k4.y, b4.y));
+                            mt = max3(mt, fmaf(__uint_as_float(x[j + 2]), k4.z, b4.z), fmaf(__uint_as_float(x[j + 3]), k4.w, b4.w));
+                        }
+                        behind = false;
+                        if (!move_reference(i, mt, 0.f)) { ready = false; i += STEP; continue; }
+                    }
                     // One block of straight code: the exponential unit takes most of it, everything else fits in between
+                    const float nm = -m_used;
 #pragma unroll
                     for (int j = 0; j < NC; j += 4) {
                         const float4 k4 = KX ? tab4(tab + j) : make_float4(c, c, c, c);
@@ -911,11 +936,11 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                     const float limit = VX ? tab[4 * N + 1 - first_col] : TC_SUM_MAX;
                     const bool high = !((s0 + s1) + (s2 + s3) <= limit);
                     if (!settled && pair_any(high)) { ready = behind = true; continue; }
-                    if constexpr (NC == 64) tmem_st32(s_addr, ph); else tmem_st16(s_addr + half * 16, *reinterpret_cast<uint32_t (*)[16]>(ph));
+                    store_p();
                 }
                 l0 += s0; l1 += s1; l2 += s2; l3 += s3;
                 i += STEP;
-                ready = !ALT && i < T && tile_ready(i);       // (ALT: the next tile of a warp is seldom there yet)
+                ready = block && i < T && tile_ready(i);
                 tmem_wait_st();
                 tc_fence_before();
                 mbar_arrive(&bar_p[t * SB + s]);
