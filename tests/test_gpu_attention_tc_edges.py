@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from oracle import varq_oracle as O
+from test_gpu_attention_normalised import attend_qnorm, exact, rel
 from VAR_Q import _cabi
 from VAR_Q.attention import attend_cached
 from VAR_Q.quant import VAR_Q
@@ -53,3 +54,29 @@ def test_query_tiles_per_cta(B, H, lq, lk):
     out = attend_cached(q, kq, vq, 0.125, out_dtype=torch.float32).transpose(1, 2).double()
     ref = torch.softmax(q.double() @ kq.dequant_all().double().transpose(-1, -2) * 0.125, -1) @ vq.dequant_all().double()
     assert ((out - ref).norm() / ref.norm()).item() <= 1e-3        # fp16 weights
+
+
+@pytest.mark.parametrize("normalised", [False, True])
+@pytest.mark.parametrize("dtype,shift,pad", [(torch.float32, 1, 1), (torch.bfloat16, 1, 0), (torch.bfloat16, 0, 3), (torch.float16, 3, 1)])
+@pytest.mark.parametrize("kw", [dict(quant_bits=8, quant_method="G_TOKEN_HEAD"), dict(quant_bits=4, quant_method="G_TOKEN_HEAD", symmetric=False, group_size=32),
+                                dict(quant_bits=2, quant_method="G_SCALE_HEAD_DIM", symmetric=False)], ids=["head8", "group32", "dim2"])
+@pytest.mark.parametrize("D,lq", [(64, 45), (64, 150), (128, 45), (128, 150)])
+def test_query_rows_off_a_16_byte_boundary(D, lq, kw, dtype, shift, pad, normalised):
+    """Rows that start anywhere and lie any distance apart, in every kind of kernel that reads them in pieces of 16 bytes."""
+    B, H, lk = 2, 3, 150
+    g = torch.Generator(device=DEV).manual_seed(lq + shift)
+    kq, vq = (VAR_Q(qkv_format="BHLc", max_tokens=lk, **kw) for _ in range(2))
+    for n in (50, 100):
+        kq.append(torch.nn.functional.normalize(torch.randn((B, H, n, D), generator=g, device=DEV), dim=-1))
+        vq.append(torch.randn((B, H, n, D), generator=g, device=DEV))
+    row = H * D + pad
+    flat = torch.randn(B * lq * row + 8, generator=g, device=DEV).to(dtype)[shift:]
+    q = flat.as_strided((B, H, lq, D), (lq * row, D, row, 1))
+    mul = torch.linspace(2.0, 4.0, H, device=DEV)
+    if normalised:
+        out, ref = attend_qnorm("tc", q, kq, vq, 1.0, mul), exact(q, mul, kq.dequant_all(), vq.dequant_all(), 1.0)
+    else:
+        _cabi.force_attn_path("tc")
+        out = attend_cached(q, kq, vq, 0.2, out_dtype=torch.float32)
+        ref = (torch.softmax(q.double() @ kq.dequant_all().double().transpose(-1, -2) * 0.2, -1) @ vq.dequant_all().double()).transpose(1, 2)
+    assert rel(out, ref) <= 1e-3        # fp16 weights

@@ -164,6 +164,11 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ex2(float x) {
@@ -249,8 +254,14 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr int OFF_PREF = OFF_MISC + 16;            // ParamRef [2]
     static constexpr int OFF_XCH = OFF_PREF + 2 * 48;         // float [4][QT * 128]: the two threads of a row, maxima and sums
     static constexpr int OFF_DYN = OFF_XCH + (HV == 2 ? 4 * QT * TC_M * 4 : 0);   // packed stages, records, step tables: sizes known at launch (TcDyn)
-    static constexpr bool Q_STAGED = NQ == 2 || (D == 64 && KX);      // queries come in through shared memory:
-    static constexpr int Q_STAGE = 32 * 80;                   // bytes per softmax warp, in the V stages
+    // Queries that come in through shared memory: a warp reads contiguous pieces of rows and hands each lane its own (the V stages; the V converters
+    // leave them alone until the queries are in place).  Every lane reading its row takes 32 sectors an instruction and 7000 cycles of a CTA.  us per
+    // call, lane by lane / so: head_dim 64, int8 B64 H16 256 x 680 155 / 149, int8 per dim B100 H16 228 / 217, int4 B64 H30 324 x 645 526 / 498, 16-bit
+    // queries over exact int2 1044 x 505 85 / 80; head_dim 128, int8 per dim B16 H16 400 x 921 bf16 normalised 185 / 164, int8 per head B64 144 x 265 196 / 175.
+    // Not so: 16-bit queries over a dequantised K, where the loop behind lost more to its changed schedule (c64 int2 group 32 1237 / 1278, c128 int8
+    // 886 / 985), and up to 128 queries over grouped K at head_dim 64 (9 x 700 fp32 B48 H20 67 / 75, 100 x 255 B100 H16 68 / 74).
+    static constexpr bool Q_STAGED = NQ == 2 ? D == 128 || QT == 2 || KM != PM_GROUP : D == 64 && KX;
+    static constexpr int Q_STAGE = 32 * (D == 128 ? 144 : 80);           // bytes per softmax warp
     static_assert(K_WARP0 * Q_STAGE <= VST * T_BYTES, "query staging");
     static_assert(OFF_DYN % 16 == 0 && (OFF_TAB % 1024) == 0, "alignment");
     static_assert(QT * SB <= 4 && KST <= 3 && TS > PST + KST + SB, "barrier plan");
@@ -664,95 +675,153 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
             // ---- queries -> tensor memory as fp16 hi [, lo]; the sign of the softmax scale goes with them
             float qsum = 0.f;
             {
-                // A warp reads 64 (16-bit: 32) contiguous bytes of a row with four (two) lanes and hands each lane its own
-                // row through shared memory (the V stages, which the V converters leave alone until the queries are in place).  Every lane
-                // reading its row took 32 sectors an instruction and 7000 cycles of a CTA.  us per call, before / after: int8 B64 H16 256 x 680
-                // 155 / 149, int8 per dim B100 H16 228 / 217, int4 B64 H30 324 x 645 526 / 498; c128 group 32 400 x 921 171 / 165, 64 x 121 21 / 20, fp32 int8
-                // 1040 / 1012.  16-bit queries come so over exact K at head_dim 64 (int2, 1044 x 505 85 / 80; 244 x 258 27.0 / 25.4); in the other kernels of one
-                // operand the loop behind lost more to its changed schedule (c64 int2 group 32 1237 / 1278, c128 int8 886 / 985).
                 const long long q_own = b * a.qs_b + (long long)(q0 + (live ? r : 0)) * a.qs_l + h * a.qs_h + half * DH;
                 const long long q_first = b * a.qs_b + (long long)q0 * a.qs_l + h * a.qs_h + half * DH;
                 unsigned char* stage = smem + P::OFF_V + warp * P::Q_STAGE;
-                uint4 raw[8];
-                auto fetch = [&](auto es_c, int c0) {
-                    constexpr int ES = decltype(es_c)::value;       // bytes of an element = lanes of a row segment of 16 elements
-#pragma unroll
-                    for (int p = 0; p < 2 * ES; ++p) {
-                        const int row = t * TC_M + quarter * 32 + (p & (ES - 1)) * (32 / ES) + lane / ES;
-                        raw[p] = load_q16<ES>(a.q, q_first + (long long)(row < nq ? row : 0) * a.qs_l + c0 + (p / ES) * 16 + (lane & (ES - 1)) * (16 / ES));
-                    }
-                };
-                auto spread = [&](auto es_c, float (&v)[4][8]) {
-                    constexpr int ES = decltype(es_c)::value, PITCH = 16 * ES + 16;
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        __syncwarp();
-#pragma unroll
-                        for (int p = 0; p < ES; ++p) *reinterpret_cast<uint4*>(stage + (p * (32 / ES) + lane / ES) * PITCH + (lane & (ES - 1)) * 16) = raw[u * ES + p];
-                        __syncwarp();
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            uint4 w[ES / 2];
-#pragma unroll
-                            for (int p = 0; p < ES / 2; ++p) w[p] = *reinterpret_cast<const uint4*>(stage + lane * PITCH + (e * (ES / 2) + p) * 16);
-                            q8_floats<ES>(w, a.q_dtype, v[2 * u + e]);
-                        }
-                    }
-                };
-                auto rows_at = [&](int c0, float (&v)[4][8]) {      // 32 head_dim values from c0 on; the next ones are requested
-                    if constexpr (!P::Q_STAGED) {
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) load_q8(a.q, a.q_dtype, q_own + c0 + 8 * u, v[u]);
-                        return;
-                    }
-                    const int next = c0 + 32;
-                    if (a.q_dtype == VARQ_F32) { if (c0 == 0) fetch(IntC<4>(), 0); spread(IntC<4>(), v); if (next < DH) fetch(IntC<4>(), next); }
-                    else { if (c0 == 0) fetch(IntC<2>(), 0); spread(IntC<2>(), v); if (next < DH) fetch(IntC<2>(), next); }
-                };
                 float mul = a.scale_log2 < 0.f ? -1.f : 1.f;
                 if (fabsf(a.scale_log2) < TC_MIN_SCALE) mul *= fabsf(a.scale_log2);
-                if (a.q_norm) {       // x / max(||x||_2, eps) * scale_mul[h], on the way in
-                    float ss = 0.f;
+                // values of a row -> fp16 pairs in the order of the operands
+                auto pack = [&](auto bits_c, auto n_c, const float* v, uint32_t* hi, uint32_t* lo) {
+#pragma unroll
+                    for (int e = 0; e < decltype(n_c)::value / 2; ++e) {
+                        float y[2];
+#pragma unroll
+                        for (int z = 0; z < 2; ++z) {      // the operand is fp16: an element beyond its range saturates instead of becoming infinite
+                            const int d = ((2 * e) & ~15) + code_at(decltype(bits_c)::value, (2 * e + z) & 15);
+                            y[z] = fminf(fmaxf(v[d] * mul, -65504.f), 65504.f);
+                        }
+                        const __half2 hh = __floats2half2_rn(y[0], y[1]);
+                        const float2 hf = __half22float2(hh);
+                        hi[e] = *reinterpret_cast<const uint32_t*>(&hh);
+                        if constexpr (NQ == 2) {
+                            const __half2 hl = __floats2half2_rn(y[0] - hf.x, y[1] - hf.y);
+                            lo[e] = *reinterpret_cast<const uint32_t*>(&hl);
+                            if constexpr (KX) qsum += y[0] + y[1];
+                        } else if constexpr (KX) qsum += hf.x + hf.y;
+                    }
+                };
+                if constexpr (P::Q_STAGED && D == 128) {
+                    // 128 bytes of a row at a time (a thread's half of a 16-bit row whole, read once even where it is normalised), and no more in registers than
+                    // 16 values and their halves: with 32, and the next ones under way, every kernel of two operands spilled 164 to 312 bytes.  Calls whose
+                    // only key tile hardly fills take 0.3 us longer than lane by lane (33 x 40 fp32 H20: 6.4 / 6.7 us).
+                    const bool wide_q = a.q_dtype == VARQ_F32;
+                    const int piece = wide_q ? 32 : 64;
+                    auto stage_at = [&](int row, int ch) -> uint4* { return reinterpret_cast<uint4*>(stage + row * 144 + ch * 16); };
+                    auto each16 = [&](bool staged, auto body) {      // body(head_dim value, 16 values from there on)
+#pragma unroll 1
+                        for (int c0 = 0; c0 < DH; c0 += piece) {
+                            if (!staged) {
+                                uint4 raw[8];
+#pragma unroll
+                                for (int p = 0; p < 8; ++p) {
+                                    const int row = quarter * 32 + p * 4 + lane / 8;
+                                    const long long off = q_first + (long long)(row < nq ? row : 0) * a.qs_l + c0;
+                                    raw[p] = wide_q ? load_q16<4>(a.q, off + (lane & 7) * 4) : load_q16<2>(a.q, off + (lane & 7) * 8);
+                                }
+                                __syncwarp();
+#pragma unroll
+                                for (int p = 0; p < 8; ++p) *stage_at(p * 4 + lane / 8, lane & 7) = raw[p];
+                                __syncwarp();
+                            }
+#pragma unroll 1
+                            for (int u = 0; u < piece; u += 16) {
+                                float v[16];
+                                if (wide_q) {
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e) {
+                                        const uint4 w = *stage_at(lane, u / 4 + e);
+                                        v[4 * e] = __uint_as_float(w.x); v[4 * e + 1] = __uint_as_float(w.y); v[4 * e + 2] = __uint_as_float(w.z); v[4 * e + 3] = __uint_as_float(w.w);
+                                    }
+                                } else {
+#pragma unroll
+                                    for (int e = 0; e < 2; ++e) {
+                                        const uint4 w[1] = {*stage_at(lane, u / 8 + e)};
+                                        q8_floats<2>(w, a.q_dtype, *reinterpret_cast<float (*)[8]>(v + 8 * e));
+                                    }
+                                }
+                                body(c0 + u, v);
+                            }
+                        }
+                    };
+                    bool staged = false;
+                    if (a.q_norm) {       // x / max(||x||_2, eps) * scale_mul[h], on the way in
+                        float ss = 0.f;
+                        each16(false, [&](int, const float* v) {
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) ss = fmaf(v[e], v[e], ss);
+                        });
+                        ss = pair_sum(ss);
+                        mul *= (a.q_mul ? __ldg(a.q_mul + h) : 1.f) / fmaxf(sqrtf(ss), a.q_eps);
+                        staged = !wide_q;
+                    }
+                    if (!live) mul = 0.f;
+                    each16(staged, [&](int c, const float* v) {
+                        uint32_t hi[8], lo[8];
+                        if (kb == 8) pack(IntC<8>(), IntC<16>(), v, hi, lo); else if (kb == 4) pack(IntC<4>(), IntC<16>(), v, hi, lo); else pack(IntC<2>(), IntC<16>(), v, hi, lo);
+                        tmem_st8(lane_base + col_q + (half * DH + c) / 2, hi);
+                        tmem_st8(lane_base + col_q + D / 2 + (half * DH + c) / 2, lo);
+                    });
+                } else {
+                    uint4 raw[8];
+                    auto fetch = [&](auto es_c, int c0) {
+                        constexpr int ES = decltype(es_c)::value;       // bytes of an element = lanes of a row segment of 16 elements
+#pragma unroll
+                        for (int p = 0; p < 2 * ES; ++p) {
+                            const int row = t * TC_M + quarter * 32 + (p & (ES - 1)) * (32 / ES) + lane / ES;
+                            raw[p] = load_q16<ES>(a.q, q_first + (long long)(row < nq ? row : 0) * a.qs_l + c0 + (p / ES) * 16 + (lane & (ES - 1)) * (16 / ES));
+                        }
+                    };
+                    auto spread = [&](auto es_c, float (&v)[4][8]) {
+                        constexpr int ES = decltype(es_c)::value, PITCH = 16 * ES + 16;
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            __syncwarp();
+#pragma unroll
+                            for (int p = 0; p < ES; ++p) *reinterpret_cast<uint4*>(stage + (p * (32 / ES) + lane / ES) * PITCH + (lane & (ES - 1)) * 16) = raw[u * ES + p];
+                            __syncwarp();
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                uint4 w[ES / 2];
+#pragma unroll
+                                for (int p = 0; p < ES / 2; ++p) w[p] = *reinterpret_cast<const uint4*>(stage + lane * PITCH + (e * (ES / 2) + p) * 16);
+                                q8_floats<ES>(w, a.q_dtype, v[2 * u + e]);
+                            }
+                        }
+                    };
+                    auto rows_at = [&](int c0, float (&v)[4][8]) {      // 32 head_dim values from c0 on; the next ones are requested
+                        if constexpr (!P::Q_STAGED) {
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) load_q8(a.q, a.q_dtype, q_own + c0 + 8 * u, v[u]);
+                            return;
+                        }
+                        const int next = c0 + 32;
+                        if (a.q_dtype == VARQ_F32) { if (c0 == 0) fetch(IntC<4>(), 0); spread(IntC<4>(), v); if (next < DH) fetch(IntC<4>(), next); }
+                        else { if (c0 == 0) fetch(IntC<2>(), 0); spread(IntC<2>(), v); if (next < DH) fetch(IntC<2>(), next); }
+                    };
+                    if (a.q_norm) {       // x / max(||x||_2, eps) * scale_mul[h], on the way in
+                        float ss = 0.f;
+#pragma unroll 1
+                        for (int c0 = 0; c0 < DH; c0 += 32) {
+                            float v[4][8];
+                            rows_at(c0, v);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) ss = fmaf(v[u][e], v[u][e], ss);
+                        }
+                        ss = pair_sum(ss);
+                        mul *= (a.q_mul ? __ldg(a.q_mul + h) : 1.f) / fmaxf(sqrtf(ss), a.q_eps);
+                    }
+                    if (!live) mul = 0.f;
 #pragma unroll 1
                     for (int c0 = 0; c0 < DH; c0 += 32) {
                         float v[4][8];
                         rows_at(c0, v);
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) ss = fmaf(v[u][e], v[u][e], ss);
+                        uint32_t hi[16], lo[16];
+                        if (kb == 8) pack(IntC<8>(), IntC<32>(), &v[0][0], hi, lo); else if (kb == 4) pack(IntC<4>(), IntC<32>(), &v[0][0], hi, lo); else pack(IntC<2>(), IntC<32>(), &v[0][0], hi, lo);
+                        tmem_st16(lane_base + col_q + (half * DH + c0) / 2, hi);
+                        if constexpr (NQ == 2) tmem_st16(lane_base + col_q + D / 2 + (half * DH + c0) / 2, lo);
                     }
-                    ss = pair_sum(ss);
-                    mul *= (a.q_mul ? __ldg(a.q_mul + h) : 1.f) / fmaxf(sqrtf(ss), a.q_eps);
-                }
-                if (!live) mul = 0.f;
-#pragma unroll 1
-                for (int c0 = 0; c0 < DH; c0 += 32) {
-                    float v[4][8];
-                    rows_at(c0, v);
-                    uint32_t hi[16], lo[16];
-                    auto pack = [&](auto bits_c) {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            float y[2];
-#pragma unroll
-                            for (int z = 0; z < 2; ++z) {      // the operand is fp16: an element beyond its range saturates instead of becoming infinite
-                                const int d = ((2 * e) & ~15) + code_at(decltype(bits_c)::value, (2 * e + z) & 15);
-                                y[z] = fminf(fmaxf(v[d >> 3][d & 7] * mul, -65504.f), 65504.f);
-                            }
-                            const __half2 hh = __floats2half2_rn(y[0], y[1]);
-                            const float2 hf = __half22float2(hh);
-                            hi[e] = *reinterpret_cast<const uint32_t*>(&hh);
-                            if constexpr (NQ == 2) {
-                                const __half2 hl = __floats2half2_rn(y[0] - hf.x, y[1] - hf.y);
-                                lo[e] = *reinterpret_cast<const uint32_t*>(&hl);
-                                if constexpr (KX) qsum += y[0] + y[1];
-                            } else if constexpr (KX) qsum += hf.x + hf.y;
-                        }
-                    };
-                    if (kb == 8) pack(IntC<8>()); else if (kb == 4) pack(IntC<4>()); else pack(IntC<2>());
-                    tmem_st16(lane_base + col_q + (half * DH + c0) / 2, hi);
-                    if constexpr (NQ == 2) tmem_st16(lane_base + col_q + D / 2 + (half * DH + c0) / 2, lo);
                 }
                 tmem_wait_st();
                 tc_fence_before();
