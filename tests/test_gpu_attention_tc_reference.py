@@ -74,3 +74,27 @@ def test_scales_of_a_tile_far_apart(D, lq, q_dtype):
     kq.append(k)
     vq.append(v)
     _check(q.to(q_dtype), kq, vq, 0.3, f"{D} {lq}")
+
+
+@pytest.mark.parametrize("D,lq,q_dtype", [(64, 256, torch.float32), (64, 40, torch.bfloat16), (128, 256, torch.float32), (128, 256, torch.bfloat16)])
+@pytest.mark.parametrize("grows", [False, True])
+def test_heavy_keys_with_small_v_scales(D, lq, q_dtype, grows):
+    """The first key of most tiles is far lighter than the others and its V 10^5 times larger: the sum of the weights passes the limit of its tile,
+    the reference stays.  Some tiles are even, and in some rows larger keys follow later."""
+    B, H, lk = 1, 40, 64 * 9 + 11
+    g = torch.Generator(device=DEV).manual_seed(lq + D)
+    u = torch.nn.functional.normalize(torch.randn((B, H, 1, D), generator=g, device=DEV), dim=-1)
+    k = torch.randn((B, H, lk, D), generator=g, device=DEV) / D ** 0.5 + 3 * u
+    v = torch.randn((B, H, lk, D), generator=g, device=DEV) * 1e-2
+    k[:, :, ::64] -= 6 * u
+    v[:, :, ::64] *= 1e5
+    k[:, :, 128:256:64] += 6 * u
+    v[:, :, 128:256:64] *= 1e-5
+    if grows:
+        k[:, :, 300::150] *= 3.0
+    q = 5 * u + torch.randn((B, H, lq, D), generator=g, device=DEV)
+    q[:, :, 1::3] *= 0.2
+    kq, vq = VAR_Q(qkv_format="BHLc", max_tokens=lk, **HEAD8), VAR_Q(qkv_format="BHLc", max_tokens=lk, **HEAD8)
+    kq.append(k)
+    vq.append(v)
+    _check(q.to(q_dtype), kq, vq, 1.0, f"{D} {lq}")

@@ -841,6 +841,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 return P::TAB ? mbar_test(&bar_t[i % TS], (i / TS) & 1) && r : r;
             };
             bool ready = false;
+            constexpr bool block = P::BLOCK;
             // The reference becomes `mt` (log2 domain) where that is higher, and what has been accumulated is rescaled (a factor 1 for the other rows)
             auto move_reference = [&](int i, float mt, float margin) -> bool {
                 if (HV == 2 && !ALT) {
@@ -850,9 +851,10 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 }
                 const float m_new = mt > m_used + margin ? mt : m_used;
                 const float alpha = ex2(m_used - m_new);    // 0 for a row without a reference yet
+                const bool moved = !block || __any_sync(0xffffffffu, m_new > m_used);       // (the same in the other warp of a pair)
                 m_used = m_new;
                 l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
-                if (i < STEP) return true;
+                if (i < STEP || !moved) return true;
                 // The accumulator is stable.  With two query tiles bar_o waits for both, and the other may be so far behind that the parity
                 // of an earlier phase answers: each has barriers of its own.
                 const int o = i - STEP;
@@ -872,7 +874,6 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                 tmem_wait_st();
                 return true;
             };
-            constexpr bool block = P::BLOCK;
             bool behind = true;        // (block) the reference has to follow this tile's scores before its P is computed
             // Once a wait has expired nothing is read or written any more, but a pair's barriers are still taken: without ALT both warps
             // run all iterations.
@@ -886,9 +887,9 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                         if (HV == 1 || ALT) break;
                         if constexpr (block) {
                             if (behind) pair_sync();
-                            const bool again = !behind && pair_any(false);
+                            const bool again = pair_any(false), retry = again && !behind;
                             behind = again;
-                            if (!again) i += STEP;
+                            if (!retry) i += STEP;
                         } else {
                             if (pair_any(false)) pair_sync();
                             i += STEP;
@@ -982,8 +983,7 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                             mt = max3(mt, fmaf(__uint_as_float(x[j]), k4.x, b4.x), fmaf(__uint_as_float(x[j + 1]), k4.y, b4.y));
                             mt = max3(mt, fmaf(__uint_as_float(x[j + 2]), k4.z, b4.z), fmaf(__uint_as_float(x[j + 3]), k4.w, b4.w));
                         }
-                        behind = false;
-                        if (!move_reference(i, mt, 0.f)) { ready = false; i += STEP; continue; }
+                        if (!move_reference(i, mt, 0.f)) { behind = pair_any(false); ready = false; i += STEP; continue; }      // (the vote of the other warp's tile)
                     }
                     // One block of straight code: the exponential unit takes most of it, everything else fits in between
                     const float nm = -m_used;
@@ -1001,10 +1001,14 @@ __global__ void __launch_bounds__(TcPlan<D, NQ, QT, KM, VM>::THREADS, TcPlan<D, 
                         to_half(j, y);
                         sum_up(j);
                     }
-                    // P has room up to 65504: the sum of the tile's weights shows that none came close, without their maximum
+                    // P has room up to 65504: the sum of the tile's weights shows that none came close, without their maximum.  V scales: below the limit
+                    // the largest of the tile may meet the heaviest weight.  Where heavy keys have far smaller ones the sum passes the limit and the
+                    // reference stays: the next tile then begins with its maximum, and only the first of such tiles is computed twice (scales 10^4
+                    // apart, B16 H16 256 x 2048 fp32, us: c64 173 when all were, 117 so, 90 with even scales; c128 298, 206, 164).
                     const float limit = VX ? tab[4 * N + 1 - first_col] : TC_SUM_MAX;
-                    const bool high = !((s0 + s1) + (s2 + s3) <= limit);
-                    if (!settled && pair_any(high)) { ready = behind = true; continue; }
+                    const bool again = pair_any(!((s0 + s1) + (s2 + s3) <= limit)), retry = again && !settled;
+                    behind = again;
+                    if (retry) { ready = true; continue; }
                     store_p();
                 }
                 l0 += s0; l1 += s1; l2 += s2; l3 += s3;
