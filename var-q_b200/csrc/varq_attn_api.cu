@@ -23,6 +23,24 @@ extern "C" size_t varq_attn_workspace_bytes(int32_t B, int32_t H, int32_t Lq, in
     return s12 > s34 ? s12 : s34;
 }
 
+// 33 to 64 queries over a short cache, one scale per key, head_dim 64: one CTA of the warp-level kernel per (sample, head), four of which share an SM (three
+// with fp32 queries), against two CTAs per SM of the tcgen05 kernel.  us at H16, int8, mid / tcgen05:
+//     16-bit queries   33 over 40   48 over 64   64 over 64   36 over 91   64 over 128  48 over 200   fp32   33 over 40   48 over 64   36 over 91   64 over 128
+//     batch  20       10.3 / 12.9  11.5 / 12.2  13.2 / 12.2  13.6 / 14.8  17.0 / 14.3  21.7 / 19.3          10.9 / 13.3  11.7 / 12.6  13.9 / 15.3  16.1 / 14.4
+//            32       10.6 / 15.9  11.9 / 14.9  13.5 / 14.9  13.7 / 17.7  17.3 / 17.1  21.8 / 22.2          18.6 / 16.1  20.1 / 15.2  23.4 / 18.1  27.6 / 17.4
+//            40       18.4 / 20.9  19.5 / 19.9  20.8 / 19.9  23.9 / 23.4  27.2 / 22.7  35.7 / 29.7          19.8 / 21.1  21.4 / 20.2  24.6 / 24.0  29.7 / 23.1
+//            64       19.8 / 30.0  22.1 / 29.0  25.1 / 29.0  26.1 / 33.7  32.7 / 32.8  41.3 / 42.4          28.4 / 30.6  31.2 / 29.4  36.0 / 34.4  42.4 / 33.2
+//            128      37.7 / 53.6  41.9 / 50.9  46.1 / 51.2  49.6 / 60.2  58.9 / 58.1  78.8 / 76.3          48.7 / 54.8  51.9 / 52.2  62.8 / 61.9  73.1 / 59.4
+// (int4: mid 3 to 10 % less, 64 over 155 B64 34.2 / 39.2, 48 over 200 38.3 / 43.3.)  Up to two CTAs per SM tcgen05 is the faster one (33 over 40, batch 16:
+// 10.2 / 8.2); beyond, what counts is how full the last wave of mid is and how little work a CTA has.  Both keep weights in fp16 and sums in fp32.
+static bool mid_takes_64(bool fp32, bool narrow, long long heads, int Lq, int Lk) {
+    if (heads <= 2 * sm_count()) return false;
+    const long long wave = (fp32 ? 3 : 4) * sm_count(), waves = (heads + wave - 1) / wave;
+    if (fp32 && waves > 1) return Lq <= 40 && Lk <= 64 && heads * 10 >= waves * wave * 7;
+    const bool full = heads * 4 >= waves * wave * 3;
+    return Lk <= 96 ? full || Lq <= 48 : full && narrow && !fp32 && Lk <= 208;       // narrow: K and V below 8 bits
+}
+
 static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const varq_tensor_t* v_codes,
                      const varq_qparams_t* kp, const varq_qparams_t* vp, int32_t B, int32_t H, int32_t Lq,
                      int32_t Lk, int32_t D, int32_t kb, int32_t vb, float softmax_scale,
@@ -69,16 +87,16 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     const int force = __atomic_load_n(&g_forced_path, __ATOMIC_RELAXED);
     const bool small_q = Lq <= 4 || (Lq <= 16 && Lk <= 256);
     // head_dim 64 with one scale per key over at most 256 tokens (the early scales of a schedule), us at H16 (H30 for B128), int8, fp32 queries:
-    //              9 queries over 14 tokens         16 over 30                       25 over 55     36 over 91     64 over 155
-    //     batch    mid / decode / tcgen05 / early   mid / decode / tcgen05 / early   mid / tcgen05  mid / tcgen05  mid / tcgen05
-    //       2     10.0 /   4.3  /   7.1   /  7.4    9.9 /   4.3  /   7.2   / 10.3   10.5 /  7.2    11.6 /  8.0    14.3 /  8.8
-    //      16     10.4 /   7.4  /   8.7   /  8.6   10.7 /   8.3  /   8.8   / 12.3   11.3 /  9.0    14.1 / 10.3    18.9 / 11.7
-    //      32     11.0 /  10.6  /  16.6   / 10.5   11.5 /  12.5  /  16.7   / 14.5   12.9 / 16.9    24.0 / 19.0    32.8 / 21.5
-    //      64     19.5 /  17.6  /  30.6   / 13.5   20.0 /  20.1  /  30.7   / 20.7   22.7 / 30.9    36.4 / 35.8    49.7 / 40.6
-    //     128     48.8 /  58.1  /  96.5   / 41.8   50.8 /  67.8  /  96.9   / 66.8   58.8 / 98.2   139.9 / 115.6  187.8 / 133.9
+    //              9 queries over 14 tokens         16 over 30                       25 over 55
+    //     batch    mid / decode / tcgen05 / early   mid / decode / tcgen05 / early   mid / tcgen05
+    //       2     10.0 /   4.3  /   7.1   /  7.4    9.9 /   4.3  /   7.2   / 10.3   10.5 /  7.2
+    //      16     10.4 /   7.4  /   8.7   /  8.6   10.7 /   8.3  /   8.8   / 12.3   11.3 /  9.0
+    //      32     11.0 /  10.6  /  16.6   / 10.5   11.5 /  12.5  /  16.7   / 14.5   12.9 / 16.9
+    //      64     19.5 /  17.6  /  30.6   / 13.5   20.0 /  20.1  /  30.7   / 20.7   22.7 / 30.9
+    //     128     48.8 /  58.1  /  96.5   / 41.8   50.8 /  67.8  /  96.9   / 66.8   58.8 / 98.2
     // decode and early keep weights to fp32's accuracy (1e-7 against 2e-4 of the other two).  Up to 512 (sample, head) pairs decode takes 9 to 16 queries;
     // beyond, early takes up to 12 of them over one chunk of keys, mid the rest, decode again over more keys (16 queries over 256 tokens at B64: mid 43.8,
-    // decode 30.7).  Up to 32 queries mid is the faster of the last two where the tcgen05 kernel needs more than one wave (two CTAs per SM).
+    // decode 30.7).  17 to 32 queries: mid is the faster of the last two where the tcgen05 kernel needs more than one wave (two CTAs per SM); up to 64: mid_takes_64.
     // mid does not normalise queries: decode or tcgen05 stand in.
     const long long heads = (long long)B * H;
     const bool key_scale = D == 64 && kp->group == D && vp->group == D, few = Lq > 8 && Lq <= 16 && Lk <= 256, crowded = heads > 512 && Lk <= 32;
@@ -92,7 +110,8 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     // accuracy (3e-7 against 2e-4 for fp16 weights).
     const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (few && D == 64 && (q_norm || !crowded)));
     if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
-    const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : few || (Lq > 16 && Lq <= 32 && Lk <= 256 && heads > 2 * sm_count());
+    const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : few || (Lq > 16 && Lq <= 32 && Lk <= 256 && heads > 2 * sm_count())
+                                                                                 || (Lq > 32 && Lq <= 64 && mid_takes_64(q->dtype == VARQ_F32, kb < 8 && vb < 8, heads, Lq, Lk));
     if (want_mid && !q_norm && attn_mid_eligible(a, kb, vb)) return attn_mid_run(a, kb, vb, (cudaStream_t)stream);
     const bool want_tc = force ? (force == VARQ_ATTN_PATH_TC) : !small_q;
     if (want_tc && attn_tc_eligible(a, kb, vb)) return attn_tc_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);

@@ -5,7 +5,7 @@
 // tensor-core instructions (mma.sync m16n8k16, fp16 operands, fp32 accumulators in registers), no asynchronous machinery,
 // 18 KB of shared memory, so several thread blocks share an SM and hide each other's latencies.
 //
-// One CTA = one (sample, head) x 32 queries, two warps of 16 query rows.  Keys go through shared memory 64 at a time:
+// One CTA = one (sample, head) x 32 or 64 queries, two or four warps of 16 query rows.  Keys go through shared memory 64 at a time:
 // the packed rows are turned into exact fp16 integer codes (byte permutes), S = Q K^T on codes, the per-key K scale and
 // zero-point are applied to S in fp32 (s_k * (acc - z_k * sum q)), online softmax in registers (base 2), the per-key V scale is
 // folded into P through the exponent before it is rounded to fp16 (and divided out of the normaliser), O += P V on codes, and the V zero-point term sum_k P_k z_k is subtracted at the
@@ -81,10 +81,10 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-constexpr int MID_ROWS = 32, MID_THREADS = 64;       // many small blocks per SM: more queries than these go to the tcgen05 kernel
-
-template <int KB, int VB, bool QSPLIT>
-__global__ void __launch_bounds__(MID_THREADS, QSPLIT ? 6 : 8) attn_mid_kernel(AttnArgs a) {
+// WARPS = 2 (32 queries per CTA; up to 32 queries measured fastest with many small blocks per SM) or 4 (64 queries)
+template <int KB, int VB, bool QSPLIT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, (QSPLIT ? 12 : 16) / WARPS) attn_mid_kernel(AttnArgs a) {
+    constexpr int MID_ROWS = WARPS * 16, MID_THREADS = WARPS * 32;
     constexpr int D = 64, PITCH = D + 8;                 // halves per shared-memory row: 144 bytes, conflict-free for ldmatrix
     constexpr int KW = D * KB / 32, VW = D * VB / 32;    // packed words per row
     constexpr int NQ = QSPLIT ? 2 : 1;
@@ -327,21 +327,22 @@ bool attn_mid_eligible(const AttnArgs& a, int kb, int vb) {
     return a.D == 64 && a.kp.group == a.D && a.vp.group == a.D;      // one scale / zero-point per key
 }
 
-template <int KB, int VB>
+template <int KB, int VB, int WARPS>
 static int launch_mid(AttnArgs& a, cudaStream_t st) {
+    constexpr int MID_ROWS = WARPS * 16, MID_THREADS = WARPS * 32;
     const int nqt = (a.Lq + MID_ROWS - 1) / MID_ROWS;
     const long long blocks = (long long)a.B * a.H * nqt;
     if (blocks > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 thread blocks");
     a.n_qtiles = nqt;
-    if (a.q_dtype == VARQ_F32) launch_pdl(attn_mid_kernel<KB, VB, true>, (unsigned)blocks, MID_THREADS, 0, st, 1, a);
-    else launch_pdl(attn_mid_kernel<KB, VB, false>, (unsigned)blocks, MID_THREADS, 0, st, 1, a);
+    if (a.q_dtype == VARQ_F32) launch_pdl(attn_mid_kernel<KB, VB, true, WARPS>, (unsigned)blocks, MID_THREADS, 0, st, 1, a);
+    else launch_pdl(attn_mid_kernel<KB, VB, false, WARPS>, (unsigned)blocks, MID_THREADS, 0, st, 1, a);
     VARQ_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return VARQ_OK;
 }
 
 int attn_mid_run(AttnArgs& a, int kb, int vb, cudaStream_t st) {
-#define GO(K_, V_) if (kb == K_ && vb == V_) return launch_mid<K_, V_>(a, st);
+#define GO(K_, V_) if (kb == K_ && vb == V_) return a.Lq <= 32 ? launch_mid<K_, V_, 2>(a, st) : launch_mid<K_, V_, 4>(a, st);
     GO(8, 8) GO(8, 4) GO(8, 2) GO(4, 8) GO(4, 4) GO(4, 2) GO(2, 8) GO(2, 4) GO(2, 2)
 #undef GO
     return fail(VARQ_ERR_ARG, "varq_attn_fwd: store bits must be 2, 4 or 8");
