@@ -86,21 +86,27 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     // fp16) the first scales of a per-dim or group-wise cache are 2e-4 away from the exact result, here 2e-7.
     const int force = __atomic_load_n(&g_forced_path, __ATOMIC_RELAXED);
     const bool small_q = Lq <= 4 || (Lq <= 16 && Lk <= 256);
-    // head_dim 64 with one scale per key over at most 256 tokens (the early scales of a schedule), us at H16 (H30 for B128), int8, fp32 queries:
-    //              9 queries over 14 tokens         16 over 30                       25 over 55
-    //     batch    mid / decode / tcgen05 / early   mid / decode / tcgen05 / early   mid / tcgen05
-    //       2     10.0 /   4.3  /   7.1   /  7.4    9.9 /   4.3  /   7.2   / 10.3   10.5 /  7.2
-    //      16     10.4 /   7.4  /   8.7   /  8.6   10.7 /   8.3  /   8.8   / 12.3   11.3 /  9.0
-    //      32     11.0 /  10.6  /  16.6   / 10.5   11.5 /  12.5  /  16.7   / 14.5   12.9 / 16.9
-    //      64     19.5 /  17.6  /  30.6   / 13.5   20.0 /  20.1  /  30.7   / 20.7   22.7 / 30.9
-    //     128     48.8 /  58.1  /  96.5   / 41.8   50.8 /  67.8  /  96.9   / 66.8   58.8 / 98.2
-    // decode and early keep weights to fp32's accuracy (1e-7 against 2e-4 of the other two).  Up to 512 (sample, head) pairs decode takes 9 to 16 queries;
-    // beyond, early takes up to 12 of them over one chunk of keys, mid the rest, decode again over more keys (16 queries over 256 tokens at B64: mid 43.8,
-    // decode 30.7).  17 to 32 queries: mid is the faster of the last two where the tcgen05 kernel needs more than one wave (two CTAs per SM); up to 64: mid_takes_64.
-    // mid does not normalise queries: decode or tcgen05 stand in.
+    // head_dim 64 with one scale per key over at most 256 tokens (the early scales of a schedule), us at H16, int8:
+    //               9 queries over 14 tokens                            12 over 30                                          16 over 30
+    //               fp32                  16-bit                normal. fp32                  16-bit                normal. fp32                  16-bit                normal.
+    //     batch     mid / decode / early  mid / decode / early  early   mid / decode / early  mid / decode / early  early   mid / decode / early  mid / decode / early  early
+    //       2       9.4 /  3.9 /  6.1     8.8 /  3.9 /  6.6     7.2     9.7 /  3.9 /  7.8     9.1 /  4.0 /  8.4     8.9     9.6 /  4.1 /  8.2     9.0 /  4.2 /  8.8     9.5
+    //      16      10.5 /  7.1 /  7.2    10.0 /  7.1 /  7.7     8.3    10.9 /  7.5 /  9.5    10.3 /  7.6 / 10.1    10.6    10.8 /  8.1 / 10.5    10.3 /  8.3 / 11.1    11.8
+    //      32      10.9 / 10.3 /  8.1    11.4 / 10.3 /  8.6     8.9    11.3 / 11.2 / 10.6    11.9 / 11.2 / 11.2    11.9    11.2 / 12.2 / 11.5    11.8 / 12.2 / 12.2    13.4
+    //      40      11.0 / 11.6 /  9.4    11.6 / 11.5 /  9.9    10.4    11.4 / 12.2 / 12.8    12.2 / 12.1 / 13.2    13.8    11.4 / 12.6 / 13.9    12.2 / 12.6 / 14.6    15.4
+    //      64      19.3 / 17.3 /  9.6    11.8 / 17.2 / 10.0    10.6    19.9 / 18.7 / 13.0    12.4 / 18.6 / 13.4    14.1    19.7 / 19.9 / 14.2    12.4 / 19.9 / 14.8    15.6
+    //     128      29.2 / 32.0 / 17.8    21.7 / 31.8 / 18.6    19.7    30.4 / 35.1 / 24.0    22.6 / 34.7 / 24.9    26.2    30.2 / 37.6 / 26.4    22.5 / 37.9 / 27.6    29.0
+    // (decode on normalised queries 0.3 to 4 us more than on fp32, early at 30 heads or a batch of 30 up to 13 % more than between its neighbours.)  decode and early
+    // keep weights to fp32's accuracy (1e-7 against 2e-4).  Over one chunk of keys early takes up to 12 queries, and 13 to 16 where mid would need fp32 operands
+    // or cannot normalise, beyond 5 (sample, head) pairs per SM; from 3 per SM on only while half a chunk is enough.  13 to 16 queries of more than 512 pairs
+    // that early leaves go to mid, everything else to decode, also over more keys: there mid is the faster one on 16-bit queries (16 over 64 B64
+    // 13.2 / 21.2, 16 over 256 30.3 / 30.1) and decode keeps its accuracy.
+    // 17 to 32 queries: mid where the tcgen05 kernel needs more than one wave (two CTAs per SM; 25 over 55, mid / tcgen05: B16 11.3 / 9.0, B32 12.9 / 16.9,
+    // B64 22.7 / 30.9); up to 64: mid_takes_64.
     const long long heads = (long long)B * H;
-    const bool key_scale = D == 64 && kp->group == D && vp->group == D, few = Lq > 8 && Lq <= 16 && Lk <= 256, crowded = heads > 512 && Lk <= 32;
-    if (!force && key_scale && few && crowded && Lq <= 12 && attn_early_eligible(a)) return attn_early_run(a, kb, vb, (cudaStream_t)stream);
+    const bool key_scale = D == 64 && kp->group == D && vp->group == D, few = Lq > 8 && Lq <= 16 && Lk <= 256, mid_few = heads > 512 && Lk <= 32 && Lq > 12;
+    const bool early_few = few && Lk <= 32 && (heads > 5 * sm_count() ? Lq <= 12 || q->dtype == VARQ_F32 || q_norm : heads > 3 * sm_count() && Lk <= 16);
+    if (!force && key_scale && early_few && attn_early_eligible(a)) return attn_early_run(a, kb, vb, (cudaStream_t)stream);
     // A handful of queries over a long cache: warp-level tensor-core instructions fed from global memory, where one scale covers a key.
     // us at H16, int4, bf16 queries, decode / tcgen05 (the streaming kernel takes 1.8 to 6 times decode's time):
     //     B64 c64   8 x 300: 22 / 47, 16 x 300: 37 / 47, 16 x 2240: 205 / 179, 8 x 10521: 421 / 754, 16 x 10521: 763 / 757
@@ -108,7 +114,7 @@ static int attn_impl(const varq_tensor_t* q, const varq_tensor_t* k_codes, const
     //     B2  c128  8 x 300: 10.4 / 10.0, 16 x 2240: 26 / 20, 16 x 10521: 50 / 44;   B2 c64  16 x 2240: 18 / 21, 16 x 10521: 39 / 56
     // Up to 8 queries (one CTA's worth) it is the faster one; from 9 to 16 it takes 0.6 to 1.4 times as long and stays for its
     // accuracy (3e-7 against 2e-4 for fp16 weights).
-    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (few && D == 64 && (q_norm || !crowded)));
+    const bool want_decode = force ? (force == VARQ_ATTN_PATH_DECODE) : Lq <= 16 && (Lk > 256 || (few && D == 64 && (q_norm || !mid_few)));
     if (want_decode && Lq <= 16 && attn_decode_eligible(a, kb, vb)) return attn_decode_run(a, kb, vb, workspace, workspace_bytes, (cudaStream_t)stream);
     const bool want_mid = force ? (force == VARQ_ATTN_PATH_MID) : few || (Lq > 16 && Lq <= 32 && Lk <= 256 && heads > 2 * sm_count())
                                                                                  || (Lq > 32 && Lq <= 64 && mid_takes_64(q->dtype == VARQ_F32, kb < 8 && vb < 8, heads, Lq, Lk));

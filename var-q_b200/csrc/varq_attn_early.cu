@@ -8,9 +8,15 @@
 // values of two (four at head_dim 128) queries.
 // Sums are kept in short chains (four partial sums of a score, even and odd keys of a chunk): the error stays below the general kernel's.
 // Bound by latency: three dependent global round trips (step of a token, its parameters, the codes beside them) and three block barriers per
-// 32 keys; 23 KB of shared memory and 72 registers at head_dim 64 let seven CTAs share an SM.  The general kernel (varq_attn_small.cu) stages 128
-// keys for four queries and reads the parameters of every (query, key) again.  us at B100 H16 c64 int8, general / this, 1 / 4 / 9 / 16 queries
-// over 1 / 5 / 14 / 30 tokens: 34 / 12, 36 / 13, 89 / 19, 130 / 26; B128 H30, K per dim int4: 61 / 24, 65 / 28, 187 / 39, 272 / 57.
+// 32 keys.  The general kernel (varq_attn_small.cu) stages 128 keys for four queries and reads the parameters of every (query, key) again.  us at B100
+// H16 c64 int8, general / this, 1 / 4 / 9 / 16 queries over 1 / 5 / 14 / 30 tokens: 34 / 12, 36 / 13, 89 / 19, 130 / 26; B128 H30, K per dim int4:
+// 61 / 24, 65 / 28, 187 / 39, 272 / 57.
+// Where a word's codes share their parameters (ONE: groups of at least 4 to 16, one scale per key) a thread keeps one pair of them per column instead
+// of one per code: 9 queries over 14 tokens, B64 H16 c64, int8 per head 13.4 -> 9.6, int4 per head 13.5 -> 8.6.
+// CTAs per SM (23 KB of shared memory at c64, 37 KB at 128) against spilled registers, mean of 60 calls each (2 to 128 samples, 1 to 16 queries, 1 to 256
+// tokens), relative: c64 per dim 7 (148 to 208 bytes spilled) 1, 6 (136 to 152) 1.02 int8 and 0.92 int4 but 1.13 to 1.29 where 7 make one wave less,
+// 5 (44 to 120) 0.90 to 1.01 and up to 1.33; c128 per dim 5 (96 to 280) 1, 4 (0 to 80) 0.79 int4, 0.86 int8 but 1.08 where 5 make one wave less, 3 (none) 0.76
+// and 0.88, up to 1.22; ONE at c64, 9 over 14 B64 int8: 8 (136 to 184) 12.4 us, 7 (8 to 80) 9.6 us, 6 11.6 us.
 #include <cfloat>
 
 #include "varq_attn.cuh"
@@ -21,10 +27,10 @@ namespace {
 
 constexpr int EA_THREADS = 128, EA_Q = 16, EA_KEYS = 32;
 
-// Word column `w` of a thread: 32 / BITS consecutive head_dim values, parameters of the last step seen
-template <int BITS> struct EaColumn {
-    static constexpr int N = 32 / BITS;
-    float scale[N], zp[N];
+// Word column `w` of a thread: 32 / BITS consecutive head_dim values, parameters of the last step seen.  ONE: the word lies inside one group.
+template <int BITS, bool ONE> struct EaColumn {
+    static constexpr int N = 32 / BITS, NP = ONE ? 1 : N;
+    float scale[NP], zp[NP];
     int row = -1;
     __device__ __forceinline__ void fetch(const ParamView& pv, long long base, int r, int d0) {
         if (r == row) return;
@@ -32,7 +38,10 @@ template <int BITS> struct EaColumn {
         const long long at = base + r * pv.sr;
         const float* sp = pv.scale + at + (long long)(d0 / pv.group) * pv.sg;
         const float* zq = pv.zp ? pv.zp + at + (long long)(d0 / pv.group) * pv.sg : nullptr;
-        if (pv.group == 1 && pv.sg == 1 && ((reinterpret_cast<uintptr_t>(sp) | reinterpret_cast<uintptr_t>(zq)) & 15u) == 0) {
+        if constexpr (ONE) {
+            scale[0] = __ldg(sp);
+            zp[0] = zq ? __ldg(zq) : 0.f;
+        } else if (pv.group == 1 && pv.sg == 1 && ((reinterpret_cast<uintptr_t>(sp) | reinterpret_cast<uintptr_t>(zq)) & 15u) == 0) {
 #pragma unroll
             for (int j = 0; j < N; j += 4) {
                 const float4 s = __ldg(reinterpret_cast<const float4*>(sp + j));
@@ -58,14 +67,14 @@ template <int BITS> struct EaColumn {
         for (int j = 0; j < N; j += 4) {
             float v[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = ((__uint_as_float(0x4B000000u | (x >> ((j + e) * BITS) & mask)) - bias) - zp[j + e]) * scale[j + e];
+            for (int e = 0; e < 4; ++e) v[e] = ((__uint_as_float(0x4B000000u | (x >> ((j + e) * BITS) & mask)) - bias) - zp[ONE ? 0 : j + e]) * scale[ONE ? 0 : j + e];
             *reinterpret_cast<float4*>(dst + j) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
 };
 
-template <int KB, int VB, int D>
-__global__ void __launch_bounds__(EA_THREADS, KB == 2 || VB == 2 ? 4 : D == 64 ? 7 : 5) attn_early_kernel(AttnArgs a) {
+template <int KB, int VB, int D, bool ONE>
+__global__ void __launch_bounds__(EA_THREADS, D == 128 || (!ONE && (KB == 2 || VB == 2)) ? 4 : 7) attn_early_kernel(AttnArgs a) {
     constexpr int KW = D * KB / 32, VW = D * VB / 32;                          // words per row
     constexpr int KSTEP = EA_THREADS / KW, VSTEP = EA_THREADS / VW;            // keys per pass of the CTA (at least 4)
     constexpr int KIT = KSTEP < EA_KEYS ? EA_KEYS / KSTEP : 1, VIT = VSTEP < EA_KEYS ? EA_KEYS / VSTEP : 1;
@@ -81,8 +90,8 @@ __global__ void __launch_bounds__(EA_THREADS, KB == 2 || VB == 2 ? 4 : D == 64 ?
     const int32_t* vbase = a.vc + b * a.vs_b + h * a.vs_h;
     const long long k_par = a.kp.index(b, 0, h, 0), v_par = a.vp.index(b, 0, h, 0);
     const int kw = tid % KW, kk0 = tid / KW, vw = tid % VW, vk0 = tid / VW;
-    EaColumn<KB> kcol;
-    EaColumn<VB> vcol;
+    EaColumn<KB, ONE> kcol;
+    EaColumn<VB, ONE> vcol;
 
     // ---- queries: a warp per query, scaled (and normalised) on the way in
     for (int q = warp; q < nq; q += EA_THREADS / 32) {
@@ -227,8 +236,8 @@ __global__ void __launch_bounds__(EA_THREADS, KB == 2 || VB == 2 ? 4 : D == 64 ?
     }
 }
 
-template <int KB, int VB, int D> int launch_early(const AttnArgs& a, cudaStream_t st) {
-    VARQ_CUDA_TRY(launch_pdl(attn_early_kernel<KB, VB, D>, (unsigned)((long long)a.B * a.H * a.n_qtiles), EA_THREADS, 0, st, 1, a));
+template <int KB, int VB, int D, bool ONE> int launch_early(const AttnArgs& a, cudaStream_t st) {
+    VARQ_CUDA_TRY(launch_pdl(attn_early_kernel<KB, VB, D, ONE>, (unsigned)((long long)a.B * a.H * a.n_qtiles), EA_THREADS, 0, st, 1, a));
     count_launches(1);
     return VARQ_OK;
 }
@@ -240,7 +249,8 @@ bool attn_early_eligible(const AttnArgs& a) { return a.D == 64 || a.D == 128; }
 int attn_early_run(AttnArgs& a, int kb, int vb, cudaStream_t st) {
     a.n_qtiles = (a.Lq + EA_Q - 1) / EA_Q;
     if ((long long)a.B * a.H * a.n_qtiles > 0x7fffffffLL) return fail(VARQ_ERR_UNSUPPORTED, "varq_attn_fwd: more than 2^31 thread blocks");
-#define GO(K_, V_) if (kb == K_ && vb == V_) return a.D == 64 ? launch_early<K_, V_, 64>(a, st) : launch_early<K_, V_, 128>(a, st)
+    const bool one = a.kp.group % (32 / kb) == 0 && a.vp.group % (32 / vb) == 0;
+#define GO(K_, V_) if (kb == K_ && vb == V_) return one ? (a.D == 64 ? launch_early<K_, V_, 64, true>(a, st) : launch_early<K_, V_, 128, true>(a, st)) : a.D == 64 ? launch_early<K_, V_, 64, false>(a, st) : launch_early<K_, V_, 128, false>(a, st)
     GO(8, 8); GO(8, 4); GO(8, 2); GO(4, 8); GO(4, 4); GO(4, 2); GO(2, 8); GO(2, 4); GO(2, 2);
 #undef GO
     return fail(VARQ_ERR_ARG, "varq_attn_fwd: store bits must be 2, 4 or 8");
