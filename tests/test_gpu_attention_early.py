@@ -1,7 +1,9 @@
 """The fp32 kernel of the first scales (parameters that vary along head_dim) at the edges of its 16 queries and 32 keys.
 
-Against float64 over the dequantised cache.  The dequantised values are exact in both, scores and sums are fp32: with n terms and unit rows the
-relative error stays below about sqrt(n) 2^-24 per sum, 4e-7 here for up to 256 keys; 2e-6 covers queries of length 4 and exponentials.
+Against float64 over the dequantised cache.  The dequantised values are exact in both, scores and sums are fp32.  A chain of n rounded additions errs by
+about sqrt(n) 2^-24 of its sum: the kernel's longest are 32 (four partial sums of a score over 128 dims), 16 (the keys of a chunk, even and odd) and 8
+(chunks), 3.4e-7, 2.4e-7 and 1.7e-7.  A score's error counts in full in its weight, times the score (up to 4 for unit keys and queries of length 4, scale
+0.7: 2.8): 9.5e-7 + 4e-7 in all, below 2e-6.
 """
 import pytest
 import torch

@@ -56,6 +56,23 @@ def test_query_tiles_per_cta(B, H, lq, lk):
     assert ((out - ref).norm() / ref.norm()).item() <= 1e-3        # fp16 weights
 
 
+@pytest.mark.parametrize("kw", [dict(quant_bits=4, quant_method="G_TOKEN_HEAD", symmetric=False, group_size=32), dict(quant_bits=8, quant_method="G_SCALE_HEAD_DIM")],
+                         ids=["group32", "dim8"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,H,lq,lk", [(2, 16, 169, 424), (4, 16, 256, 680), (5, 16, 256, 680), (1, 16, 169, 424), (2, 16, 256, 1025)])
+def test_query_tiles_per_cta_with_dequantised_k(B, H, lq, lk, dtype, kw):
+    """The same line for caches whose K and V every query tile of a CTA of its own has to convert again."""
+    g = torch.Generator(device="cuda").manual_seed(lq + lk)
+    kq, vq = (VAR_Q(qkv_format="BHLc", max_tokens=lk, **kw) for _ in range(2))
+    for qz in (kq, vq):
+        for n in (lk // 3, lk - lk // 3):
+            qz.append(torch.randn((B, H, n, 64), generator=g, device="cuda"))
+    q = torch.randn((B, H, lq, 64), generator=g, device="cuda").to(dtype)
+    out = attend_cached(q, kq, vq, 0.125, out_dtype=torch.float32).transpose(1, 2).double()
+    ref = torch.softmax(q.double() @ kq.dequant_all().double().transpose(-1, -2) * 0.125, -1) @ vq.dequant_all().double()
+    assert ((out - ref).norm() / ref.norm()).item() <= 1e-3        # fp16 weights and V
+
+
 @pytest.mark.parametrize("normalised", [False, True])
 @pytest.mark.parametrize("dtype,shift,pad", [(torch.float32, 1, 1), (torch.bfloat16, 1, 0), (torch.bfloat16, 0, 3), (torch.float16, 3, 1)])
 @pytest.mark.parametrize("kw", [dict(quant_bits=8, quant_method="G_TOKEN_HEAD"), dict(quant_bits=4, quant_method="G_TOKEN_HEAD", symmetric=False, group_size=32),

@@ -138,7 +138,7 @@ def _attn_call(path, q, kq, vq, scale, out_dtype):
     return out.payload.view(B, Lq, H, D), lib.varq_launch_count() - n0
 
 
-@pytest.mark.parametrize("path", ["small", "stream", "tc", "mid", "decode"])
+@pytest.mark.parametrize("path", ["small", "stream", "tc", "mid", "decode", "early"])
 @pytest.mark.parametrize("D,kb,vb", [(64, 8, 4), (128, 4, 2)])
 @pytest.mark.parametrize("lq,lk", [(1, 1), (1, 333), (3, 129), (16, 2047), (17, 65), (130, 131), (257, 1000)])
 def test_attention_kernels_stay_inside_their_buffers(path, D, kb, vb, lq, lk):
@@ -155,3 +155,20 @@ def test_attention_kernels_stay_inside_their_buffers(path, D, kb, vb, lq, lk):
         ref = O.attention(q, kd, vd, fmt, 1.0 / D ** 0.5).transpose(1, 2)
         tol = 2e-3 if out_dtype == torch.float32 else 2e-2
         assert (out.float().cpu() - ref).abs().max().item() <= tol
+
+
+@pytest.mark.parametrize("path", ["early", "tc"])
+@pytest.mark.parametrize("D,kb,vb", [(64, 8, 8), (128, 4, 2)])
+@pytest.mark.parametrize("lq,lk", [(1, 1), (16, 31), (17, 65), (130, 131), (257, 300)])
+def test_parameters_along_head_dim_stay_inside_their_buffers(path, D, kb, vb, lq, lk):
+    """Per-dim parameters in two steps (the early kernel loads them four at a time), several and ragged query tiles."""
+    B, H = 2, 3
+    kq, vq = (VAR_Q(b, "BHLc", "G_SCALE_HEAD_DIM", symmetric=False) for b in (kb, vb))
+    for n in (lk - lk // 3, lk // 3):
+        if n:
+            kq.append(O.synthetic_kv((B, H, n, D), "BHLc", lk + n, n_outlier=2).to(DEV))
+            vq.append(O.synthetic_kv((B, H, n, D), "BHLc", lk + n + 1, n_outlier=0).to(DEV))
+    q = torch.randn((B, H, lq, D), generator=torch.Generator().manual_seed(lq))
+    out, _ = _attn_call(path, q.to(DEV), kq, vq, 1.0 / D ** 0.5, torch.float32)
+    ref = O.attention(q, kq.dequant_all().cpu(), vq.dequant_all().cpu(), "BHLc", 1.0 / D ** 0.5).transpose(1, 2)
+    assert (out.float().cpu() - ref).abs().max().item() <= 2e-3

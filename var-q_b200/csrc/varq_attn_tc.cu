@@ -43,7 +43,9 @@ bool attn_tc_eligible(const AttnArgs& a, int kb, int vb) {
 // Two query tiles per CTA share every converted K / V tile; a second tile needs queries to fill it.  Where such CTAs would fill less than half
 // of the SMs and the cache is short, single tiles occupy twice as many, and need no key splits and no merge.  us, two / one tile, int8 per head
 // H16: 169 queries over 424 tokens B2 18.8 / 13.5, B4 15.3 / 14.1; 256 over 680 B2 22.3 / 17.2, B4 21.1 / 18.0.  Over long caches the splits are worth
-// more (256 over 8000 int4 group 32 B2 50 / 98), and with fewer CTAs still both are split (169 over 424, per dim, B1 15.3 / 16.7).
+// more (256 over 8000 int4 group 32 B2 50 / 98), and with fewer CTAs still both are split (169 over 424, per dim, B1 15.3 / 16.7).  Grouped and per-dim caches,
+// which a CTA of its own converts again, gain as much: one / two over 24 to 64 CTAs of two tiles, 0.66 to 0.96 (200 to 400 queries over 500 to 1024 tokens,
+// int8 per head 0.70 to 0.93, int8 per dim 0.67 to 0.96, groups of 32 0.66 to 0.92, int4 per dim 0.76 to 0.98), 0.89 to 1.03 for 130 over 200.
 static int tc_query_tiles(int B, int H, int Lq, int Lk, int D) {
     if (D != 64 || Lq <= TC_M) return 1;
     const long long heads = (long long)B * H, one = heads * ((Lq + TC_M - 1) / TC_M), two = heads * ((Lq + 2 * TC_M - 1) / (2 * TC_M));
