@@ -52,11 +52,6 @@ template <int BITS> struct CodeMagic {
 template <int BITS> struct Item {           // 16 consecutive codes of one key: 4, 2 or 1 packed words -> 8 pairs
     static constexpr int NW = BITS / 2;
     static constexpr int CLS = BITS == 8 ? 1 : BITS == 4 ? 2 : 4;      // classes of bit position: pair i has class i % CLS
-    static __device__ __forceinline__ void load(const uint32_t* p, uint32_t (&w)[NW]) {
-        if constexpr (NW == 4) { const uint4 v = *reinterpret_cast<const uint4*>(p); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
-        else if constexpr (NW == 2) { const uint2 v = *reinterpret_cast<const uint2*>(p); w[0] = v.x; w[1] = v.y; }
-        else w[0] = *p;
-    }
     // pairs holding 1024 + 2^p (code + bias)
     static __device__ __forceinline__ void raw(const uint32_t* w, uint32_t (&h)[8], const CodeMagic<BITS>& cm) {
         if constexpr (BITS == 8) {
