@@ -862,7 +862,7 @@ def run_case(name):
     g = torch.Generator(device=dev).manual_seed(0)
     nbytes = None
     if name.startswith("attn"):
-        # attn: the VAR-d16 last scale at a quarter of the batch (exact-code K); attn_early: one of its early scales; attn_perdim: VAR-d30 K/V settings, Lq 1024 over
+        # attn: the VAR-d16 last scale at a quarter of the batch (exact-code K); attn_early: one of its early scales; attn_first: a first scale with K per dim; attn_perdim: VAR-d30 K/V settings, Lq 1024 over
         # 2240 tokens in ten steps, 8 samples; attn_group: Infinity settings, Lq 1024 over 4096 tokens, 4 samples
         if name == "attn":
             B, H, D, fmt, steps, lq = 16, 16, 64, "BLHc", (680,), 256
@@ -870,6 +870,9 @@ def run_case(name):
         elif name == "attn_early":      # the fifth scale of the VAR-d16 schedule at full batch: 25 queries over 55 cached tokens
             B, H, D, fmt, steps, lq = 64, 16, 64, "BLHc", (1, 4, 9, 16, 25), 25
             ka, va = (8, "G_TOKEN_HEAD", {}), (8, "G_TOKEN_HEAD", {})
+        elif name == "attn_first":      # the third scale of the VAR-d30 schedule at full batch: 9 queries over 14 cached tokens, K per dim
+            B, H, D, fmt, steps, lq = 128, 30, 64, "BLHc", WORKLOADS["var_d30"]["steps_l"][:3], 9
+            ka, va = WORKLOADS["var_d30"]["k"], WORKLOADS["var_d30"]["v"]
         elif name == "attn_perdim":
             B, H, D, fmt, steps, lq = 8, 30, 64, "BLHc", WORKLOADS["var_d30"]["steps_l"], 1024
             ka, va = WORKLOADS["var_d30"]["k"], WORKLOADS["var_d30"]["v"]
@@ -927,7 +930,7 @@ def main():
     ap.add_argument("--no-sweep", action="store_true", help="skip the isolated dequant-attention sweep")
     ap.add_argument("--quick", action="store_true", help="headline measurement only (no per-kernel rooflines, sweep, other workloads, CPU leg)")
     ap.add_argument("--no-graph", action="store_true", help="launch every kernel from Python instead of replaying a CUDA graph")
-    ap.add_argument("--case", choices=("attn", "attn_early", "attn_perdim", "attn_group", "decode", "stream", "quant", "quant2", "dequant") +
+    ap.add_argument("--case", choices=("attn", "attn_first", "attn_early", "attn_perdim", "attn_group", "decode", "stream", "quant", "quant2", "dequant") +
                     tuple("layer_" + n for n in sorted(WORKLOADS)),
                     help="run one kernel on a small case and exit (profiling aid)")
     args = ap.parse_args()

@@ -19,10 +19,17 @@
 // More than 128 queries share each converted tile (QT = 2, head_dim 64, all 512 TMEM columns); up to 128 queries run as two CTAs per SM of
 // 256 columns each, one CTA's set-up and dependent waits under the other's tiles.  At head_dim 128 one CTA keeps three or four score
 // tiles in flight.
-// What bounds it: at head_dim 64 the softmax warps, two per sub-partition (64 x 256 scores: 1024 cycles of the exponential unit, 1900 to 2300 in
-// all beside conversion and tensor pipe; 2800 while the maximum came before the exponentials).  Without exponentials 1299 -> 923 us (B64 H16
-// 256 x 10521, int2 group 32), without tables 1279 -> 1180 (B32 H30 1024 x 2240, int4, K per dim).  At 128 softmax and conversion share the issue slots
-// (1650 and 1800 cycles a tile, tensor pipe 1024), and long calls run into the power limit: what fewer cycles save the clock gives back in part.
+// What bounds it, from builds that leave out arithmetic and keep every load, store, barrier and product (us a call: whole / no exponentials / constant
+// operand tiles instead of conversion / neither; constant operands also draw less power):
+//   c 64   B64 H16 256 x 10521, int2 group 32, bf16 queries       1237 /  853 / 1026 /  719
+//          B32 H30 1024 x 2240, int4, K per dim, fp32 queries      1298 / 1150 / 1178 / 1072
+//          B64 H16 256 x 680, int8 per head, fp32 queries          151 /  152 /  146 /  138
+//   c 128  B4 H16 4096 x 10521, int4 and int2 group 32, fp32      2622 / 2591 / 1715 / 1425
+//          B6 H16 1600 x 6000, int8 per dim, fp32                 1067 / 1063 /  653 /  630
+//          B2 H16 4096 x 10521, int8 per head, bf16               1043 / 1083 /  952 /  943
+// At head_dim 64 over long caches the softmax warps, two per sub-partition: 64 x 256 scores need 1024 cycles of the exponential unit, a tile takes 2100;
+// over short ones what surrounds the tile loop.  At 128 the conversion of a dequantised K, in issue slots and in what its hi + lo operands draw (2250 cycles
+// a tile at the full clock, 1024 of them the tensor pipe's; long calls run into the power limit).
 // Few CTAs over a long cache: the key range is split across CTAs and a second kernel merges the partial rows.
 // Numerics: integer codes are exact in fp16; an fp32 query is split into hi + lo fp16 halves, a dequantised K likewise (the lo x lo
 // product is below fp32 resolution), so S has fp32-like accuracy; P and a dequantised V are rounded to fp16 once; sums are fp32.
@@ -255,7 +262,7 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     static constexpr int OFF_XCH = OFF_PREF + 2 * 48;         // float [4][QT * 128]: the two threads of a row, maxima and sums
     static constexpr int OFF_DYN = OFF_XCH + (HV == 2 ? 4 * QT * TC_M * 4 : 0);   // packed stages, records, step tables: sizes known at launch (TcDyn)
     // Queries that come in through shared memory: a warp reads contiguous pieces of rows and hands each lane its own (the V stages; the V converters
-    // leave them alone until the queries are in place).  Every lane reading its row takes 32 sectors an instruction and 7000 cycles of a CTA.  us per
+    // leave them alone until the queries are in place).  Every lane reading its row takes 32 sectors an instruction.  us per
     // call, lane by lane / so: head_dim 64, int8 B64 H16 256 x 680 155 / 149, int8 per dim B100 H16 228 / 217, int4 B64 H30 324 x 645 526 / 498, 16-bit
     // queries over exact int2 1044 x 505 85 / 80; head_dim 128, int8 per dim B16 H16 400 x 921 bf16 normalised 185 / 164, int8 per head B64 144 x 265 196 / 175.
     // Not so: 16-bit queries over a dequantised K, where the loop behind lost more to its changed schedule (c64 int2 group 32 1237 / 1278, c128 int8
@@ -353,7 +360,7 @@ struct StepRegs { uint32_t sh[8], sl[8], nz[8]; int step; };
 // Parameters of n steps from r0 on -> a table fp16 [n][3][D]: scale hi, scale lo, zero-point constant, in operand order (the
 // zero-point constants of a 16-wide slice start with PAR_SLOW when one of its elements is out of bounds).  By nthr threads, a lane per
 // element and eight elements' loads in flight: a CTA converts nothing before its table is there (a thread per slice, whose loads waited for one
-// another, took 10000 cycles of the 95000 of a CTA over 2240 tokens).
+// another: int8 per dim B100 H16 256 x 680 237 us, 221 so).
 template <int D>
 __device__ __forceinline__ void fill_steps(unsigned char* steptab, const ParamRef* ref, int r0, int n, int bits, int ptid, int nthr) {
     __half* tb = reinterpret_cast<__half*>(steptab);
