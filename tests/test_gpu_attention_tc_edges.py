@@ -73,6 +73,14 @@ def test_query_tiles_per_cta_with_dequantised_k(B, H, lq, lk, dtype, kw):
     assert ((out - ref).norm() / ref.norm()).item() <= 1e-3        # fp16 weights and V
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,H,lq,lk", [(2, 18, 256, 1100), (2, 19, 200, 1100), (2, 37, 129, 1024), (2, 37, 129, 1300), (5, 15, 200, 1300)])
+def test_query_tiles_per_cta_over_longer_caches(B, H, lq, lk, dtype):
+    """36 CTAs of two tiles (their key range is split), 38 and 74 (single tiles), 75 (two again)."""
+    test_query_tiles_per_cta_with_dequantised_k(B, H, lq, lk, dtype, dict(quant_bits=8, quant_method="G_SCALE_HEAD_DIM"))
+    test_query_tiles_per_cta(B, H, lq, lk)
+
+
 @pytest.mark.parametrize("normalised", [False, True])
 @pytest.mark.parametrize("dtype,shift,pad", [(torch.float32, 1, 1), (torch.bfloat16, 1, 0), (torch.bfloat16, 0, 3), (torch.float16, 3, 1)])
 @pytest.mark.parametrize("kw", [dict(quant_bits=8, quant_method="G_TOKEN_HEAD"), dict(quant_bits=4, quant_method="G_TOKEN_HEAD", symmetric=False, group_size=32),

@@ -40,16 +40,19 @@ bool attn_tc_eligible(const AttnArgs& a, int kb, int vb) {
     return true;
 }
 
-// Two query tiles per CTA share every converted K / V tile; a second tile needs queries to fill it.  Where such CTAs would fill less than half
-// of the SMs and the cache is short, single tiles occupy twice as many, and need no key splits and no merge.  us, two / one tile, int8 per head
-// H16: 169 queries over 424 tokens B2 18.8 / 13.5, B4 15.3 / 14.1; 256 over 680 B2 22.3 / 17.2, B4 21.1 / 18.0.  Over long caches the splits are worth
-// more (256 over 8000 int4 group 32 B2 50 / 98), and with fewer CTAs still both are split (169 over 424, per dim, B1 15.3 / 16.7).  Grouped and per-dim caches,
-// which a CTA of its own converts again, gain as much: one / two over 24 to 64 CTAs of two tiles, 0.66 to 0.96 (200 to 400 queries over 500 to 1024 tokens,
-// int8 per head 0.70 to 0.93, int8 per dim 0.67 to 0.96, groups of 32 0.66 to 0.92, int4 per dim 0.76 to 0.98), 0.89 to 1.03 for 130 over 200.
+// Two query tiles per CTA share every converted K / V tile; a second tile needs queries to fill it.  Where such CTAs would fill at most half
+// of the SMs, single tiles occupy twice as many.  One / two, int8 per head, int8 per dim and int4 in groups of 32, bf16 and fp32 queries, H16 and H30:
+//   CTAs of two tiles      300 to 680 tokens   1024          2048          4096
+//   38 to 72               0.78 to 1.00        0.78 to 0.97  0.78 to 1.00  0.77 to 1.01     (neither is split; 74 of 150 queries 0.84 to 1.02, fp32 per dim 1.04 to 1.12)
+//   80 to 144              1.00 to 1.10        1.06 to 1.17  1.07 to 1.22  1.07 to 1.23     (two single tiles share an SM and convert everything twice)
+//   20 to 37               0.63 to 0.91        0.83 to 1.02  1.13 to 1.39  1.57 to 1.81     (the key range of two tiles is split, that of one is not)
+// In the last row one / two cross at 1100 to 1300 tokens.  With fewer CTAs still both are split: 0.81 to 0.97 for 256 queries of 16 pairs, but 1.09 for
+// 169 over 424 tokens, per dim.
 static int tc_query_tiles(int B, int H, int Lq, int Lk, int D) {
     if (D != 64 || Lq <= TC_M) return 1;
     const long long heads = (long long)B * H, one = heads * ((Lq + TC_M - 1) / TC_M), two = heads * ((Lq + 2 * TC_M - 1) / (2 * TC_M));
-    return Lk <= 16 * TC_N && two * 2 <= sm_count() && one * 4 > sm_count() ? 1 : 2;
+    const bool split = two * 4 <= sm_count();
+    return two * 2 <= sm_count() && one * 4 > sm_count() && (!split || Lk <= 16 * TC_N) ? 1 : 2;
 }
 
 // Key range of a CTA.  Splitting pays when the CTAs of the unsplit grid leave most of the chip idle and every part still has a few
