@@ -266,7 +266,9 @@ template <int D, int NQ, int QT, int KM, int VM> struct TcPlan {
     // call, lane by lane / so: head_dim 64, int8 B64 H16 256 x 680 155 / 149, int8 per dim B100 H16 228 / 217, int4 B64 H30 324 x 645 526 / 498, 16-bit
     // queries over exact int2 1044 x 505 85 / 80; head_dim 128, int8 per dim B16 H16 400 x 921 bf16 normalised 185 / 164, int8 per head B64 144 x 265 196 / 175.
     // Not so: 16-bit queries over a dequantised K, where the loop behind lost more to its changed schedule (c64 int2 group 32 1237 / 1278, c128 int8
-    // 886 / 985), and up to 128 queries over grouped K at head_dim 64 (9 x 700 fp32 B48 H20 67 / 75, 100 x 255 B100 H16 68 / 74).
+    // 886 / 985), and up to 128 queries over grouped K at head_dim 64 (9 x 700 fp32 B48 H20 67 / 75, 100 x 255 B100 H16 68 / 74;
+    // over 8, 4 and 2 bits, 32 to 1920 (sample, head) pairs, 17 to 128 queries and 121 to 5200 tokens it takes 1.02, 1.04 and 1.03 times as long on average: up to
+    // 1.41 over long caches, 0.94 to 0.98 over two tiles of keys, 0.89 to 0.97 for 36 to 56 queries of 1280 pairs and more over 500 to 1800 tokens).
     static constexpr bool Q_STAGED = NQ == 2 ? D == 128 || QT == 2 || KM != PM_GROUP : D == 64 && KX;
     static constexpr int Q_STAGE = 32 * (D == 128 ? 144 : 80);           // bytes per softmax warp
     static_assert(K_WARP0 * Q_STAGE <= VST * T_BYTES, "query staging");
